@@ -43,6 +43,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fp64_stage.cuh"
 #include "near_mixed.cuh"
 #include "tc_common.cuh"
 
@@ -64,12 +65,12 @@ struct NearJob {
   int na, nb, N;       // valid rows along a and b; output columns
   int brow;            // B (matrix) row of t-point 0, column 0
   int koff;            // the job's K columns start at koff in its matrix rows
-  int kr_ps;           // K bands per t-point (128-column tiles)
+  int kr_ps;           // K bands per t-point (kBandCols columns each)
   int inst;            // density of the set (scales)
   int ta;              // 32-row blocks along a
   int pad_;
   long long ooff;      // intermediate stages: first output slice
-  const int2 *band;    // K band [first, last] per (t-point, 128-column tile)
+  const int2 *band;    // K band [first, last] per (t-point, kBandCols columns)
   double *V;           // last stage: V at the box's first owned point
   long long vs_b, vs_n;
 };
@@ -146,7 +147,11 @@ __device__ __forceinline__ void near_mma_run(uint32_t P, uint32_t Cc, uint64_t d
 // K blocks [first, last] of job j, n-tile nt, t-point p + gi
 template <int TNW>
 __device__ __forceinline__ int2 near_kblocks(const NearArgs &a, const NearJob &j, int nt, int gi) {
-  const int2 r = j.band[(size_t)(a.p + gi) * j.kr_ps + (nt * TNW) / 128];
+  const int2 *b = j.band + (size_t)(a.p + gi) * j.kr_ps + nt * (TNW / kBandCols);
+  int2 r = b[0];
+#pragma unroll
+  for (int g = 1; g < TNW / kBandCols; ++g)
+    if (nt * TNW + g * kBandCols < j.N) r = make_int2(min(r.x, b[g].x), max(r.y, b[g].y));
   return make_int2((r.x + j.koff) / BKN, (r.y + j.koff) / BKN);
 }
 
@@ -889,7 +894,7 @@ int near_f16_set_bind(NearF16Set *st, const double *const *rho, double *const *V
       x.nb = g.nq[2][vz];
       x.N = g.own[0][vx];
       x.brow = pl->brow[0][vx];
-      x.kr_ps = ceil_div(x.N, 128);
+      x.kr_ps = ceil_div(x.N, kBandCols);
       x.band = g.band[0][vx];
       x.ooff = xoff;  // U slices of this job: x own
       x.ta = ceil_div(x.na, kRowsA);
@@ -902,7 +907,7 @@ int near_f16_set_bind(NearF16Set *st, const double *const *rho, double *const *V
       y.nb = g.own[0][vx];
       y.N = g.own[1][vy];
       y.brow = pl->brow[1][vy];
-      y.kr_ps = ceil_div(y.N, 128);
+      y.kr_ps = ceil_div(y.N, kBandCols);
       y.band = g.band[1][vy];
       y.ooff = yoff;  // W slices: y own
       y.ta = ceil_div(y.na, kRowsA);
@@ -915,7 +920,7 @@ int near_f16_set_bind(NearF16Set *st, const double *const *rho, double *const *V
       z.nb = g.own[1][vy];
       z.N = g.own[2][vz];
       z.brow = pl->brow[2][vz];
-      z.kr_ps = ceil_div(z.N, 128);
+      z.kr_ps = ceil_div(z.N, kBandCols);
       z.band = g.band[2][vz];
       z.ta = ceil_div(z.na, kRowsA);
       z.inst = i;

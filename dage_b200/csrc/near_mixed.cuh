@@ -19,7 +19,7 @@ namespace dage {
 // Geometry of one GBFMM grid (plan): per axis, per box position, the near
 // region (first point, points) and the owned output points, and the FP64
 // near-field matrices T[pos][p][own][nq] with their K bands per (t-point,
-// 128-row tile).
+// kBandCols rows).
 struct NearGeom {
   int npts[3] = {0, 0, 0};
   int P = 0;

@@ -14,6 +14,7 @@
 // (and one tensor-core kernel in op3d_mixed.cu) serves all three.  This is
 // the same arithmetic as the reference's per-slice DGEMMs
 // (src/bubbles/function3d.F90:4296-4332), reordered for coalescing.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <string>
@@ -144,7 +145,7 @@ int launch_tmatrix(const TmatArgs &a, int nlip, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // FP64 contraction stage (fp64_stage.cuh) on DMMA
 // ---------------------------------------------------------------------------
-constexpr int BM = kFp64TileM, BN = kFp64TileN, BK = 16, SROW = BK + 4, NST = 3;
+constexpr int BM = kFp64TileM, BK = 16, SROW = BK + 4, NST = 3;
 
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
   const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
@@ -167,99 +168,143 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// TN: tile width in n (32, 64 or 128); warps 2 (M) x 4 (N), each 64 x TN/4.
 template <int TN>
 constexpr int stage_smem() {
   return NST * (BM + TN) * SROW * (int)sizeof(double);
 }
+// blocks per SM: two of the narrower tiles fit (77 and 92 KB, at most 128
+// registers a thread), one of 128 columns (123 KB)
+template <int TN>
+constexpr int stage_blocks() {
+  return TN == 128 ? 1 : 2;
+}
 
+// One tile (rows m0.., columns n0..) for the t-points p0 .. p0 + np - 1: the
+// K loop runs through their bands one after another.  X and out are those of
+// t-point p0's slot; with np > 1 the products are summed.
 template <bool ACCUM, int TN>
-__device__ __forceinline__ void stage_tile(const StageDesc &d, double alpha, int m0, int n0) {
-  constexpr int NB = TN / 32;   // 8-column MMA tiles per warp
+__device__ __forceinline__ void stage_tile(const StageDesc &d, const double *X, double *out,
+                                           int p0, int np, double alpha, int m0, int n0) {
+  constexpr int WN = TN / 32;   // warps along n, 32 columns each
+  constexpr int MB = TN / 16;   // 8-row MMA tiles per warp
   constexpr int BR = TN / 16;   // B rows copied per thread per K step
   extern __shared__ double fsm[];
   double *As = fsm;                    // [NST][BM][SROW]
   double *Bs = fsm + NST * BM * SROW;  // [NST][TN][SROW]
+  __shared__ int2 band[kMaxPointGroup][WN];  // per t-point and 32 columns
+  __shared__ int2 span[kMaxPointGroup];      // their union, first rounded down to 4
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 64, wn = (warp >> 1) * (TN / 4);
-  int kt0 = 0, kt1 = (d.K + BK - 1) / BK - 1;
-  if (d.krange) {  // bands are kept per 128 columns
-    const int2 r = d.krange[n0 / kFp64TileN];
-    kt0 = r.x / BK;
-    kt1 = r.y / BK;
+  // warps 4 apart share a scheduler: give them different columns, so that
+  // bands of different lengths spread over the schedulers
+  const int gn = WN == 1 ? 0 : WN == 2 ? warp >> 2 : (warp & 1) + 2 * (warp >> 2);
+  const int gm = WN == 1 ? warp : WN == 2 ? warp & 3 : (warp >> 1) & 1;
+  const int wm = gm * MB * 8, wn = gn * 32;
+  for (int i = tid; i < np; i += blockDim.x) {
+    int lo = d.K, hi = 0;
+#pragma unroll
+    for (int g = 0; g < WN; ++g) {
+      int2 r = make_int2(0, -1);
+      if (n0 + 32 * g < d.N)
+        r = d.krange ? d.krange[(size_t)(p0 + i) * d.kr_ps + n0 / kBandCols + g]
+                     : make_int2(0, d.K - 1);
+      band[i][g] = r;
+      if (r.y >= r.x) lo = min(lo, r.x), hi = max(hi, r.y);
+    }
+    span[i] = make_int2(lo & ~3, hi);
   }
-  const int nk = kt1 - kt0 + 1;
+  __syncthreads();
+  int nsteps = 0;
+  for (int i = 0; i < np; ++i) nsteps += (span[i].y - span[i].x) / BK + 1;
 
-  // this thread copies rows (tid >> 4) + 16 i at K offset tid & 15
+  // this thread copies rows (tid >> 4) + 16 i at K offset tid & 15; row
+  // offsets are relative to row m0 (a tile spans 128 rows: 32 bits do)
   const int kk = tid & 15;
-  const double *arow[8];
-  const double *brow[BR];
+  const uint32_t ad0 = (uint32_t)d.a_d0;
+  const long long abase = ((uint32_t)m0 % ad0) * d.a_s1 + ((uint32_t)m0 / ad0) * d.a_s2;
+  int aoff[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const long long m = m0 + (tid >> 4) + 16 * i;
-    arow[i] = m < d.M ? d.X + (m % d.a_d0) * d.a_s1 + (m / d.a_d0) * d.a_s2 : nullptr;
+    const uint32_t m = m0 + (tid >> 4) + 16 * i;
+    aoff[i] = m < (uint32_t)d.M ? (int)((m % ad0) * d.a_s1 + (m / ad0) * d.a_s2 - abase) : -1;
   }
-#pragma unroll
-  for (int i = 0; i < BR; ++i) {
-    const int n = n0 + (tid >> 4) + 16 * i;
-    brow[i] = n < d.N ? d.T + (size_t)n * d.ldt : nullptr;
-  }
-  auto load = [&](int slot, int kt) {
-    const int k = kt * BK + kk;
+  const int nrow = n0 + (tid >> 4);
+  const double *xb = X + abase + kk;
+  const double *tb = d.T + (size_t)p0 * d.t_ps + (size_t)nrow * d.ldt + kk;
+  int li = 0, lk = span[0].x, lhi = span[0].y;  // the next step to copy
+  auto load = [&](int slot) {
+    const bool pk = lk + kk < d.K;
     double *as = As + slot * BM * SROW + (tid >> 4) * SROW + kk;
     double *bs = Bs + slot * TN * SROW + (tid >> 4) * SROW + kk;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const bool pa = arow[i] && k < d.K;
-      cp_async8(as + 16 * i * SROW, pa ? arow[i] + k : d.X, pa);
+      const bool pa = pk && aoff[i] >= 0;
+      cp_async8(as + 16 * i * SROW, pa ? xb + aoff[i] + lk : X, pa);
     }
 #pragma unroll
     for (int i = 0; i < BR; ++i) {
-      const bool pb = brow[i] && k < d.K;
-      cp_async8(bs + 16 * i * SROW, pb ? brow[i] + k : d.T, pb);
+      const bool pb = pk && nrow + 16 * i < d.N;
+      cp_async8(bs + 16 * i * SROW, pb ? tb + (size_t)(16 * i) * d.ldt + lk : d.T, pb);
+    }
+    lk += BK;
+    if (lk > lhi && ++li < np) {
+      lk = span[li].x;
+      lhi = span[li].y;
+      xb += d.x_ps;
+      tb += d.t_ps;
     }
   };
 
-  double acc[8][NB][2];
+  double acc[MB][4][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < MB; ++i)
 #pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
 #pragma unroll
   for (int st = 0; st < NST - 1; ++st) {
-    if (st < nk) load(st, kt0 + st);
+    if (st < nsteps) load(st);
     cp_async_commit();
   }
-  for (int i = 0; i < nk; ++i) {
+  int ci = 0, ck = span[0].x, chi = span[0].y;
+  int2 gb = band[0][gn];
+  for (int i = 0; i < nsteps; ++i) {
     cp_async_wait<NST - 2>();
     __syncthreads();  // slot i landed for all threads; slot i-1 is free
-    if (i + NST - 1 < nk) load((i + NST - 1) % NST, kt0 + i + NST - 1);
+    if (i + NST - 1 < nsteps) load((i + NST - 1) % NST);
     cp_async_commit();
     const double *as = As + (i % NST) * BM * SROW + (wm + (lane >> 2)) * SROW + (lane & 3);
     const double *bs = Bs + (i % NST) * TN * SROW + (wn + (lane >> 2)) * SROW + (lane & 3);
+    const int ks0 = (gb.x - ck) >> 2, ks1 = (gb.y - ck) >> 2;  // this warp's band
 #pragma unroll
     for (int ks = 0; ks < BK / 4; ++ks) {
-      double fa[8], fb[NB];
+      if (ks < ks0 || ks > ks1) continue;  // uniform in the warp
+      double fa[MB], fb[4];
 #pragma unroll
-      for (int mb = 0; mb < 8; ++mb) fa[mb] = as[mb * 8 * SROW + ks * 4];
+      for (int mb = 0; mb < MB; ++mb) fa[mb] = as[mb * 8 * SROW + ks * 4];
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb) fb[nb] = bs[nb * 8 * SROW + ks * 4];
+      for (int nb = 0; nb < 4; ++nb) fb[nb] = bs[nb * 8 * SROW + ks * 4];
 #pragma unroll
-      for (int mb = 0; mb < 8; ++mb)
+      for (int mb = 0; mb < MB; ++mb)
 #pragma unroll
-        for (int nb = 0; nb < NB; ++nb) dmma(acc[mb][nb], fa[mb], fb[nb]);
+        for (int nb = 0; nb < 4; ++nb) dmma(acc[mb][nb], fa[mb], fb[nb]);
+    }
+    ck += BK;
+    if (ck > chi && ++ci < np) {
+      ck = span[ci].x;
+      chi = span[ci].y;
+      gb = band[ci][gn];
     }
   }
   cp_async_wait<0>();
 
+  const uint32_t od0 = (uint32_t)d.o_d0;
 #pragma unroll
-  for (int mb = 0; mb < 8; ++mb) {
-    const long long m = m0 + wm + mb * 8 + (lane >> 2);
-    if (m >= d.M) continue;
-    double *orow = d.out + (m % d.o_d0) * d.o_s1 + (m / d.o_d0) * d.o_s2;
+  for (int mb = 0; mb < MB; ++mb) {
+    const uint32_t m = m0 + wm + mb * 8 + (lane >> 2);
+    if (m >= (uint32_t)d.M) continue;
+    double *orow = out + (m % od0) * d.o_s1 + (m / od0) * d.o_s2;
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
+    for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int n = n0 + wn + nb * 8 + 2 * (lane & 3) + h;
@@ -273,24 +318,32 @@ __device__ __forceinline__ void stage_tile(const StageDesc &d, double alpha, int
   }
 }
 
-template <bool ACCUM, int TN>
-__global__ void __launch_bounds__(256, 1)
-    stage_fp64_kernel(const __grid_constant__ StageDesc d, double alpha) {
-  stage_tile<ACCUM, TN>(d, alpha, blockIdx.x * BM, blockIdx.y * TN);
+// grid.x: tiles, n fastest (the blocks in flight share rows of X); grid.y:
+// t-point slots.  SUM: one block takes the whole group of np t-points.
+template <bool ACCUM, int TN, bool SUM>
+__global__ void __launch_bounds__(256, stage_blocks<TN>())
+    stage_fp64_kernel(const __grid_constant__ StageDesc d, int p0, int np, double alpha) {
+  const int nt = (d.N + TN - 1) / TN;
+  const int m0 = (blockIdx.x / nt) * BM, n0 = (blockIdx.x % nt) * TN;
+  if (SUM) {
+    stage_tile<ACCUM, TN>(d, d.X, d.out, p0, np, alpha, m0, n0);
+  } else {
+    const int i = blockIdx.y, p = p0 + i;
+    stage_tile<ACCUM, TN>(d, d.X + i * d.x_ps, d.out + i * d.o_ps, p, 1, d.wp ? d.wp[p] : alpha,
+                          m0, n0);
+  }
 }
 
 template <bool ACCUM, int TN>
-__global__ void __launch_bounds__(256, 1)
-    stage_fp64_batched_kernel(const StageDesc *__restrict__ descs, int p, double alpha) {
-  StageDesc d = descs[blockIdx.z];
-  d.T += p * d.t_ps;
-  if (d.krange) d.krange += p * d.kr_ps;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * TN;
+__global__ void __launch_bounds__(256, stage_blocks<TN>())
+    stage_fp64_batched_kernel(const StageDesc *__restrict__ descs, int nt, int p, double alpha) {
+  const StageDesc d = descs[blockIdx.z];
+  const int m0 = (blockIdx.x / nt) * BM, n0 = (blockIdx.x % nt) * TN;
   if (m0 >= d.M || n0 >= d.N) return;  // uniform across the block
-  stage_tile<ACCUM, TN>(d, d.wp ? d.wp[p] : alpha, m0, n0);
+  stage_tile<ACCUM, TN>(d, d.X, d.out, p, 1, d.wp ? d.wp[p] : alpha, m0, n0);
 }
 
-// Band of each (t-point, 128-row tile) of an axis matrix T[p][n][K]: the
+// Band of each (t-point, kBandCols rows) of an axis matrix T[p][n][K]: the
 // first and last K index holding an entry above 2^-64 of its row's scale
 // 2^ceil(log2 max_K |T(n, :)|).  One block per (p, tile), one warp per row.
 // Tiles of all-zero rows get [0, 0].
@@ -304,8 +357,8 @@ __global__ void band_kernel(const double *__restrict__ T, int K, int N, int ntil
     hi = -1;
   }
   __syncthreads();
-  for (int rr = warp; rr < BN; rr += blockDim.x >> 5) {
-    const int n = tile * BN + rr;
+  for (int rr = warp; rr < kBandCols; rr += blockDim.x >> 5) {
+    const int n = tile * kBandCols + rr;
     if (n >= N) break;
     const double *row = T + ((size_t)p * N + n) * K;
     double m = 0.0;
@@ -396,7 +449,9 @@ __global__ void sum_partials_kernel(const double *partials, int n, double *resul
 
 template <bool ACCUM, int TN>
 int attr_variants() {
-  DAGE_CUDA_TRY(cudaFuncSetAttribute(stage_fp64_kernel<ACCUM, TN>,
+  DAGE_CUDA_TRY(cudaFuncSetAttribute(stage_fp64_kernel<ACCUM, TN, false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, stage_smem<TN>()));
+  DAGE_CUDA_TRY(cudaFuncSetAttribute(stage_fp64_kernel<ACCUM, TN, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, stage_smem<TN>()));
   DAGE_CUDA_TRY(cudaFuncSetAttribute(stage_fp64_batched_kernel<ACCUM, TN>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, stage_smem<TN>()));
@@ -420,12 +475,16 @@ int prepare_fp64_stages() {
 }
 
 template <bool ACCUM, int TN>
-int launch_single(const StageDesc &d, double alpha, cudaStream_t s) {
-  auto kern = stage_fp64_kernel<ACCUM, TN>;
+int launch_single(const StageDesc &d, int p0, int np, bool sum, double alpha, cudaStream_t s) {
   DAGE_TRY(prepare_fp64_stages());
-  dim3 grid(ceil_div(d.M, BM), ceil_div(d.N, TN));
-  if (grid.y > 65535) return fail(DAGE_E_UNSUPPORTED, "N=%d too large", d.N);
-  kern<<<grid, 256, stage_smem<TN>(), s>>>(d, alpha);
+  const long long tiles = (long long)ceil_div(d.M, BM) * ceil_div(d.N, TN);
+  if (tiles >= (1LL << 31)) return fail(DAGE_E_UNSUPPORTED, "M=%d x N=%d too large", d.M, d.N);
+  if (sum)
+    stage_fp64_kernel<ACCUM, TN, true>
+        <<<(unsigned)tiles, 256, stage_smem<TN>(), s>>>(d, p0, np, alpha);
+  else
+    stage_fp64_kernel<ACCUM, TN, false>
+        <<<dim3((unsigned)tiles, np), 256, stage_smem<TN>(), s>>>(d, p0, np, alpha);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -435,19 +494,26 @@ int launch_batched(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, i
                    double alpha, cudaStream_t s) {
   auto kern = stage_fp64_batched_kernel<ACCUM, TN>;
   DAGE_TRY(prepare_fp64_stages());
-  dim3 grid(mtiles, ceil_div(ncols, TN), ndesc);
-  if (grid.y > 65535 || ndesc > 65535) return fail(DAGE_E_UNSUPPORTED, "batch too large");
-  kern<<<grid, 256, stage_smem<TN>(), s>>>(d_descs, p, alpha);
+  const int nt = ceil_div(ncols, TN);
+  if ((long long)mtiles * nt >= (1LL << 31) || ndesc > 65535)
+    return fail(DAGE_E_UNSUPPORTED, "batch too large");
+  kern<<<dim3(mtiles * nt, 1, ndesc), 256, stage_smem<TN>(), s>>>(d_descs, nt, p, alpha);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
 
-int launch_fp64_stage(const StageDesc &d, double alpha, bool accumulate, cudaStream_t s, int tn) {
+int launch_fp64_stage(const StageDesc &d, int p0, int np, bool sum, double alpha, bool accumulate,
+                      cudaStream_t s, int tn) {
+  if (np < 1 || np > kMaxPointGroup) return fail(DAGE_E_INVALID, "group of %d t-points", np);
+#define DAGE_SINGLE(TNV)                                                       \
+  return accumulate ? launch_single<true, TNV>(d, p0, np, sum, alpha, s)       \
+                    : launch_single<false, TNV>(d, p0, np, sum, alpha, s)
   switch (tn) {
-    case 32: return accumulate ? launch_single<true, 32>(d, alpha, s) : launch_single<false, 32>(d, alpha, s);
-    case 64: return accumulate ? launch_single<true, 64>(d, alpha, s) : launch_single<false, 64>(d, alpha, s);
-    case 128: return accumulate ? launch_single<true, 128>(d, alpha, s) : launch_single<false, 128>(d, alpha, s);
+    case 32: DAGE_SINGLE(32);
+    case 64: DAGE_SINGLE(64);
+    case 128: DAGE_SINGLE(128);
   }
+#undef DAGE_SINGLE
   return fail(DAGE_E_INVALID, "tile width %d", tn);
 }
 
@@ -469,12 +535,12 @@ int launch_fp64_stages(const StageDesc *d_descs, int ndesc, int mtiles, int ncol
 int launch_stage_fp64(const double *X, long long ldx, int M, int N, int K, const double *T,
                       long long ldt, double *out, double alpha, bool accumulate,
                       cudaStream_t s, const int2 *krange, int tn) {
-  return launch_fp64_stage(cube_stage(X, ldx, M, N, K, T, ldt, out, krange), alpha, accumulate, s,
-                           tn);
+  return launch_fp64_stage(cube_stage(X, ldx, M, N, K, T, ldt, out, krange), 0, 1, false, alpha,
+                           accumulate, s, tn);
 }
 
 int launch_band(const double *T, int K, int N, int P, int2 *range, cudaStream_t s) {
-  const int ntiles = ceil_div(N, BN);
+  const int ntiles = ceil_div(N, kBandCols);
   band_kernel<<<P * ntiles, 256, 0, s>>>(T, K, N, ntiles, range);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
@@ -703,7 +769,7 @@ static int build_matrices(dage_op3d *op, const char *cache_dir = nullptr) {
       DAGE_TRY(build_axis_matrix(ai, ao.points.data(), ao.n(), d_tp.as<double>(), op->P,
                                  op->Tbuf[d].as<double>(), s));
     }
-    DAGE_TRY(op->band[d].alloc(sizeof(int2) * (size_t)op->P * ceil_div(ao.n(), BN)));
+    DAGE_TRY(op->band[d].alloc(sizeof(int2) * (size_t)op->P * ceil_div(ao.n(), kBandCols)));
     DAGE_TRY(launch_band(op->Tbuf[d].as<double>(), ai.n(), ao.n(), op->P,
                          op->band[d].as<int2>(), s));
   }
@@ -787,8 +853,7 @@ static void destroy_impl(dage_op3d *op) {
   op->d_w.release();
   op->d_rho.release();
   op->d_V.release();
-  op->tmp1.release();
-  op->tmp2.release();
+  op->tmp.release();
   op->partials.release();
   if (op->pipe_in) cudaStreamSynchronize(op->pipe_in);
   if (op->pipe_out) cudaStreamSynchronize(op->pipe_out);
@@ -807,12 +872,70 @@ static void destroy_impl(dage_op3d *op) {
   delete op;
 }
 
+// t-points per launch of the FP64 path.  A small cube's stage has too few
+// tiles to fill the GPU and its launches cost more than its work (25^3: 5
+// tiles of 128 rows), so as many t-points share a launch as it takes for eight
+// blocks on every SM, and as fit a 96 MB intermediate (it then stays in the
+// 126 MB L2, and V is read and written once per group instead of once per
+// t-point).  The intermediates may take 1 GiB at most.
+static int fp64_group(const dage_op3d *op) {
+  const double niy = op->nin[1], niz = op->nin[2], nox = op->nout[0], noy = op->nout[1];
+  const double bytes = 8.0 * std::max(niy * niz * nox, niz * nox * noy);
+  const double tiles = std::ceil(std::min(niy * niz, niz * nox) / BM) * std::ceil(nox / 32);
+  const int fill = (int)std::ceil(8.0 * sm_count() / tiles);
+  const int l2 = (int)(96e6 / bytes);
+  const int most = std::min(kMaxPointGroup, (int)std::min(1e6, (double)(1 << 30) / (2 * bytes)));
+  return std::max(1, std::min({op->P, most, std::max(fill, l2)}));
+}
+
+// The intermediates of G t-points in one allocation (a first apply on a new
+// operator pays ~0.4 ms for each allocation above 1 MB): U, then W at nu.
+// Where a group does not fit the free memory it becomes a single t-point.
+static int fp64_workspace(const dage_op3d *op, DevBuf &buf, int &G, size_t &nu) {
+  const size_t niy = op->nin[1], niz = op->nin[2], nox = op->nout[0], noy = op->nout[1];
+  for (;;) {
+    nu = G * niy * niz * nox;
+    const int rc = buf.alloc(sizeof(double) * (nu + G * niz * nox * noy));
+    if (!rc || G == 1) return rc;
+    cudaGetLastError();
+    clear_error();
+    G = 1;
+  }
+}
+
+// The three stages of one group of t-points: every t-point's U and W in its
+// own slot (W carries the weight w_p), the last stage summed over the group.
+struct Fp64Stages {
+  StageDesc d[3];
+};
+static Fp64Stages fp64_stages(const dage_op3d *op, const double *rho, double *U, double *W,
+                              double *V) {
+  const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
+  const int nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
+  const int M[3] = {niy * niz, niz * nox, nox * noy}, N[3] = {nox, noy, noz},
+            K[3] = {nix, niy, niz};
+  const double *X[3] = {rho, U, W};
+  double *out[3] = {U, W, V};
+  Fp64Stages st;
+  for (int d = 0; d < 3; ++d) {
+    st.d[d] = cube_stage(X[d], K[d], M[d], N[d], K[d], op->T(d), K[d], out[d],
+                         op->band[op->Towner[d]].as<int2>());
+    st.d[d].t_ps = (long long)N[d] * K[d];
+    st.d[d].kr_ps = ceil_div(N[d], kBandCols);
+  }
+  const long long su = (long long)M[0] * N[0], sw = (long long)M[1] * N[1];
+  st.d[0].o_ps = st.d[1].x_ps = su;
+  st.d[1].o_ps = st.d[2].x_ps = sw;
+  st.d[1].wp = op->d_w.as<double>();
+  return st;
+}
+
 // Autotuner of the FP64 path: the tile width (32, 64 or 128 output columns)
-// of each stage, timed on the operator's own matrices at three t-points
-// (first, middle, last: the widest and narrowest bands) over scratch cubes;
-// keyed on (device, input and output points per axis, t-points) in the tune
-// cache.  Small cubes fill the GPU only with narrow tiles (121^3: 115 row
-// tiles of 128 for 148 SMs).
+// of each stage, timed on the operator's own matrices for the first, the
+// middle and the last group of t-points (the widest to the narrowest bands)
+// over scratch cubes; keyed on (device, input and output points per axis,
+// t-points) in the tune cache.  The width changes no arithmetic: every warp
+// sums its 32 columns over the same K in the same order.
 static int tune_fp64(dage_op3d *op) {
   std::string key = tune_device_key() + "/op3d_fp64/";
   for (int d = 0; d < 3; ++d) key += std::to_string(op->nin[d]) + "x" + std::to_string(op->nout[d]) + ",";
@@ -823,32 +946,28 @@ static int tune_fp64(dage_op3d *op) {
     return 0;
   }
   cudaStream_t s = op->stream;
-  const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
-  const int nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
-  TmpBuf X, U, W, V;
-  DAGE_TRY(X.alloc(sizeof(double) * (size_t)nix * niy * niz));
-  DAGE_TRY(U.alloc(sizeof(double) * (size_t)niy * niz * nox));
-  DAGE_TRY(W.alloc(sizeof(double) * (size_t)niz * nox * noy));
-  DAGE_TRY(V.alloc(sizeof(double) * (size_t)nox * noy * noz));
+  const size_t nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
+  const size_t nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
+  int G = fp64_group(op);
+  TmpBuf X, U, V;
+  size_t nu;
+  DAGE_TRY(X.alloc(sizeof(double) * nix * niy * niz));
+  DAGE_TRY(V.alloc(sizeof(double) * nox * noy * noz));
+  DAGE_TRY(fp64_workspace(op, U, G, nu));
   DAGE_CUDA_TRY(cudaMemsetAsync(X.ptr, 0, X.bytes, s));
   DAGE_CUDA_TRY(cudaMemsetAsync(U.ptr, 0, U.bytes, s));
-  DAGE_CUDA_TRY(cudaMemsetAsync(W.ptr, 0, W.bytes, s));
   cudaEvent_t e0, e1;
   DAGE_CUDA_TRY(cudaEventCreate(&e0));
   DAGE_CUDA_TRY(cudaEventCreate(&e1));
-  const size_t sT[3] = {(size_t)nox * nix, (size_t)noy * niy, (size_t)noz * niz};
-  const double *in[3] = {X.as<double>(), U.as<double>(), W.as<double>()};
-  double *outp[3] = {U.as<double>(), W.as<double>(), V.as<double>()};
-  const int M[3] = {niy * niz, niz * nox, nox * noy}, N[3] = {nox, noy, noz}, K[3] = {nix, niy, niz};
-  const int ps[3] = {0, op->P / 2, op->P - 1};
+  const Fp64Stages st = fp64_stages(op, X.as<double>(), U.as<double>(), U.as<double>() + nu, V.as<double>());
+  const int last = (op->P - 1) / G * G;
+  const int ps[3] = {0, last / G / 2 * G, last};
   int rc = 0;
   for (int d = 0; d < 3 && !rc; ++d) {
     float best = 1e30f;
     for (int tn : {32, 64, 128}) {
       auto run = [&](int p) {
-        const int2 *band = op->band[op->Towner[d]].as<int2>() + (size_t)p * ceil_div(N[d], BN);
-        return launch_stage_fp64(in[d], K[d], M[d], N[d], K[d], op->T(d) + sT[d] * p, K[d], outp[d],
-                                 1.0, false, s, band, tn);
+        return launch_fp64_stage(st.d[d], p, std::min(G, op->P - p), d == 2, 1.0, false, s, tn);
       };
       rc = run(ps[0]);  // warm-up
       if (!rc) rc = cudaEventRecord(e0, s) == cudaSuccess ? 0 : fail(DAGE_E_CUDA, "event");
@@ -873,29 +992,18 @@ static int tune_fp64(dage_op3d *op) {
 
 static int apply_fp64(dage_op3d *op, const double *rho, double *V, bool accumulate) {
   cudaStream_t s = op->stream;
-  const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
-  const int nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
-  DAGE_TRY(op->tmp1.alloc(sizeof(double) * (size_t)niy * niz * nox));
-  DAGE_TRY(op->tmp2.alloc(sizeof(double) * (size_t)niz * nox * noy));
-  double *U = op->tmp1.as<double>(), *W = op->tmp2.as<double>();
-  const size_t sx = (size_t)nox * nix, sy = (size_t)noy * niy, sz = (size_t)noz * niz;
-  auto band = [&](int d, int p) {
-    return op->band[op->Towner[d]].as<int2>() + (size_t)p * ceil_div(op->nout[d], BN);
-  };
-  for (int p = 0; p < op->P; ++p) {
-    int t = op->tmark_begin(0);
-    DAGE_TRY(launch_stage_fp64(rho, nix, niy * niz, nox, nix, op->T(0) + sx * p, nix, U, 1.0,
-                               false, s, band(0, p), op->tile_n[0]));
-    op->tmark_end(t);
-    t = op->tmark_begin(0);
-    DAGE_TRY(launch_stage_fp64(U, niy, niz * nox, noy, niy, op->T(1) + sy * p, niy, W, 1.0,
-                               false, s, band(1, p), op->tile_n[1]));
-    op->tmark_end(t);
-    t = op->tmark_begin(0);
-    DAGE_TRY(launch_stage_fp64(W, niz, nox * noy, noz, niz, op->T(2) + sz * p, niz, V,
-                               op->w[p], accumulate || p > 0, s, band(2, p), op->tile_n[2]));
-    op->tmark_end(t);
-  }
+  int G = fp64_group(op);
+  size_t nu;
+  DAGE_TRY(fp64_workspace(op, op->tmp, G, nu));
+  double *U = op->tmp.as<double>();
+  const Fp64Stages st = fp64_stages(op, rho, U, U + nu, V);
+  for (int p = 0; p < op->P; p += G)
+    for (int d = 0; d < 3; ++d) {
+      const int t = op->tmark_begin(0);
+      DAGE_TRY(launch_fp64_stage(st.d[d], p, std::min(G, op->P - p), d == 2, 1.0,
+                                 d == 2 && (accumulate || p > 0), s, op->tile_n[d]));
+      op->tmark_end(t);
+    }
   return 0;
 }
 

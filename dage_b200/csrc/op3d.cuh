@@ -25,7 +25,7 @@ struct dage_op3d {
   dage::DevBuf Tbuf[3];
   int Towner[3] = {0, 1, 2};
   // per axis owner: K band (first, last index, inclusive) of each t-point's
-  // 128-row tiles, int2[P][ceil(n_out / 128)]
+  // groups of kBandCols rows, int2[P][ceil(n_out / kBandCols)]
   dage::DevBuf band[3];
   const double *T(int axis) const { return Tbuf[Towner[axis]].as<double>(); }
 
@@ -33,7 +33,7 @@ struct dage_op3d {
   dage::DevBuf wts[3];
   dage::DevBuf d_w;          // weights w_p on the device
   dage::DevBuf d_rho, d_V;   // staging for host pointers
-  dage::DevBuf tmp1, tmp2;   // intermediates of the FP64 path
+  dage::DevBuf tmp;          // intermediates of the FP64 path, U then W
   dage::DevBuf partials;     // energy reduction partial sums
 
   // FP64 path: contraction tile width (32, 64 or 128 output columns) of each
@@ -74,12 +74,12 @@ namespace dage {
 
 // FP64 "contract the fastest index and rotate" stage:
 //   out[R + n*M] (= or +=) alpha * sum_K X[R*ldx + K] * T[n*ldt + K]
-// krange (optional): per 128-column tile of out, the K band [first, last].
+// krange (optional): per kBandCols columns of out, the K band [first, last].
 int launch_stage_fp64(const double *X, long long ldx, int M, int N, int K, const double *T,
                       long long ldt, double *out, double alpha, bool accumulate,
                       cudaStream_t s, const int2 *krange = nullptr, int tn = 128);
 
-// K band of every (t-point, 128-row tile) of an axis matrix T[p][n][K]: the
+// K band of every (t-point, kBandCols rows) of an axis matrix T[p][n][K]: the
 // first and last K index holding an entry above 2^-64 of its row's scale.
 int launch_band(const double *T, int K, int N, int P, int2 *range, cudaStream_t s);
 

@@ -71,6 +71,7 @@
 #include <string>
 #include <vector>
 
+#include "fp64_stage.cuh"
 #include "op3d.cuh"
 #include "tc_common.cuh"
 #include "tune.h"
@@ -233,7 +234,12 @@ __device__ __forceinline__ void corr_product(int nsx, int i, int &a, int &b) {
 
 // K blocks [first, last] of the band of sub-problem gi, n-tile nt
 __device__ __forceinline__ int2 kblocks(const StageArgs &a, int gi, int nt) {
-  const int2 r = a.k_range[gi * a.n_ntiles + nt];
+  const int ngr = (a.N + kBandCols - 1) / kBandCols;  // bands of one t-point
+  const int2 *b = a.k_range + gi * ngr + nt * (BN / kBandCols);
+  int2 r = b[0];
+#pragma unroll
+  for (int g = 1; g < BN / kBandCols; ++g)
+    if (nt * BN + g * kBandCols < a.N) r = make_int2(min(r.x, b[g].x), max(r.y, b[g].y));
   return make_int2(r.x / BK, r.y / BK);
 }
 
@@ -949,7 +955,7 @@ int run_stages(dage_op3d *op, MixedState &st, const double *d_rho, double *d_V, 
   auto common = [&](StageArgs &a, int stage, int p) {
     const int ow = st.towner[stage];
     a.scale = st.sc[ow].as<float>() + (size_t)p * no[stage];
-    a.k_range = op->band[ow].as<int2>() + (size_t)p * ceil_div(no[stage], BN);
+    a.k_range = op->band[ow].as<int2>() + (size_t)p * ceil_div(no[stage], kBandCols);
   };
   // last-stage input: slot p % G of X[2], parts stored [part][slot][rows][ld]
   auto slot_plane = [&](int part, int slot) {
