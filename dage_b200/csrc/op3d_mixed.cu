@@ -35,8 +35,13 @@
 // consecutive values of R mod d0 for one R / d0, so that every warp holds
 // exactly one 32-run and a warp-wide max reduction gives its quantum.  The
 // last stage multiplies by w_p s_n and adds into V (FP64) with L2
-// reductions; the sum over t-points is FP64.  K blocks outside the band of
-// the matrix tile (entries below 2^-64 of their row's scale) are skipped.
+// reductions; the sum over t-points is FP64.  The bands of the matrices are
+// kept per 32 columns: a K block multiplies only the columns from the first to
+// the last group whose band holds it (its window), and every epilogue warp
+// drains the partials of its own group only.  Outside the band entries are
+// below 2^-64 of their row's scale (fp16x3: both FP16 parts are zero, which
+// narrows the bands further and changes no bit).  At 481^3 the windows hold
+// 0.38 of the dense product (ranges per 128 columns: 0.53).
 //
 // "fp16x3" keeps the bf16x3 structure (two parts, three products, per-run
 // main-product partials) with FP16 parts: 11-bit significands give the two
@@ -52,8 +57,8 @@
 // the odd ones) before summing, which removes that bias.
 //
 // Kernel structure (one persistent CTA per SM, 18 warps):
-//   warp 0      TMA producer: X and T tiles -> shared-memory ring (SW64)
-//   warp 1      TMEM allocator + single-thread MMA issuer
+//   warp 0      producer: bulk copies of X and T tiles -> shared-memory ring
+//   warp 1      TMEM allocator + MMA issuer (one elected lane)
 //   warps 2-17  epilogue, four warps per scheduler (32 columns each):
 //               partial sums -> scale -> split -> global stores
 // TMEM holds three 128-column partial buffers (the MMAs of the next slices
@@ -131,26 +136,29 @@ __device__ __forceinline__ __nv_bfloat162 f32x2_to_bf16x2_exact(float2 v) {
 
 
 
-// The same split for two values sharing one run maximum m, on packed FP32x2
-// arithmetic; part s of (v.x, v.y) lands in o[s] as a BF16 pair.
+// The same split for two values of two runs with the maxima m, on packed
+// FP32x2 arithmetic; part s of (v.x, v.y) lands in o[s] as a BF16 pair.
 template <int NS>
-__device__ __forceinline__ void split_pair_f32(float2 v, float m, __nv_bfloat162 (&o)[NS]) {
+__device__ __forceinline__ void split_pair_f32(float2 v, float2 m, __nv_bfloat162 (&o)[NS]) {
   const float2 neg1 = make_float2(-1.0f, -1.0f);
   float2 l;
   if (NS == 2) {
     o[0] = __floats2bfloat162_rn(v.x, v.y);
     l = bf16x2_to_f32x2(o[0]);
   } else {
-    const uint32_t mb = __float_as_uint(m);
-    const int E = (int)((mb >> 23) & 0xff) - 127 + ((mb & 0x7fffff) != 0);
-    if (m == 0.0f || E < -119) {
-      l = make_float2(0.0f, 0.0f);
-    } else {
-      const float up = __uint_as_float((uint32_t)(127 + 7 - E) << 23);    // 2^(7-E)
-      const float down = __uint_as_float((uint32_t)(127 - 7 + E) << 23);  // 2^(E-7)
-      const float2 t = __fmul2_rn(v, make_float2(up, up));
-      l = __fmul2_rn(make_float2(rintf(t.x), rintf(t.y)), make_float2(down, down));
-    }
+    // 2^(7-E) and 2^(E-7), zeros below E = -119
+    auto scales = [](float mm, float &up, float &down) {
+      const uint32_t mb = __float_as_uint(mm);
+      const int E = (int)((mb >> 23) & 0xff) - 127 + ((mb & 0x7fffff) != 0);
+      const bool none = mm == 0.0f || E < -119;
+      up = none ? 0.0f : __uint_as_float((uint32_t)(127 + 7 - E) << 23);
+      down = none ? 0.0f : __uint_as_float((uint32_t)(127 - 7 + E) << 23);
+    };
+    float2 up, down;
+    scales(m.x, up.x, down.x);
+    scales(m.y, up.y, down.y);
+    const float2 t = __fmul2_rn(v, up);
+    l = __fmul2_rn(make_float2(rintf(t.x), rintf(t.y)), down);
     o[0] = f32x2_to_bf16x2_exact(l);  // an 8-bit integer times a power of two
   }
   float2 r = __ffma2_rn(l, neg1, v);  // v - lead, exact
@@ -162,39 +170,75 @@ __device__ __forceinline__ void split_pair_f32(float2 v, float m, __nv_bfloat162
 }
 
 // ---------------------------------------------------------------------------
+// Operand layout
+// ---------------------------------------------------------------------------
+// Both operands live in global memory in the order the tensor core wants them
+// in shared memory, so that a tile is one contiguous piece and arrives by one
+// plain bulk copy.  The unit is an atom of 8 rows x 32 K: per part 8 rows of 64
+// bytes with their 16-byte chunks permuted as the 64-byte swizzle does, the
+// NSX parts one after another.  A stage input is [outer][K block][row atom],
+// "rows" the fast index of the stage's row pair (R = outer * d0 + row), a
+// matrix [t-point][K block][row atom].  Tensor-map copies of 128 rows of 64
+// bytes move 22 B/cycle per SM whatever the source; bulk copies of 16 KB moved
+// 54 (L2-resident source, 148 SMs at once: 15.4 TB/s), 8 KB 43, 32 KB 61.
+// With the column windows below and a warp-uniform MMA issue loop, 481^3
+// fp16x3 takes 45.3 ms per apply (67.0 before), 253^3 bf16x6 10.1 (11.6).
+constexpr int kAtomRows = 8;
+template <int NSX>
+constexpr int atom_bytes() {
+  return NSX * kAtomRows * BK * 2;
+}
+// element (row, k) of part s inside its atom, in elements
+__host__ __device__ __forceinline__ int atom_off(int row, int k, int s) {
+  const int r = row & 7;
+  return s * kAtomRows * BK + r * BK + ((((k >> 3) & 3) ^ (r >> 1)) << 3) + (k & 7);
+}
+
+// ---------------------------------------------------------------------------
 // Stage kernel
 // ---------------------------------------------------------------------------
+// The K blocks of one (t-point, n-tile) that the bands of its four 32-column
+// groups touch ("runs"), as a list ended by kRunEnd:
+//   bits 0-15 K block, 16-19 groups inside their band, 20-21 the first of the
+//   groups from the first to the last such one (the run's window), 22-24 their
+//   number.
+// Every role of the kernel walks the same list; it is built with the operator
+// so that none of them spends instructions on the bands.
+constexpr uint32_t kRunEnd = 0xffffffffu;
+__device__ __forceinline__ int run_block(uint32_t w) { return w & 0xffff; }
+__device__ __forceinline__ int run_first(uint32_t w) { return (w >> 20) & 3; }
+__device__ __forceinline__ int run_groups(uint32_t w) { return (w >> 22) & 7; }
+
 struct StageArgs {
-  int M, N, K;           // D is M x N, contraction length K
+  int N;                 // output columns
   int n_ntiles, ntiles;  // tiles: m-tile major, n-tile minor
-  int nkb, last_k16;     // K blocks; MMAs of K=16 in the last block
-  int brow0;             // first row of this t-point in the T-part maps
-  // M tiling: nrb == 0: tile mt covers rows [128 mt, 128 mt + 128);
-  // nrb > 0 (intermediate stages): tile mt covers R = r1 d0 + r0 with
-  // r1 = mt / nrb and r0 in [128 (mt % nrb), +128) intersected with [0, d0)
-  int nrb;
-  // Sub-problems per tile: the last stage sums ng t-points p0 .. p0+ng-1 in
-  // one pass over V; sub-problem g reads A rows from g * gM, matrix rows
-  // from brow0 + g * N, bands k_range[g * n_ntiles + nt], scales
-  // scale[g * N + n] and weight wcoef[g].  Intermediate stages: ng = 1.
-  int ng, gM;
-  const float *scale;    // s_n, row scales of the t-points
+  // rows: tile mt covers rows [128 (mt % nrb), +128) of the d0 rows of outer
+  // index mt / nrb
+  int nrb, d0, outer;
+  int nkb, natA, natB;   // K blocks, row atoms of the input and of the matrix
+  const uint8_t *X, *T;  // operands (T: of the first t-point)
+  // Sub-problems per tile: the last stage sums ng t-points in one pass over V;
+  // sub-problem g reads outer index + g * outer, the g-th matrix, the run list
+  // at runs + (g * n_ntiles + nt) (nkb + 1), scales scale[g * N + n] and weight
+  // wcoef[g].
+  // Intermediate stages: ng = 1.
+  int ng;
+  const float *scale;    // s_n, row scales of the t-points (bf16x6)
   const float *wcoef;    // w_p of the t-points (device)
   // FP16 intermediate stages: the stage's power-of-two output factor (device
   // scalar, from the bound-based input scales); null for the BF16 modes
   const float *gscale;
-  // intermediate output: part s of element (R, n) at
-  //   out[s][(R / d0 + d1 * n) * ldn + R % d0]
-  __nv_bfloat16 *out0, *out1, *out2;  // FP16 mode: the same bytes as __half
-  int d0, d1;
-  long long ldn;
-  // final output V[R + M * n] (FP64)
+  // intermediate output: the next stage's input, whose rows are this stage's
+  // outer index, whose K is this stage's row and whose outer index is n
+  __nv_bfloat16 *out;    // FP16 mode: the same bytes as __half
+  int nkbN, natN;
+  // final output V[row + d0 * outer index + vn * n] (FP64)
   double *V;
+  long long vn;
   int accumulate;
-  // per t-point and n-tile: first and last K index holding a matrix entry
-  // above 2^-64 of its row's scale (the matrices are banded for large t; K
-  // blocks outside the band add nothing and are skipped)
-  const int2 *k_range;
+  // the matrices are banded for large t; K blocks outside a group's band add
+  // nothing and are skipped, column groups outside it too
+  const uint32_t *runs;
   int *err;
   long long wait_limit;   // normal waits (dage_set_wait_limit)
   long long drain_limit;  // waits for in-flight copies/MMAs after a timeout
@@ -202,10 +246,9 @@ struct StageArgs {
 
 template <int NSX, int NS, bool F16 = false>
 struct StageCfg {
-  static constexpr int kRowBytes = BK * 2;
-  static constexpr int kABytes = BM * kRowBytes;  // one part of the A tile
-  static constexpr int kBBytes = BN * kRowBytes;  // one part of the B tile
-  static constexpr int kStageBytes = NSX * kABytes + NSX * kBBytes;
+  static constexpr int kAtom = atom_bytes<NSX>();
+  static constexpr int kABytes = BM / kAtomRows * kAtom;  // all parts of the A tile
+  static constexpr int kStageBytes = 2 * kABytes;         // A and B tiles
   // fp16x3 folds its correction products into each 32-run's partial (issued
   // before the main product, so their truncations happen at the corrections'
   // scale, 2^-11 below it): four partial buffers, no correction accumulator
@@ -232,46 +275,50 @@ __device__ __forceinline__ void corr_product(int nsx, int i, int &a, int &b) {
   }
 }
 
-// K blocks [first, last] of the band of sub-problem gi, n-tile nt
-__device__ __forceinline__ int2 kblocks(const StageArgs &a, int gi, int nt) {
-  const int ngr = (a.N + kBandCols - 1) / kBandCols;  // bands of one t-point
-  const int2 *b = a.k_range + gi * ngr + nt * (BN / kBandCols);
-  int2 r = b[0];
-#pragma unroll
-  for (int g = 1; g < BN / kBandCols; ++g)
-    if (nt * BN + g * kBandCols < a.N) r = make_int2(min(r.x, b[g].x), max(r.y, b[g].y));
-  return make_int2(r.x / BK, r.y / BK);
-}
+// The tiles of one CTA, blockIdx.x + i gridDim.x, as (n-tile, row block, outer
+// index): the decoding divides once, then adds with carries.
+struct TileWalk {
+  int nt, rb, r1, left;
+  int dnt, drb, dr1;
+  __device__ __forceinline__ explicit TileWalk(const StageArgs &a) {
+    split(a, blockIdx.x, nt, rb, r1);
+    split(a, gridDim.x, dnt, drb, dr1);
+    left = (a.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;  // grid <= ntiles
+  }
+  __device__ static void split(const StageArgs &a, int t, int &n, int &b, int &o) {
+    n = t % a.n_ntiles;
+    b = t / a.n_ntiles % a.nrb;
+    o = t / a.n_ntiles / a.nrb;
+  }
+  __device__ __forceinline__ void next(const StageArgs &a) {
+    --left;
+    nt += dnt;
+    rb += drb;
+    r1 += dr1;
+    if (nt >= a.n_ntiles) nt -= a.n_ntiles, ++rb;
+    if (rb >= a.nrb) rb -= a.nrb, ++r1;
+  }
+};
 
-__device__ __forceinline__ int tile_row0(const StageArgs &a, int mt) {
-  return a.nrb ? (mt / a.nrb) * a.d0 + (mt % a.nrb) * BM : mt * BM;
-}
-
-// The MMAs of one 32-run of K (d0: the run's first K column in the stage):
-// the main product (part 0 x part 0) into the fresh partial P, committed to
-// `pfull` as soon as it is issued, and the correction products into the
-// accumulator Cc.  NK K=16 steps; FIRST: the tile's first run (the
-// correction accumulator starts).
-template <int NSX, int NK, bool FIRST = false>
-__device__ __forceinline__ void mma_run(uint32_t P, uint32_t Cc, uint64_t d0, uint32_t idesc,
-                                           bool first, uint32_t pfull_bar) {
-  constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;  // one part of a tile
+// The MMAs of one 32-run of K for the columns of one window: the main product
+// (part 0 x part 0) into the fresh partial P, committed to `pfull` as soon as
+// it is issued, and the correction products into the accumulator Cc (which the
+// epilogue leaves at zero: the columns of a tile enter at different runs).
+template <int NSX>
+__device__ __forceinline__ void mma_run(uint32_t P, uint32_t Cc, uint64_t da, uint64_t db,
+                                        uint32_t idesc, uint32_t pfull_bar) {
+  constexpr int kPart = kAtomRows * BK * 2;
   constexpr int NCORR = NSX == 2 ? 2 : 5;
 #pragma unroll
-  for (int k = 0; k < NK; ++k) {
-    umma_bf16_c(P, d0 + ((k * 32) >> 4), d0 + ((NSX * kABytes + k * 32) >> 4), idesc, k != 0);
-    if (k == NK - 1) umma_commit(pfull_bar);
+  for (int k = 0; k < 2; ++k) {
+    umma_bf16_c(P, da + ((k * 32) >> 4), db + ((k * 32) >> 4), idesc, k != 0);
+    if (k == 1) umma_commit(pfull_bar);
 #pragma unroll
     for (int pr = 0; pr < NCORR; ++pr) {
       int ia, ib;
       corr_product(NSX, pr, ia, ib);
-      const uint64_t ad = d0 + ((ia * kABytes + k * 32) >> 4);
-      const uint64_t bd = d0 + ((NSX * kABytes + ib * kBBytes + k * 32) >> 4);
-      if (NK == 1) {
-        umma_bf16(Cc, ad, bd, idesc, (!first || pr != 0) ? 1u : 0u);
-      } else {
-        umma_bf16_c(Cc, ad, bd, idesc, !(FIRST && k == 0 && pr == 0));
-      }
+      umma_bf16_c(Cc, da + ((ia * kPart + k * 32) >> 4), db + ((ib * kPart + k * 32) >> 4), idesc,
+                  true);
     }
   }
 }
@@ -282,36 +329,98 @@ __device__ __forceinline__ void mma_run(uint32_t P, uint32_t Cc, uint64_t d0, ui
 // every accumulation; the corrections' truncations are ~2^-11 of the main
 // product's ulp, so the partial carries the same directed rounding as a
 // main-product-only partial (two truncations at its own scale).
-template <int NK>
-__device__ __forceinline__ void fold_run(uint32_t P, uint64_t d0, uint32_t idesc,
+__device__ __forceinline__ void fold_run(uint32_t P, uint64_t da, uint64_t db, uint32_t idesc,
                                          uint32_t pfull_bar) {
-  constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;
+  constexpr int kPart = kAtomRows * BK * 2;
 #pragma unroll
-  for (int k = 0; k < NK; ++k) {
-    umma_bf16_c(P, d0 + ((kABytes + k * 32) >> 4), d0 + ((2 * kABytes + k * 32) >> 4), idesc,
-                k != 0);
-    umma_bf16_c(P, d0 + ((k * 32) >> 4), d0 + ((2 * kABytes + kBBytes + k * 32) >> 4), idesc,
-                true);
+  for (int k = 0; k < 2; ++k) {
+    umma_bf16_c(P, da + ((kPart + k * 32) >> 4), db + ((k * 32) >> 4), idesc, k != 0);
+    umma_bf16_c(P, da + ((k * 32) >> 4), db + ((kPart + k * 32) >> 4), idesc, true);
   }
 #pragma unroll
-  for (int k = 0; k < NK; ++k)
-    umma_bf16_c(P, d0 + ((k * 32) >> 4), d0 + ((2 * kABytes + k * 32) >> 4), idesc, true);
+  for (int k = 0; k < 2; ++k)
+    umma_bf16_c(P, da + ((k * 32) >> 4), db + ((k * 32) >> 4), idesc, true);
   umma_commit(pfull_bar);
 }
 
-// NSX parts per operand; NS shared-memory stages; the main product starts a
-// fresh partial every kGroup / 16 MMAs (one 32-run of K).
-// 576 threads x 96 registers (55296 of the SM's 65536): one CTA per SM.
+// acc += 32 columns of a partial, FP16 with the toward-zero correction; WIDE:
+// one 32-register load (the last stage, with two sets of sums, has registers
+// for 16 at a time).
+template <bool F16, bool WIDE>
+__device__ __forceinline__ void drain32(uint32_t taddr, float2 (&acc)[16]) {
+  constexpr int W = WIDE ? 32 : 16;
+#pragma unroll
+  for (int h = 0; h < 32 / W; ++h) {
+    uint32_t r[W];
+    if constexpr (WIDE)
+      tmem_ld32(taddr, r);
+    else
+      tmem_ld16(taddr + h * W, r);
+#pragma unroll
+    for (int j = 0; j < W / 2; ++j) {
+      float2 pv = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+      if (F16) pv = make_float2(unbias_rz(pv.x), unbias_rz(pv.y));
+      acc[h * (W / 2) + j] = __fadd2_rn(acc[h * (W / 2) + j], pv);
+    }
+  }
+}
+
+// A warp's 32 columns (rows = lanes) into the next stage's input, see the
+// epilogue.  FULL: all 32 columns exist (else the first nv).
+template <int NSX, bool F16, bool COLSCALE, bool FULL>
+__device__ __forceinline__ void store_columns(const float2 (&acc)[16], float gfac, float scl,
+                                              __nv_bfloat16 *dst, size_t nstep, bool odd, bool live,
+                                              int nv) {
+  constexpr int kPart = kAtomRows * BK;
+  const uint32_t sel = odd ? 0x3276u : 0x5410u;  // (received high, own high) : (own low, received low)
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    if (!FULL && j >= nv) break;  // uniform across the warp
+    // The warp's 32 column scales are one per lane (scl, loaded at the
+    // tile's start): loads placed between the loop's global stores could
+    // not be moved ahead of them (the compiler cannot rule out aliasing),
+    // and each would expose its full latency.
+    const float2 sc = COLSCALE ? make_float2(__shfl_sync(0xffffffffu, scl, j),
+                                             __shfl_sync(0xffffffffu, scl, j + 1))
+                               : make_float2(gfac, gfac);
+    const float2 v = (COLSCALE || F16) ? __fmul2_rn(acc[j >> 1], sc) : acc[j >> 1];
+    uint32_t o[NSX];
+    if (F16) {
+      __half2 h[2];
+      split_pair_f16(v, h);
+      o[0] = *reinterpret_cast<uint32_t *>(&h[0]);
+      o[1] = *reinterpret_cast<uint32_t *>(&h[1]);
+    } else {
+      float2 m = make_float2(0.0f, 0.0f);
+      if (NSX > 2) {
+        // largest |value| of the run per column; lanes that store nothing hold
+        // no part of it
+        const uint32_t keep = live ? 0x7fffffffu : 0u;
+        m.x = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.x) & keep));
+        m.y = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.y) & keep));
+      }
+      __nv_bfloat162 p[NSX];
+      split_pair_f32<NSX>(v, m, p);
+#pragma unroll
+      for (int s = 0; s < NSX; ++s) o[s] = *reinterpret_cast<uint32_t *>(&p[s]);
+    }
+    const bool store = live && (FULL || !odd || j + 1 < nv);
+#pragma unroll
+    for (int s = 0; s < NSX; ++s) {
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, o[s], 1);
+      const uint32_t pair = __byte_perm(o[s], other, sel);
+      if (store) *reinterpret_cast<uint32_t *>(dst + s * kPart) = pair;
+    }
+    dst += 2 * nstep;
+  }
+}
+
+// NSX parts per operand; NS shared-memory stages of one K block each.
+// 576 threads x 96 registers (five warps of 18 share a scheduler and its 16384
+// registers): one CTA per SM.
 template <int NSX, int NS, bool FINAL, bool F16 = false>
-__global__ void __maxnreg__(96)
-    stage_bf16_kernel(const __grid_constant__ CUtensorMap mapA0,
-                      const __grid_constant__ CUtensorMap mapA1,
-                      const __grid_constant__ CUtensorMap mapA2,
-                      const __grid_constant__ CUtensorMap mapB0,
-                      const __grid_constant__ CUtensorMap mapB1,
-                      const __grid_constant__ CUtensorMap mapB2, const StageArgs a) {
+__global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageArgs a) {
   using C = StageCfg<NSX, NS, F16>;
-  constexpr int GRAN = kGroup / 16;
   // an earlier launch of this apply timed out: do nothing
   if (*reinterpret_cast<volatile int *>(a.err)) return;
   extern __shared__ uint8_t smem_raw[];
@@ -358,44 +467,41 @@ __global__ void __maxnreg__(96)
     *abort_flag = 1;
     atomicCAS(a.err, 0, 1);
   };
-  // K=16 steps of a tile with K blocks [lo, hi]
-  auto tile_steps = [&](int2 r) {
-    return (r.y - r.x) * (BK / 16) + (r.y == a.nkb - 1 ? a.last_k16 : BK / 16);
-  };
+  auto run_list = [&](int gi, int nt) { return a.runs + (size_t)(gi * a.n_ntiles + nt) * (a.nkb + 1); };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
-      const CUtensorMap *mA[3] = {&mapA0, &mapA1, &mapA2};
-      const CUtensorMap *mB[3] = {&mapB0, &mapB1, &mapB2};
       int s = 0;
       uint32_t ph = 0;
       int issued[NS];
       uint32_t issued_ph[NS];
       for (int i = 0; i < NS; ++i) issued[i] = 0, issued_ph[i] = 0;
-      for (int u = blockIdx.x * a.ng; u < a.ntiles * a.ng && !*abort_flag;
-           u += (u % a.ng == a.ng - 1) ? (gridDim.x - 1) * a.ng + 1 : 1) {
-        const int tile = u / a.ng, gi = u % a.ng;
-        const int row0 = tile_row0(a, tile / a.n_ntiles) + gi * a.gM;
-        const int n0 = (tile % a.n_ntiles) * BN + gi * a.N;
-        const int2 r = kblocks(a, gi, tile % a.n_ntiles);
-        for (int kb = r.x; kb <= r.y; ++kb) {
-          if (!mbar_wait(empty(s), ph ^ 1, a.wait_limit)) {
-            on_timeout();
-            break;
+      for (TileWalk t(a); t.left > 0 && !*abort_flag; t.next(a)) {
+        const uint32_t abytes = min(16, a.natA - 16 * t.rb) * C::kAtom;
+        const int bmost = a.natB - 16 * t.nt;  // row atoms of the matrix from this n-tile on
+        for (int gi = 0; gi < a.ng; ++gi) {
+          const uint8_t *xa = a.X + ((size_t)(t.r1 + gi * a.outer) * a.nkb * a.natA + 16 * t.rb) * C::kAtom;
+          const uint8_t *tb = a.T + ((size_t)gi * a.nkb * a.natB + 16 * t.nt) * C::kAtom;
+          const uint32_t *rw = run_list(gi, t.nt);
+          for (uint32_t w = __ldg(rw), wn; w != kRunEnd; w = wn) {
+            wn = __ldg(++rw);
+            const int kb = run_block(w), g0 = run_first(w);
+            if (!mbar_wait(empty(s), ph ^ 1, a.wait_limit)) {
+              on_timeout();
+              break;
+            }
+            const uint32_t st = smem_u32(tiles + s * C::kStageBytes);
+            const uint32_t bbytes = min(4 * run_groups(w), bmost - 4 * g0) * C::kAtom;
+            mbar_expect_tx(full(s), abytes + bbytes);
+            bulk_load(st, xa + (size_t)kb * a.natA * C::kAtom, abytes, full(s));
+            bulk_load(st + C::kABytes + 4 * g0 * C::kAtom,
+                      tb + ((size_t)kb * a.natB + 4 * g0) * C::kAtom, bbytes, full(s));
+            issued[s] = 1;
+            issued_ph[s] = ph;
+            if (++s == NS) s = 0, ph ^= 1;
           }
-          uint8_t *st = tiles + s * C::kStageBytes;
-          mbar_expect_tx(full(s), C::kStageBytes);
-#pragma unroll
-          for (int i = 0; i < NSX; ++i)
-            tma_load_2d(smem_u32(st + i * C::kABytes), mA[i], full(s), kb * BK, row0);
-#pragma unroll
-          for (int j = 0; j < NSX; ++j)
-            tma_load_2d(smem_u32(st + NSX * C::kABytes + j * C::kBBytes), mB[j], full(s),
-                        kb * BK, a.brow0 + n0);
-          issued[s] = 1;
-          issued_ph[s] = ph;
-          if (++s == NS) s = 0, ph ^= 1;
+          if (*abort_flag) break;
         }
       }
       if (*abort_flag)  // let every copy that was issued land first
@@ -407,80 +513,80 @@ __global__ void __maxnreg__(96)
     // The tensor core runs these MMAs back to back only if the issuing
     // thread spends almost nothing between them (a 128x128x16 MMA is 64
     // cycles): every K block is straight-line code with compile-time
-    // operand offsets and accumulate flags.
-    if (lane == 0) {
+    // operand offsets and accumulate flags.  The whole warp walks the loop
+    // with warp-uniform values and one elected lane issues, so that the
+    // descriptors stay in uniform registers: issued by a lane of a divergent
+    // branch, each MMA first moved them there, ~1000 cycles a run.
+    {
+      const bool leader = elect_one();
       int s = 0;
       uint32_t ph = 0;
       int b = 0;            // partial buffer of the current K block (one 32-run)
       uint32_t pph = 0;     // phase of the partial buffers' current round
-      int t = 0;
+      uint32_t tph = 0;     // phase of the tile (sub-problem)
       bool ok = true;
-      const uint64_t dbase = sdesc(smem_u32(tiles));
-      int u = blockIdx.x * a.ng;
-      int2 r = u < a.ntiles * a.ng ? kblocks(a, u % a.ng, (u / a.ng) % a.n_ntiles) : make_int2(0, -1);
-      for (; u < a.ntiles * a.ng && ok && !*abort_flag; ++t) {
-        const int tile = u / a.ng;
-        const int n0 = (tile % a.n_ntiles) * BN;
-        int nt = a.N - n0;
-        if (nt > BN) nt = BN;
-        nt = (nt + 15) & ~15;
-        const uint32_t idesc = idesc_f16kind<F16>(BM, nt);
-        const int2 rc = r;
-        // next tile's band, loaded while this tile's MMAs run
-        u += (u % a.ng == a.ng - 1) ? (gridDim.x - 1) * a.ng + 1 : 1;
-        if (u < a.ntiles * a.ng) r = kblocks(a, u % a.ng, (u / a.ng) % a.n_ntiles);
-        for (int kb = rc.x; kb <= rc.y; ++kb) {
-          const bool first = kb == rc.x;
-          if (!mbar_wait(full(s), ph, a.wait_limit) ||
-              (!FOLD && first && !mbar_wait(cempty, (t & 1) ^ 1, a.wait_limit))) {
-            on_timeout();
+      const uint64_t dbase = sdesc64(smem_u32(tiles), C::kAtom);
+      uint64_t da = dbase;
+      constexpr uint32_t kIdesc = idesc_f16kind<F16>(BM, 0);
+      TileWalk t(a);
+      const uint32_t *rw = run_list(0, t.nt);
+      uint32_t w = __shfl_sync(0xffffffffu, __ldg(rw), 0);
+      while (t.left > 0 && ok && !*abort_flag) {
+        for (int gi = 0; gi < a.ng && ok; ++gi) {
+          // the first run of the next sub-problem, loaded while this one's MMAs run
+          if (gi == a.ng - 1) t.next(a);
+          const uint32_t *rnext = run_list(gi == a.ng - 1 ? 0 : gi + 1, t.nt);
+          const uint32_t wfirst = __ldg(rnext);
+          if (!FOLD && !mbar_wait_warp(cempty, tph, a.wait_limit)) {
+            if (leader) on_timeout();
             ok = false;
             break;
           }
-          tc_fence_after();
-          const uint64_t d0 = dbase + (uint64_t)((s * C::kStageBytes) >> 4);
-          const int nk16 = (kb == a.nkb - 1) ? a.last_k16 : BK / 16;
-#pragma unroll
-          for (int rr = 0; rr < BK / kGroup; ++rr) {
-            const int nk = min(nk16 - rr * GRAN, GRAN);  // K=16 steps of this run
-            if (nk <= 0) break;
-            if (!mbar_wait(pempty(b), pph ^ 1, a.wait_limit)) {
-              on_timeout();
+          while (w != kRunEnd) {
+            const uint32_t wn = __ldg(++rw);
+            const int g0 = run_first(w);
+            const uint32_t idesc = kIdesc | ((uint32_t)(4 * run_groups(w)) << 17);
+            const uint64_t db = da + (uint64_t)(C::kABytes >> 4) + (uint64_t)(g0 * ((4 * C::kAtom) >> 4));
+            const uint32_t P = tmem_base + b * BN + 32 * g0;
+            if (!mbar_wait_warp(pempty(b), pph ^ 1, a.wait_limit) ||
+                !mbar_wait_warp(full(s), ph, a.wait_limit)) {
+              if (leader) on_timeout();
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint64_t dr = d0 + (uint64_t)((rr * kGroup * 2) >> 4);
-            const uint32_t P = tmem_base + b * BN;
-            if (FOLD) {
-              if (nk == 1)
-                fold_run<1>(P, dr, idesc, pfull(b));
+            if (leader) {
+              if (FOLD)
+                fold_run(P, da, db, idesc, pfull(b));
               else
-                fold_run<2>(P, dr, idesc, pfull(b));
-            } else if (nk == 1) {
-              mma_run<NSX, 1>(P, tmem_corr, dr, idesc, first && rr == 0, pfull(b));
-            } else if (first && rr == 0) {
-              mma_run<NSX, 2, true>(P, tmem_corr, dr, idesc, true, pfull(b));
-            } else {
-              mma_run<NSX, 2, false>(P, tmem_corr, dr, idesc, false, pfull(b));
+                mma_run<NSX>(P, tmem_corr + 32 * g0, da, db, idesc, pfull(b));
+              umma_commit(empty(s));
             }
+            __syncwarp();
             if (++b == C::kNP) b = 0, pph ^= 1;
+            da += (uint64_t)(C::kStageBytes >> 4);
+            if (++s == NS) s = 0, ph ^= 1, da = dbase;
+            w = __shfl_sync(0xffffffffu, wn, 0);
           }
-          if (!ok) break;
-          umma_commit(empty(s));
-          if (++s == NS) s = 0, ph ^= 1;
+          if (ok && !FOLD && leader) umma_commit(cfull);
+          __syncwarp();
+          tph ^= 1;
+          rw = rnext;
+          w = __shfl_sync(0xffffffffu, wfirst, 0);
         }
-        if (ok && !FOLD) umma_commit(cfull);
       }
-      // every MMA this thread issued has completed once `drain` fires
-      umma_commit(drain);
+      // every MMA this warp issued has completed once `drain` fires
+      if (leader) umma_commit(drain);
+      __syncwarp();
       mbar_wait(drain, 0, a.drain_limit);
     }
   } else {
     // ------------------------------------------------------------ epilogue
     // 16 warps, four per scheduler: warp w reads TMEM lanes 32 (w % 4) ..
-    // +31 (the hardware's lane quarter) and the 32 columns (w - 2) / 4.
+    // +31 (the hardware's lane quarter) and the 32 columns (w - 2) / 4, one
+    // column group of the band: it drains the partials of its own band only.
     constexpr int CW = BN / 4;
+    static_assert(CW == kBandCols, "a warp's columns are one band group");
     // Per-column matrix scales matter only for bf16x6 (fixed-point matrix
     // leads on a per-row quantum); bf16x3 splits the unscaled matrix and
     // fp16x3 scales each t-point's matrix by one power of two, folded into
@@ -489,69 +595,67 @@ __global__ void __maxnreg__(96)
     const float gfac = (F16 && !FINAL) ? *a.gscale : 1.0f;
     const int q = warp & 3;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
-    const uint32_t col0 = ((warp - 2) >> 2) * CW;
-    int g = 0, t = 0;
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+    const int grp = (warp - 2) >> 2;
+    const uint32_t col0 = grp * CW;
+    if (!FOLD) {  // the correction accumulator starts at zero
+      tmem_zero16(tmem_corr + lane_off + col0);
+      tmem_zero16(tmem_corr + lane_off + col0 + 16);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(cempty);
+    }
+    int b = 0;
+    uint32_t pph = 0, tph = 0;
+    const uint32_t mymask = 0x10000u << grp;
+    const uint32_t taddr = tmem_base + lane_off + col0;
+    for (TileWalk t(a); t.left > 0; t.next(a)) {
       float2 acc[CW / 2];   // one t-point, columns (2j, 2j + 1)
       float2 accg[CW / 2];  // last stage: sum over the group of w_p s_n D_p
 #pragma unroll
       for (int j = 0; j < CW / 2; ++j) accg[j] = make_float2(0.0f, 0.0f);
       bool ok = true;
-      const int ncol = (tile % a.n_ntiles) * BN + col0 + lane;  // this lane's column
+      const int n0 = t.nt * BN + col0;
+      const int ncol = n0 + lane;  // this lane's column
       // intermediate stages: the scale of column ncol, loaded before the
       // partial drains so its latency overlaps them
       const float scl = (!FINAL && kColScale && ncol < a.N) ? a.scale[ncol] : 0.0f;
-      for (int gi = 0; gi < a.ng && ok; ++gi, ++t) {
-        // last stage: w_p s_n of column ncol for sub-problem gi
-        const float fcol = (FINAL && ncol < a.N) ? a.wcoef[gi] * a.scale[(size_t)gi * a.N + ncol] : 0.0f;
+      for (int gi = 0; gi < a.ng && ok; ++gi) {
+        const uint32_t *rw = run_list(gi, t.nt);
+        uint32_t w = __ldg(rw);
+        // last stage: w_p [s_n of column ncol] for sub-problem gi
+        float fcol = FINAL ? a.wcoef[gi] : 0.0f;
+        if (FINAL && kColScale) fcol = ncol < a.N ? fcol * a.scale[(size_t)gi * a.N + ncol] : 0.0f;
 #pragma unroll
         for (int j = 0; j < CW / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
-        const int nparts =
-            (tile_steps(kblocks(a, gi, tile % a.n_ntiles)) + GRAN - 1) / GRAN;
-        for (int pi = 0; pi < nparts; ++pi, ++g) {
-          const int b = g % C::kNP;
+        for (uint32_t wn; w != kRunEnd; w = wn) {
+          wn = __ldg(++rw);
           // warp-uniform outcome: the TMEM loads below are warp-collective
-          const bool got = __all_sync(0xffffffffu, mbar_wait(pfull(b), (g / C::kNP) & 1, a.wait_limit));
-          if (!got) {
+          if (!mbar_wait_warp(pfull(b), pph, a.wait_limit)) {
             on_timeout();
             ok = false;
             break;
           }
-          tc_fence_after();
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {  // 16 columns at a time: fewer live registers
-            uint32_t r[16];
-            tmem_ld16(tmem_base + lane_off + b * BN + col0 + hh * 16, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float2 pv = make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-              if (F16) pv = make_float2(unbias_rz(pv.x), unbias_rz(pv.y));
-              acc[hh * 8 + j] = __fadd2_rn(acc[hh * 8 + j], pv);
-            }
+          if (w & mymask) {
+            tc_fence_after();
+            drain32<F16, !FINAL && NSX == 2>(taddr + b * BN, acc);
+            tc_fence_before();
           }
-          tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(pempty(b));
+          if (++b == C::kNP) b = 0, pph ^= 1;
         }
         if (!ok) break;
         if (!FOLD) {
-          const bool got = __all_sync(0xffffffffu, mbar_wait(cfull, t & 1, a.wait_limit));
-          if (!got) {
+          if (!mbar_wait_warp(cfull, tph, a.wait_limit)) {
             on_timeout();
             ok = false;
             break;
           }
+          tph ^= 1;
           tc_fence_after();
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            uint32_t r[16];
-            tmem_ld16(tmem_corr + lane_off + col0 + hh * 16, r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              acc[hh * 8 + j] = __fadd2_rn(acc[hh * 8 + j],
-                                           make_float2(__uint_as_float(r[2 * j]),
-                                                       __uint_as_float(r[2 * j + 1])));
-          }
+          drain32<false, false>(tmem_corr + lane_off + col0, acc);
+          tmem_zero16(tmem_corr + lane_off + col0);
+          tmem_zero16(tmem_corr + lane_off + col0 + 16);
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(cempty);
@@ -559,93 +663,55 @@ __global__ void __maxnreg__(96)
         if (FINAL) {
 #pragma unroll
           for (int j = 0; j < CW / 2; ++j) {
-            const float2 f = make_float2(__shfl_sync(0xffffffffu, fcol, 2 * j),
-                                         __shfl_sync(0xffffffffu, fcol, 2 * j + 1));
+            const float2 f = kColScale ? make_float2(__shfl_sync(0xffffffffu, fcol, 2 * j),
+                                                     __shfl_sync(0xffffffffu, fcol, 2 * j + 1))
+                                       : make_float2(fcol, fcol);
             accg[j] = __ffma2_rn(f, acc[j], accg[j]);
           }
         }
       }
       if (!ok) break;
-      const int mt = tile / a.n_ntiles, n0 = (tile % a.n_ntiles) * BN + col0;
+      const int r1 = t.r1, kbk = t.rb * 4 + q;
+      const int r0 = 32 * kbk + lane;  // row of this lane
       if (FINAL) {
-        // V[R + M n] (+)= sum over the group of w_p s_n D_p (FP32 sum of the
+        // V (+)= sum over the group of w_p s_n D_p (FP32 sum of the
         // group's terms, round to nearest).  Additions are L2 reductions:
         // each element gets exactly one correctly rounded FP64 add per group,
         // and the warp does not wait for the old values.
-        const int R = mt * BM + 32 * q + lane;
-        if (R < a.M) {
-          double *col = a.V + (size_t)R;
+        if (r0 < a.d0) {
+          double *dst = a.V + r0 + (size_t)a.d0 * r1 + (size_t)a.vn * n0;
+          const int nv = min(CW, a.N - n0);
 #pragma unroll
           for (int j = 0; j < CW; ++j) {
-            const int n = n0 + j;
-            if (n < a.N) {
+            if (j < nv) {
               const double add = (double)((j & 1) ? accg[j >> 1].y : accg[j >> 1].x);
-              double *dst = col + (size_t)a.M * n;
               if (a.accumulate)
                 atomicAdd(dst, add);
               else
                 __stcs(dst, add);
             }
+            dst += a.vn;
           }
         }
-      } else {
-        // next stage: row R / d0 + d1 n, K index R mod d0; this warp holds
-        // one aligned 32-run of that K index.  Columns go in pairs: the two
-        // lanes of a pair swap one value so that the even lane holds K
-        // indices (r0, r0 + 1) of column j and the odd lane those of column
-        // j + 1; each stores its two elements as one packed BF16 pair per
-        // part.  (ld is even; index d0 < ld is padding and receives zeros.)
-        const int r1 = mt / a.nrb;
-        const int r0 = (mt % a.nrb) * BM + 32 * q + lane;
-        const bool valid = r0 < a.d0;
+      } else if (32 * kbk < a.d0) {
+        // next stage: outer index n, row r1, K index r0; this warp holds one
+        // aligned 32-run of that K index, 64 bytes of one row per part.
+        // Columns go in pairs: the two lanes of a pair swap one value so that
+        // the even lane holds K indices (r0, r0 + 1) of column j and the odd
+        // lane those of column j + 1; each stores its two elements as one
+        // packed pair per part.  (Rows from d0 on are zero rows of X up to the
+        // end of their atom, so the pair of an odd d0 stores a zero for the
+        // padding; lanes beyond it store nothing.)
         const bool odd = lane & 1;
-        const int rpair = r0 & ~1;
-        // The warp's 32 column scales are one per lane (scl, loaded at the
-        // tile's start): loads placed between the loop's global stores could
-        // not be moved ahead of them (the compiler cannot rule out aliasing),
-        // and each would expose its full latency.
-#pragma unroll
-        for (int j = 0; j < CW; j += 2) {
-          const int n = n0 + j;
-          if (n < a.N) {  // uniform across the warp
-            const bool has1 = n + 1 < a.N;
-            const float2 sc = kColScale ? make_float2(__shfl_sync(0xffffffffu, scl, j),
-                                                      __shfl_sync(0xffffffffu, scl, j + 1))
-                                        : make_float2(gfac, gfac);
-            const float2 v = !valid ? make_float2(0.0f, 0.0f)
-                             : (kColScale || F16) ? __fmul2_rn(acc[j >> 1], sc) : acc[j >> 1];
-            float m = 0.0f;
-            if (NSX > 2) {
-              const float m0 =
-                  __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.x) & 0x7fffffffu));
-              const float m1 =
-                  __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.y) & 0x7fffffffu));
-              m = odd ? m1 : m0;
-            }
-            const float recv = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-            const float mine = odd ? v.y : v.x;
-            const float2 vv = odd ? make_float2(recv, mine) : make_float2(mine, recv);
-            const size_t off =
-                (size_t)(r1 + (long long)a.d1 * (n + (odd ? 1 : 0))) * a.ldn + rpair;
-            const bool store = rpair < a.d0 && (!odd || has1);
-            if (F16) {
-              __half2 hh2[2];
-              split_pair_f16(vv, hh2);
-              if (store) {
-                *reinterpret_cast<__half2 *>(a.out0 + off) = hh2[0];
-                *reinterpret_cast<__half2 *>(a.out1 + off) = hh2[1];
-              }
-            } else {
-              __nv_bfloat162 pp[NSX];
-              split_pair_f32<NSX>(vv, m, pp);
-              if (store) {
-                *reinterpret_cast<__nv_bfloat162 *>(a.out0 + off) = pp[0];
-                *reinterpret_cast<__nv_bfloat162 *>(a.out1 + off) = pp[1];
-                if (NSX > 2) *reinterpret_cast<__nv_bfloat162 *>(a.out2 + off) = pp[NSX > 2 ? 2 : 0];
-              }
-            }
-          }
-        }
+        const size_t nstep = (size_t)a.nkbN * a.natN * (C::kAtom / 2);
+        __nv_bfloat16 *dst = a.out + ((size_t)kbk * a.natN + (r1 >> 3)) * (C::kAtom / 2) +
+                             atom_off(r1, lane & ~1, 0) + nstep * (n0 + (odd ? 1 : 0));
+        const bool live = (r0 & ~1) < a.d0;
+        const int nv = min(CW, a.N - n0);
+        if (nv == CW)
+          store_columns<NSX, F16, kColScale, true>(acc, gfac, scl, dst, nstep, odd, live, nv);
+        else
+          store_columns<NSX, F16, kColScale, false>(acc, gfac, scl, dst, nstep, odd, live, nv);
       }
     }
   }
@@ -661,53 +727,53 @@ __global__ void __maxnreg__(96)
 // ---------------------------------------------------------------------------
 // Input and matrix preparation
 // ---------------------------------------------------------------------------
-// rho (FP64, x fastest, rows of K) -> NSX BF16 parts, rows of ld elements.
-// One warp per 32-run of a row; the run's largest |rho| sets the quantum of
-// the leading part.  Elements K..ld-1 are written as zeros.
-template <int NSX>
-__global__ void split_input_kernel(const double *__restrict__ rho, int K, long long rows,
-                                   long long ld, __nv_bfloat16 *o0, __nv_bfloat16 *o1,
-                                   __nv_bfloat16 *o2) {
-  const int runs = (int)((ld + kGroup - 1) / kGroup);
-  const long long nwork = rows * runs;
-  const int lane = threadIdx.x & 31;
+// rho (FP64, x fastest, niz x niy rows of K) -> the first stage's input atoms
+// (rows y, outer index z).  One warp per atom: four lanes to a row, eight
+// consecutive K each, so that every lane writes 16 bytes per part and the warp
+// whole parts of 512 bytes.  BF16: a 32-run's largest |rho| sets the quantum
+// of its leading part.  FP16: rho * 2^-e0 (device scalar *gin, from max |rho|).
+// Elements from K on are written as zeros.
+template <int NSX, bool F16>
+__global__ void split_input_kernel(const double *__restrict__ rho, int K, int niy, long long natoms,
+                                   int nkb, int natA, const float *__restrict__ gin,
+                                   __nv_bfloat16 *out) {
+  const int lane = threadIdx.x & 31, row = lane >> 2, chunk = lane & 3;
+  const double g = F16 ? (double)*gin : 1.0;
   const long long wstride = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w < nwork;
+  for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w < natoms;
        w += wstride) {
-    const long long r = w / runs;
-    const int k = (int)(w % runs) * kGroup + lane;
-    const double v = k < K ? rho[r * K + k] : 0.0;
-    double m = fabs(v);
+    const int at = (int)(w % natA);
+    const long long zk = w / natA;  // z * nkb + K block
+    const int k0 = (int)(zk % nkb) * BK + chunk * 8;
+    const int y = at * kAtomRows + row;
+    const double *src = rho + ((zk / nkb) * niy + y) * K + k0;
+    double v[8], m = 0.0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __nv_bfloat16 p[NSX];
-    split_lead_f64<NSX>(v, m, p);
-    if (k < ld) {
-      const size_t off = (size_t)r * ld + k;
-      o0[off] = p[0];
-      o1[off] = p[1];
-      if (NSX > 2) o2[off] = p[NSX > 2 ? 2 : 0];
+    for (int j = 0; j < 8; ++j) {
+      v[j] = y < niy && k0 + j < K ? src[j] * g : 0.0;
+      m = fmax(m, fabs(v[j]));
     }
-  }
-}
-
-// FP16 mode: rho * 2^-e0 (device scalar *gin, from max |rho|) -> two FP16
-// parts, rows of ld elements, zeros from K to ld.
-__global__ void split_input_f16_kernel(const double *__restrict__ rho, int K, long long rows,
-                                       long long ld, const float *__restrict__ gin, __half *o0,
-                                       __half *o1) {
-  const double g = (double)*gin;
-  // one warp per row, lanes over k (no per-element index division)
-  const int lane = threadIdx.x & 31;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
-       r += nwarps) {
-    for (int k = lane; k < ld; k += 32) {
-      __half p[2];
-      split_f16_f64(k < K ? rho[r * K + k] * g : 0.0, p);
-      o0[r * ld + k] = p[0];
-      o1[r * ld + k] = p[1];
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    __align__(16) __nv_bfloat16 o[NSX][8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (F16) {
+        __half p[2];
+        split_f16_f64(v[j], p);
+        o[0][j] = *reinterpret_cast<__nv_bfloat16 *>(&p[0]);
+        o[1][j] = *reinterpret_cast<__nv_bfloat16 *>(&p[1]);
+      } else {
+        __nv_bfloat16 p[NSX];
+        split_lead_f64<NSX>(v[j], m, p);
+#pragma unroll
+        for (int s = 0; s < NSX; ++s) o[s][j] = p[s];
+      }
     }
+    __nv_bfloat16 *dst = out + (size_t)w * (atom_bytes<NSX>() / 2) + atom_off(row, chunk * 8, 0);
+#pragma unroll
+    for (int s = 0; s < NSX; ++s)
+      *reinterpret_cast<uint4 *>(dst + s * kAtomRows * BK) = *reinterpret_cast<const uint4 *>(o[s]);
   }
 }
 
@@ -777,17 +843,17 @@ __global__ void row_l1max_kernel(const double *__restrict__ T, int N, int K, dou
   }
 }
 
-// One block per matrix row (p, n).  bf16x6: s = 2^ceil(log2 max_K |T|),
-// parts of T / s with the leading part on the quantum 2^-7.  bf16x3: the
-// floating BF16 parts of T itself (s = 1).  fp16x3: floating FP16 parts of
-// 2^14 T / S(p), S(p) the t-point's power-of-two scale (pscale, rows of N),
+// One block per matrix row (p, n), into the row's atoms.  bf16x6: s =
+// 2^ceil(log2 max_K |T|), parts of T / s with the leading part on the quantum
+// 2^-7.  bf16x3: the floating BF16 parts of T itself (s = 1).  fp16x3: floating
+// FP16 parts of 2^14 T / S(p), S(p) the t-point's power-of-two scale (pscale),
 // and s = 1 (S(p) goes into the stage factors).
 template <int NSX, bool F16 = false>
-__global__ void split_matrix_kernel(const double *__restrict__ T, int K, long long ld,
-                                    float *scale, double *scale64, __nv_bfloat16 *o0,
-                                    __nv_bfloat16 *o1, __nv_bfloat16 *o2,
-                                    const double *__restrict__ pscale = nullptr, int N = 1) {
+__global__ void split_matrix_kernel(const double *__restrict__ T, int K, int N, int nkb, int natB,
+                                    float *scale, __nv_bfloat16 *out,
+                                    const double *__restrict__ pscale) {
   const long long row = blockIdx.x;
+  const int p = (int)(row / N), n = (int)(row % N);
   const double *src = T + row * K;
   __shared__ double red[32];
   double m = 0.0;
@@ -803,25 +869,81 @@ __global__ void split_matrix_kernel(const double *__restrict__ T, int K, long lo
   __syncthreads();
   // power-of-two scale: the division is exact
   const double s = (NSX == 2 || F16) ? 1.0 : red[0] > 0.0 ? exp2(ceil(log2(red[0]))) : 1.0;
-  const double tsc = F16 ? ldexp(1.0, 14) / pscale[row / N] : 1.0;
-  if (threadIdx.x == 0) {
-    scale[row] = (float)s;
-    scale64[row] = s;
-  }
-  for (int k = threadIdx.x; k < (int)ld; k += blockDim.x) {
-    const size_t off = (size_t)row * ld + k;
+  const double tsc = F16 ? ldexp(1.0, 14) / pscale[p] : 1.0;
+  if (threadIdx.x == 0) scale[row] = (float)s;
+  for (int k = threadIdx.x; k < nkb * BK; k += blockDim.x) {
+    __nv_bfloat16 *dst = out + (((size_t)p * nkb + k / BK) * natB + n / kAtomRows) * (atom_bytes<NSX>() / 2);
     if (F16) {
       __half h[2];
       split_f16_f64(k < K ? src[k] * tsc : 0.0, h);
-      reinterpret_cast<__half *>(o0)[off] = h[0];
-      reinterpret_cast<__half *>(o1)[off] = h[1];
+      reinterpret_cast<__half *>(dst)[atom_off(n, k, 0)] = h[0];
+      reinterpret_cast<__half *>(dst)[atom_off(n, k, 1)] = h[1];
       continue;
     }
-    __nv_bfloat16 p[NSX];
-    split_lead_f64<NSX>(k < K ? src[k] / s : 0.0, 1.0, p);
-    o0[off] = p[0];
-    o1[off] = p[1];
-    if (NSX > 2) o2[off] = p[NSX > 2 ? 2 : 0];
+    __nv_bfloat16 o[NSX];
+    split_lead_f64<NSX>(k < K ? src[k] / s : 0.0, 1.0, o);
+#pragma unroll
+    for (int i = 0; i < NSX; ++i) dst[atom_off(n, k, i)] = o[i];
+  }
+}
+
+// First and last K block (lo | hi << 16, lo > hi: none) of every (t-point,
+// n-tile, column group) from the K bands of the FP64 matrix.  FP16: only the entries that the two FP16 parts
+// hold at all (those from 2^-39 of the largest on; the parts of all others are
+// zeros, so leaving them out changes no bit).  One block per (t-point, group).
+template <bool F16>
+__global__ void kbands_kernel(const double *__restrict__ T, int K, int N, int n_ntiles,
+                              const int2 *__restrict__ band, const double *__restrict__ pscale,
+                              uint32_t *kb) {
+  const int ng = n_ntiles * 4, ngr = (N + kBandCols - 1) / kBandCols;
+  const int p = blockIdx.x / ng, g = blockIdx.x % ng;
+  __shared__ int lo, hi;
+  if (g >= ngr) {
+    if (threadIdx.x == 0) kb[blockIdx.x] = 1;  // lo > hi: no block
+    return;
+  }
+  const int2 r = band[(size_t)p * ngr + g];
+  if (threadIdx.x == 0) {
+    lo = F16 ? K : r.x;
+    hi = F16 ? -1 : r.y;
+  }
+  __syncthreads();
+  if (F16) {
+    const double tsc = ldexp(1.0, 14) / pscale[p];
+    const int lane = threadIdx.x & 31;
+    for (int n = g * kBandCols + (threadIdx.x >> 5); n < min((g + 1) * kBandCols, N);
+         n += blockDim.x >> 5) {
+      const double *row = T + ((size_t)p * N + n) * K;
+      int l = K, h = -1;
+      for (int k = r.x + lane; k <= r.y; k += 32)
+        if (!__heq(__double2half(fabs(row[k]) * tsc), __float2half(0.0f))) l = min(l, k), h = k;
+      atomicMin(&lo, l);
+      atomicMax(&hi, h);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    // an all-zero group keeps one block (its product is zero)
+    const int l = hi < lo ? 0 : lo / BK, h = hi < lo ? 0 : hi / BK;
+    kb[blockIdx.x] = (uint32_t)l | ((uint32_t)h << 16);
+  }
+}
+
+// The run lists of every (t-point, n-tile) from the blocks of its four groups.
+__global__ void runs_kernel(const uint4 *__restrict__ kb, int count, int nkb, uint32_t *runs) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const uint4 v = kb[i];
+    const uint32_t g[4] = {v.x, v.y, v.z, v.w};
+    uint32_t *out = runs + (size_t)i * (nkb + 1);
+    for (int b = 0; b < nkb; ++b) {
+      uint32_t m = 0;
+      for (int j = 0; j < 4; ++j)
+        if (b >= (int)(g[j] & 0xffff) && b <= (int)(g[j] >> 16)) m |= 1u << j;
+      if (!m) continue;
+      const uint32_t first = __ffs(m) - 1, n = 32 - __clz(m) - first;
+      *out++ = (uint32_t)b | (m << 16) | (first << 20) | (n << 22);
+    }
+    *out = kRunEnd;
   }
 }
 
@@ -829,58 +951,33 @@ __global__ void split_matrix_kernel(const double *__restrict__ T, int K, long lo
 // Host side
 // ---------------------------------------------------------------------------
 
-// 2-D BF16 map: inner extent `inner` (contiguous), `rows` rows of `ld`
-// elements; box = box_inner x box_rows with the swizzle matching BK.
-int make_map(CUtensorMap *m, const void *base, long long inner, long long rows, long long ld,
-             int box_inner, int box_rows) {
-  auto fn = encode_fn();
-  if (!fn) return fail(DAGE_E_CUDA, "cuTensorMapEncodeTiled unavailable");
-  if (reinterpret_cast<uintptr_t>(base) % 16 || (ld * 2) % 16)
-    return fail(DAGE_E_INVALID, "tensor map base/stride not 16-byte aligned");
-  cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
-  cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  const CUtensorMapSwizzle sw =
-      box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims,
-                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(DAGE_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return 0;
-}
-
 struct MixedState {
   bool f16 = false; // FP16 parts (fp16x3) instead of BF16
-  int nparts = 2;   // BF16 parts per operand
+  int nparts = 2;   // parts per operand
   int G = 1;        // t-points per pass of the last stage (used slots of X[2])
   int Gmax = 1;     // allocated slots of X[2]
-  int ns = 6;       // TMA/MMA ring stages of the stage kernel (autotuned)
+  int ns = 6;       // copy/MMA ring stages of the stage kernel (autotuned)
   DevBuf wdev;      // w_p as FP32 on the device
-  long long ld[3];  // padded K extent of each stage's input rows
-  long long rows[3];
-  DevBuf X[3];      // stage inputs: nparts planes of rows x ld BF16
-  DevBuf Tp[3];     // per-axis matrix parts: nparts planes of P*n_out x ld
-  DevBuf sc[3], sc64[3];
+  // stage inputs: rows d0 (natA atoms), outer indices, K blocks
+  int d0[3], outer[3], nkb[3], natA[3];
+  size_t xbytes[3]; // of one stage input (one slot)
+  DevBuf X[3];
+  DevBuf Tp[3];     // per-axis matrix atoms
+  int natB[3];
+  size_t tbytes[3]; // of one t-point's matrix
+  DevBuf sc[3];
+  DevBuf runs[3];   // run lists [P][n-tiles][nkb + 1]
   int towner[3];
-  CUtensorMap mapA[3][3], mapB[3][3];
   DevBuf err;
   // FP16 mode: per-t-point largest row L1 norm of each owner axis's matrix,
   // the weights in FP64, and the per-apply scales (f16_scales_kernel)
   DevBuf l1[3], psc[3], w64, maxbits, gin, g01, wcoef;
 };
 
-long long round_up(long long v, long long m) { return (v + m - 1) / m * m; }
-
-__nv_bfloat16 *plane(DevBuf &b, int part, long long plane_elems) {
-  return b.as<__nv_bfloat16>() + (size_t)part * plane_elems;
-}
-
-// One stage launch.  nrb > 0 selects the two-dimensional M tiling of the
-// intermediate stages (see StageArgs).
+// One stage launch over ng t-points from p on.
 template <int NSX, int NS, bool FINAL, bool F16>
-int launch_stage(MixedState &st, int stage, int M, int N, int K, int p, int nrb, int ng,
-                 const StageArgs &base, cudaStream_t s) {
+int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int ng, StageArgs a,
+                 cudaStream_t s) {
   using C = StageCfg<NSX, NS, F16>;
   auto kern = stage_bf16_kernel<NSX, NS, FINAL, F16>;
   static bool attr_set = false;
@@ -889,24 +986,23 @@ int launch_stage(MixedState &st, int stage, int M, int N, int K, int p, int nrb,
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
     attr_set = true;
   }
-  StageArgs a = base;
-  a.M = M;
-  a.N = N;
-  a.K = K;
-  a.nrb = nrb;
+  const int ow = st.towner[stage];
+  a.N = op->nout[stage];
+  a.n_ntiles = ceil_div(a.N, BN);
+  a.d0 = st.d0[stage];
+  a.outer = st.outer[stage];
+  a.nrb = ceil_div(a.d0, BM);
+  a.ntiles = a.outer * a.nrb * a.n_ntiles;
+  a.nkb = st.nkb[stage];
+  a.natA = st.natA[stage];
+  a.natB = st.natB[ow];
+  a.X = st.X[stage].as<uint8_t>();
+  a.T = st.Tp[ow].as<uint8_t>() + (size_t)p * st.tbytes[ow];
+  a.runs = st.runs[ow].as<uint32_t>() + (size_t)p * a.n_ntiles * (a.nkb + 1);
+  a.scale = st.sc[ow].as<float>() + (size_t)p * a.N;
   a.ng = ng;
-  a.gM = M;
-  a.n_ntiles = ceil_div(N, BN);
-  const long long nmt = nrb ? (long long)(M / a.d0) * nrb : ceil_div(M, BM);
-  a.ntiles = (int)(nmt * a.n_ntiles);
-  a.nkb = ceil_div(K, BK);
-  a.last_k16 = ceil_div(K - (a.nkb - 1) * BK, 16);
-  a.brow0 = p * N;
   const int grid = std::min(a.ntiles, sm_count());
-  const CUtensorMap *mA = st.mapA[stage];
-  const CUtensorMap *mB = st.mapB[st.towner[stage]];
-  kern<<<grid, kThreads, C::kSmem, s>>>(mA[0], mA[1], mA[NSX > 2 ? 2 : 1], mB[0], mB[1],
-                                        mB[NSX > 2 ? 2 : 1], a);
+  kern<<<grid, kThreads, C::kSmem, s>>>(a);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -914,13 +1010,11 @@ int launch_stage(MixedState &st, int stage, int M, int N, int K, int p, int nrb,
 template <int NSX, int NS, bool F16>
 int run_stages(dage_op3d *op, MixedState &st, const double *d_rho, double *d_V, cudaStream_t s) {
   const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
-  const int nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
-  const long long pe[3] = {st.rows[0] * st.ld[0], st.rows[1] * st.ld[1], st.rows[2] * st.ld[2]};
   // input split (FP16: after the bound-based scales of this input)
   {
     const int t = op->tmark_begin(1);
     if (F16) {
-      const long long n = (long long)nix * st.rows[0];
+      const long long n = (long long)nix * niy * niz;
       const int blocks = (int)std::min<long long>((n + 255) / 256, sm_count() * 8LL);
       DAGE_CUDA_TRY(cudaMemsetAsync(st.maxbits.ptr, 0, sizeof(unsigned), s));
       absmax_kernel<<<blocks, 256, 0, s>>>(d_rho, n, st.maxbits.as<unsigned>());
@@ -930,18 +1024,12 @@ int run_stages(dage_op3d *op, MixedState &st, const double *d_rho, double *d_V, 
           st.psc[st.towner[1]].as<double>(), st.psc[st.towner[2]].as<double>(),
           st.w64.as<double>(), op->P, st.gin.as<float>(), st.g01.as<float>(),
           st.wcoef.as<float>());
-      const long long ne = st.rows[0] * st.ld[0];
-      split_input_f16_kernel<<<(int)std::min<long long>((ne + 255) / 256, sm_count() * 16LL), 256, 0,
-                               s>>>(d_rho, nix, st.rows[0], st.ld[0], st.gin.as<float>(),
-                                    reinterpret_cast<__half *>(plane(st.X[0], 0, pe[0])),
-                                    reinterpret_cast<__half *>(plane(st.X[0], 1, pe[0])));
-    } else {
-      const long long nwarps = st.rows[0] * ((st.ld[0] + kGroup - 1) / kGroup);
-      const int blocks = (int)std::min<long long>((nwarps + 7) / 8, sm_count() * 16LL);
-      split_input_kernel<NSX><<<blocks, 256, 0, s>>>(
-          d_rho, nix, st.rows[0], st.ld[0], plane(st.X[0], 0, pe[0]), plane(st.X[0], 1, pe[0]),
-          plane(st.X[0], NSX > 2 ? 2 : 1, pe[0]));
     }
+    const long long natoms = (long long)st.outer[0] * st.nkb[0] * st.natA[0];
+    const int blocks = (int)std::min<long long>((natoms + 7) / 8, sm_count() * 16LL);
+    split_input_kernel<NSX, F16><<<blocks, 256, 0, s>>>(
+        d_rho, nix, niy, natoms, st.nkb[0], st.natA[0], st.gin.as<float>(),
+        st.X[0].as<__nv_bfloat16>());
     DAGE_CUDA_TRY(cudaGetLastError());
     op->tmark_end(t);
   }
@@ -949,45 +1037,28 @@ int run_stages(dage_op3d *op, MixedState &st, const double *d_rho, double *d_V, 
   base.err = st.err.as<int>();
   base.wait_limit = g_wait_limit;
   base.drain_limit = 4000000000LL;  // ~2 s: copies and MMAs in flight always finish
-  const int ni[3] = {nix, niy, niz}, no[3] = {nox, noy, noz};
-  const long long M[3] = {(long long)niy * niz, (long long)niz * nox, (long long)nox * noy};
-  const int d0[3] = {niy, niz, 0}, d1[3] = {niz, nox, 0};
-  auto common = [&](StageArgs &a, int stage, int p) {
-    const int ow = st.towner[stage];
-    a.scale = st.sc[ow].as<float>() + (size_t)p * no[stage];
-    a.k_range = op->band[ow].as<int2>() + (size_t)p * ceil_div(no[stage], kBandCols);
-  };
-  // last-stage input: slot p % G of X[2], parts stored [part][slot][rows][ld]
-  auto slot_plane = [&](int part, int slot) {
-    return plane(st.X[2], part, pe[2] * st.Gmax) + (size_t)slot * pe[2];
-  };
   int p0 = 0;  // first t-point of the open group
   for (int p = 0; p < op->P; ++p) {
     for (int stage = 0; stage < 2; ++stage) {
       StageArgs a = base;
-      common(a, stage, p);
-      const int slot = p % st.G;
-      a.out0 = stage == 0 ? plane(st.X[1], 0, pe[1]) : slot_plane(0, slot);
-      a.out1 = stage == 0 ? plane(st.X[1], 1, pe[1]) : slot_plane(1, slot);
-      a.out2 = stage == 0 ? plane(st.X[1], NSX > 2 ? 2 : 1, pe[1]) : slot_plane(NSX > 2 ? 2 : 1, slot);
-      a.d0 = d0[stage];
-      a.d1 = d1[stage];
-      a.ldn = st.ld[stage + 1];
+      // last-stage input: slot p % G of X[2]
+      a.out = reinterpret_cast<__nv_bfloat16 *>(
+          st.X[stage + 1].as<uint8_t>() + (stage == 1 ? (p % st.G) * st.xbytes[2] : 0));
+      a.nkbN = st.nkb[stage + 1];
+      a.natN = st.natA[stage + 1];
       if (F16) a.gscale = st.g01.as<float>() + (size_t)stage * op->P + p;
       const int t = op->tmark_begin(0);
-      DAGE_TRY((launch_stage<NSX, NS, false, F16>(st, stage, (int)M[stage], no[stage], ni[stage], p,
-                                                  ceil_div(d0[stage], BM), 1, a, s)));
+      DAGE_TRY((launch_stage<NSX, NS, false, F16>(op, st, stage, p, 1, a, s)));
       op->tmark_end(t);
     }
     if (p - p0 + 1 == st.G || p == op->P - 1) {
       StageArgs a = base;
-      common(a, 2, p0);
-      const int ng = p - p0 + 1;
       a.wcoef = (F16 ? st.wcoef.as<float>() : st.wdev.as<float>()) + p0;
       a.V = d_V;
+      a.vn = (long long)op->nout[0] * op->nout[1];
       a.accumulate = p0 > 0;
       const int t = op->tmark_begin(0);
-      DAGE_TRY((launch_stage<NSX, NS, true, F16>(st, 2, (int)M[2], no[2], ni[2], p0, 0, ng, a, s)));
+      DAGE_TRY((launch_stage<NSX, NS, true, F16>(op, st, 2, p0, p - p0 + 1, a, s)));
       op->tmark_end(t);
       p0 = p + 1;
     }
@@ -1010,60 +1081,72 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
+template <int NSX, bool F16>
+static int split_matrices(dage_op3d *op, MixedState *st, int ax) {
+  const int K = op->nin[ax], N = op->nout[ax], n_ntiles = ceil_div(N, BN);
+  const long long nrows = (long long)op->P * N;
+  cudaStream_t s = op->stream;
+  st->natB[ax] = ceil_div(N, kAtomRows);
+  const int nkb = ceil_div(K, BK);
+  st->tbytes[ax] = (size_t)nkb * st->natB[ax] * atom_bytes<NSX>();
+  DAGE_TRY(st->Tp[ax].alloc(st->tbytes[ax] * op->P));
+  DAGE_TRY(st->sc[ax].alloc(sizeof(float) * nrows));
+  DAGE_TRY(st->runs[ax].alloc(sizeof(uint32_t) * (size_t)op->P * n_ntiles * (nkb + 1)));
+  TmpBuf kb;
+  DAGE_TRY(kb.alloc(sizeof(uint4) * (size_t)op->P * n_ntiles));
+  DAGE_CUDA_TRY(cudaMemsetAsync(st->Tp[ax].ptr, 0, st->Tp[ax].bytes, s));  // rows from N on
+  if (F16) {
+    DAGE_TRY(st->l1[ax].alloc(sizeof(double) * op->P));
+    DAGE_TRY(st->psc[ax].alloc(sizeof(double) * op->P));
+    row_l1max_kernel<<<op->P, 256, 0, s>>>(op->T(ax), N, K, st->l1[ax].as<double>(),
+                                           st->psc[ax].as<double>());
+  }
+  split_matrix_kernel<NSX, F16><<<(unsigned)nrows, 256, 0, s>>>(
+      op->T(ax), K, N, nkb, st->natB[ax], st->sc[ax].as<float>(), st->Tp[ax].as<__nv_bfloat16>(),
+      st->psc[ax].as<double>());
+  kbands_kernel<F16><<<op->P * n_ntiles * 4, 256, 0, s>>>(
+      op->T(ax), K, N, n_ntiles, op->band[ax].as<int2>(), st->psc[ax].as<double>(),
+      kb.as<uint32_t>());
+  runs_kernel<<<ceil_div(op->P * n_ntiles, 128), 128, 0, s>>>(kb.as<uint4>(), op->P * n_ntiles, nkb,
+                                                              st->runs[ax].as<uint32_t>());
+  DAGE_CUDA_TRY(cudaGetLastError());
+  return 0;
+}
+
 int mixed_setup(dage_op3d *op) {
   auto *st = new MixedState();
   op->mixed = st;
   st->f16 = op->precision == DAGE_MIXED_FP16X3;
   st->nparts = op->precision == DAGE_MIXED_BF16X6 ? 3 : 2;
-  const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
-  const int nox = op->nout[0], noy = op->nout[1];
-  const int ni[3] = {nix, niy, niz};
-  st->rows[0] = (long long)niy * niz;
-  st->rows[1] = (long long)niz * nox;
-  st->rows[2] = (long long)nox * noy;
   st->G = st->Gmax = std::min(op->P, kMaxGroup);
   st->ns = st->nparts == 3 ? 4 : 6;
+  // rows and outer indices of the three stages: (y, z), (z, x), (x, y)
+  const int rows[3] = {op->nin[1], op->nin[2], op->nout[0]};
+  const int outer[3] = {op->nin[2], op->nout[0], op->nout[1]};
   for (int s = 0; s < 3; ++s) {
-    st->ld[s] = round_up(ni[s], 8);
-    const int slots = s == 2 ? st->Gmax : 1;
-    const long long pe = st->rows[s] * st->ld[s] * slots;
-    DAGE_TRY(st->X[s].alloc(sizeof(__nv_bfloat16) * pe * st->nparts));
+    const long long tiles = (long long)outer[s] * ceil_div(rows[s], BM) * ceil_div(op->nout[s], BN);
+    if (tiles * st->Gmax >= (1LL << 31) || op->nin[s] >= (1 << 20))
+      return fail(DAGE_E_UNSUPPORTED, "cube too large for the split-precision operator");
+    st->d0[s] = rows[s];
+    st->outer[s] = outer[s];
+    st->nkb[s] = ceil_div(op->nin[s], BK);
+    st->natA[s] = ceil_div(rows[s], kAtomRows);
+    st->xbytes[s] = (size_t)outer[s] * st->nkb[s] * st->natA[s] * (st->nparts * kAtomRows * BK * 2);
+    // padding rows and K columns are never written: they stay zero
+    DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : 1)));
     DAGE_CUDA_TRY(cudaMemsetAsync(st->X[s].ptr, 0, st->X[s].bytes, op->stream));
-    for (int i = 0; i < st->nparts; ++i)
-      DAGE_TRY(make_map(&st->mapA[s][i], plane(st->X[s], i, pe), ni[s], st->rows[s] * slots,
-                        st->ld[s], BK, BM));
   }
   DAGE_TRY(st->err.alloc(sizeof(int)));
   DAGE_CUDA_TRY(cudaMemsetAsync(st->err.ptr, 0, sizeof(int), op->stream));
   for (int ax = 0; ax < 3; ++ax) {
     st->towner[ax] = op->Towner[ax];
     if (op->Towner[ax] != ax) continue;
-    const int K = op->nin[ax], N = op->nout[ax];
-    const long long ld = round_up(K, 8);
-    const long long nrows = (long long)op->P * N;
-    const long long pe = nrows * ld;
-    DAGE_TRY(st->Tp[ax].alloc(sizeof(__nv_bfloat16) * pe * st->nparts));
-    DAGE_TRY(st->sc[ax].alloc(sizeof(float) * nrows));
-    DAGE_TRY(st->sc64[ax].alloc(sizeof(double) * nrows));
-    __nv_bfloat16 *o0 = plane(st->Tp[ax], 0, pe), *o1 = plane(st->Tp[ax], 1, pe),
-                  *o2 = plane(st->Tp[ax], st->nparts > 2 ? 2 : 1, pe);
-    if (st->f16) {
-      DAGE_TRY(st->l1[ax].alloc(sizeof(double) * op->P));
-      DAGE_TRY(st->psc[ax].alloc(sizeof(double) * op->P));
-      row_l1max_kernel<<<op->P, 256, 0, op->stream>>>(op->T(ax), N, K, st->l1[ax].as<double>(),
-                                                      st->psc[ax].as<double>());
-      split_matrix_kernel<2, true><<<(unsigned)nrows, 256, 0, op->stream>>>(
-          op->T(ax), K, ld, st->sc[ax].as<float>(), st->sc64[ax].as<double>(), o0, o1, o2,
-          st->psc[ax].as<double>(), N);
-    } else if (st->nparts == 2)
-      split_matrix_kernel<2><<<(unsigned)nrows, 256, 0, op->stream>>>(
-          op->T(ax), K, ld, st->sc[ax].as<float>(), st->sc64[ax].as<double>(), o0, o1, o2);
+    if (st->f16)
+      DAGE_TRY((split_matrices<2, true>(op, st, ax)));
+    else if (st->nparts == 2)
+      DAGE_TRY((split_matrices<2, false>(op, st, ax)));
     else
-      split_matrix_kernel<3><<<(unsigned)nrows, 256, 0, op->stream>>>(
-          op->T(ax), K, ld, st->sc[ax].as<float>(), st->sc64[ax].as<double>(), o0, o1, o2);
-    DAGE_CUDA_TRY(cudaGetLastError());
-    for (int i = 0; i < st->nparts; ++i)
-      DAGE_TRY(make_map(&st->mapB[ax][i], plane(st->Tp[ax], i, pe), K, nrows, ld, BK, BN));
+      DAGE_TRY((split_matrices<3, false>(op, st, ax)));
   }
   if (st->f16) {
     DAGE_TRY(st->maxbits.alloc(sizeof(unsigned)));
@@ -1131,7 +1214,7 @@ __global__ void fill_kernel(double *x, size_t n, double v) {
 }  // namespace
 
 // Autotuner of the tensor-core path: ring depth of the stage kernel (4 or 6
-// TMA/MMA stages; bf16x6's three-part stages fit 4 only), each candidate
+// copy/MMA stages; bf16x6's three-part stages fit 4 only), each candidate
 // timed over one apply of a scratch cube after one untimed apply; keyed on
 // (device, precision, points per axis, t-points) in the tune cache.  The
 // ring depth changes no arithmetic.  The t-points summed per pass of the
@@ -1202,7 +1285,7 @@ void mixed_destroy(dage_op3d *op) {
     st->X[i].release();
     st->Tp[i].release();
     st->sc[i].release();
-    st->sc64[i].release();
+    st->runs[i].release();
     st->l1[i].release();
     st->psc[i].release();
   }

@@ -25,6 +25,13 @@ constexpr int kGroup = 32;        // K extent of one main-product partial (and o
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+               : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -54,12 +61,39 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
   }
   return true;
 }
+// The same for a whole warp, with one outcome for all of its lanes.  The first
+// look does not wait, and the budget is checked before each wait (the hardware
+// may hold a waiting thread for microseconds).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, long long limit) {
+  uint32_t ready;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ready)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  if (__all_sync(0xffffffffu, ready)) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    if (__any_sync(0xffffffffu, clock64() - t0 > limit)) return false;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  }
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar,
                                             int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+// contiguous copy into shared memory (16-byte aligned, size a multiple of 16)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
+                                          uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          dst),
+      "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
@@ -121,16 +155,36 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                : "memory");
 }
 
-// Shared-memory matrix descriptor of a K-major tile written by TMA with the
-// 64-byte swizzle: rows of 32 bf16 (64 bytes), 8-row swizzle atoms stacked
-// at SBO = 512 bytes.  (K blocks of 64 with 128-byte rows halve the TMA boxes
-// per byte but make the band blocks coarser; measured, the two are within a
-// few percent and 32 is ahead.)
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
+// the same for 32 columns
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+
+// zeros into 32 lanes x 16 consecutive 32-bit columns, completed on return
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1};\n\t"
+      "tcgen05.wait::st.sync.aligned;" ::"r"(taddr),
+      "r"(0)
+      : "memory");
+}
+
+// Shared-memory matrix descriptor of a K-major tile with the 64-byte swizzle:
+// rows of 32 16-bit values (64 bytes), 8-row swizzle atoms of 512 bytes every
+// `sbo` bytes.
+__device__ __forceinline__ uint64_t sdesc64(uint32_t saddr, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
   d |= (uint64_t)1 << 16;           // LBO (unused for swizzled K-major)
-  d |= (uint64_t)(512 >> 4) << 32;  // SBO
+  d |= (uint64_t)(sbo >> 4) << 32;  // SBO
   d |= (uint64_t)1 << 46;           // descriptor version
   d |= (uint64_t)4 << 61;           // SWIZZLE_64B
   return d;
