@@ -2027,10 +2027,7 @@ NearGeom near_geom(const dage_gbfmm *g) {
       G.own[d][v] = B.own[d];
       G.p0[d][v] = B.p0[d];
     }
-    for (int v = 0; v < nb; ++v) {
-      G.T[d].push_back(g->Tnear[d][v].as<double>());
-      G.band[d].push_back(g->band_near[d][v].as<int2>());
-    }
+    for (int v = 0; v < nb; ++v) G.T[d].push_back(g->Tnear[d][v].as<double>());
   }
   return G;
 }

@@ -23,16 +23,21 @@
 // at q0 - koff.  Rows and columns outside a job (tile edges) read zeros or
 // finite neighbouring data that meets zero matrix columns, and their
 // results are not stored.  K blocks are 64 wide (128-byte rows, SWIZZLE_128B:
-// half the TMA rows of 64-byte rows per byte moved); the main product still
-// starts a fresh TMEM partial every 32 K and the partials are added in FP32
+// half the TMA rows of 64-byte rows per byte moved); every 32 K (a run) start
+// a fresh TMEM partial, corrections first, and the partials are added in FP32
 // registers after the +1 ulp toward-zero bias correction, as in the cube
-// operator's fp16x3 stages (op3d_mixed.cu).  Scales: the cube operator's
+// operator's fp16x3 stages (op3d_mixed.cu).  Runs whose FP16 matrix parts are
+// all zero are skipped.  Scales: the cube operator's
 // bound-based powers of two, with L1 norms and entry maxima taken over all
 // box positions of the axis, and one max |rho| per density.
 //
 // Kernel structure (one persistent CTA per SM, 18 warps): warp 0 TMA
-// producer, warp 1 TMEM allocator + single-thread MMA issuer, warps 2-17
-// epilogue (four per TMEM lane quarter, TNW / 4 columns each).  Every
+// producer, warp 1 TMEM allocator + MMA issuer (one elected lane), warps 2-17
+// epilogue (four per TMEM lane quarter, TNW / 4 columns each).  A tile's MMAs
+// are short (241^3: 4 to 6 runs), so what each role must know of it is in one
+// record that is fetched ahead.  GBFMM 241^3, lmax 12, 40 t-points: 23.2 ms an
+// apply with dependent loads per tile and an accumulator of the corrections
+// that was drained between tiles, 20.1 ms so.  Every
 // mbarrier wait is bounded; on timeout the CTA sets the error word, drains
 // its copies and MMAs in flight, frees TMEM and returns.
 #include <cuda.h>
@@ -43,7 +48,6 @@
 #include <cmath>
 #include <vector>
 
-#include "fp64_stage.cuh"
 #include "near_mixed.cuh"
 #include "tc_common.cuh"
 
@@ -60,24 +64,27 @@ constexpr int kNMaxGroup = 4;      // t-points summed per pass of the last stage
 constexpr int kRowsA = 32, kRowsB = 4;  // tile rows: 32 along a x 4 along b
 static_assert(kRowsA * kRowsB == BM, "tile rows");
 
-struct NearJob {
-  int ax, ay, az;      // A tensor coordinates of the job's row (0, 0) and K column 0
-  int na, nb, N;       // valid rows along a and b; output columns
-  int brow;            // B (matrix) row of t-point 0, column 0
-  int koff;            // the job's K columns start at koff in its matrix rows
-  int kr_ps;           // K bands per t-point (kBandCols columns each)
+// One tile of a stage (32 a x 4 b rows of one box of one density, TNW output
+// columns): everything a role needs to know in three vector loads, each
+// fetched a tile or two ahead (a tile's MMAs take a few thousand cycles, a
+// chain of dependent loads of job, tile and band tables half of that).
+struct NearTile {
+  int ax, ay, az;      // A tensor coordinates of the tile's row (0, 0), K column 0
+  int brow;            // B (matrix) row of t-point 0, first column
+  int runs;            // index of the n-tile's runs in a t-point's table
+  int bps;             // B rows per t-point
   int inst;            // density of the set (scales)
-  int ta;              // 32-row blocks along a
-  int pad_;
-  long long ooff;      // intermediate stages: first output slice
-  const int2 *band;    // K band [first, last] per (t-point, kBandCols columns)
-  double *V;           // last stage: V at the box's first owned point
-  long long vs_b, vs_n;
+  int dims;            // valid rows along a (low byte) and b (second), columns (upper half)
+  long long out;       // element offset of the tile's (0, 0, first column): in an
+                       // output plane, or (last stage) in V
+  long long pad_;
 };
+static_assert(sizeof(NearTile) == 48, "three vector loads");
 
 struct NearArgs {
-  const NearJob *jobs;
-  const int4 *tiles;   // per tile: job, n-tile, a-block, b-block
+  const int4 *tiles;   // NearTile[ntiles]
+  const uint32_t *runs;  // [P][nruns]: first and last 32-run of K, lo | hi << 16
+  int nruns;
   int ntiles;
   int p;               // t-point (the group's first in the last stage)
   int ng;              // last stage: t-points of the group (member gi reads slot gi)
@@ -86,10 +93,9 @@ struct NearArgs {
   int gstride;
   const float *wcoef;  // last stage: w_p times the scales, at wcoef[inst * wstride + p]
   int wstride;
-  __half *out0, *out1; // intermediate output planes
-  long long oslice0;   // first output slice of this launch (the W slot)
-  int opad;            // rows per output slice
-  long long ldn;       // output row length
+  __half *out0, *out1; // intermediate output planes (at the W slot)
+  long long sn, sb;    // output strides of a column and of a b row (elements)
+  double *const *V;    // last stage: V of each density
   int accumulate;
   int *err;
   long long wait_limit, drain_limit;
@@ -100,8 +106,8 @@ struct NearCfg {
   static constexpr int kABytes = BM * BKN * 2;   // one FP16 part of the A tile
   static constexpr int kBBytes = TNW * BKN * 2;  // one FP16 part of the B tile
   static constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;
-  static constexpr int kNP = 3;                  // partial buffers
-  static constexpr int kTmemCols = 4 * TNW;      // 3 partials + correction
+  static constexpr int kNP = 4;                  // partial buffers
+  static constexpr int kTmemCols = 4 * TNW;
   static constexpr int kSmem = NS * kStageBytes + 1024 + 256;
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
@@ -127,33 +133,57 @@ __device__ __forceinline__ uint64_t sdesc128(uint32_t saddr) {
   return d;
 }
 
-// The MMAs of one 32-run of K: main product (part 0 x part 0) into the fresh
-// partial P (committed to pfull), corrections (1 x 0) and (0 x 1) into Cc.
-template <int TNW, bool FIRST>
-__device__ __forceinline__ void near_mma_run(uint32_t P, uint32_t Cc, uint64_t d0, uint32_t idesc,
+// The MMAs of one 32-run of K into the fresh partial P: the corrections
+// (1 x 0) and (0 x 1), then the main product (0 x 0), committed to pfull.
+template <int TNW>
+__device__ __forceinline__ void near_mma_run(uint32_t P, uint64_t d0, uint32_t idesc,
                                              uint32_t pfull_bar) {
   constexpr int kA = BM * BKN * 2, kB = TNW * BKN * 2;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    const uint64_t a0 = d0 + ((k * 32) >> 4), a1 = d0 + ((kA + k * 32) >> 4);
-    const uint64_t b0 = d0 + ((2 * kA + k * 32) >> 4), b1 = d0 + ((2 * kA + kB + k * 32) >> 4);
-    umma_bf16_c(P, a0, b0, idesc, k != 0);
-    if (k == 1) umma_commit(pfull_bar);
-    umma_bf16_c(Cc, a1, b0, idesc, !(FIRST && k == 0));
-    umma_bf16_c(Cc, a0, b1, idesc, true);
+    umma_bf16_c(P, d0 + ((kA + k * 32) >> 4), d0 + ((2 * kA + k * 32) >> 4), idesc, k != 0);
+    umma_bf16_c(P, d0 + ((k * 32) >> 4), d0 + ((2 * kA + kB + k * 32) >> 4), idesc, true);
   }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    umma_bf16_c(P, d0 + ((k * 32) >> 4), d0 + ((2 * kA + k * 32) >> 4), idesc, true);
+  umma_commit(pfull_bar);
 }
 
-// K blocks [first, last] of job j, n-tile nt, t-point p + gi
-template <int TNW>
-__device__ __forceinline__ int2 near_kblocks(const NearArgs &a, const NearJob &j, int nt, int gi) {
-  const int2 *b = j.band + (size_t)(a.p + gi) * j.kr_ps + nt * (TNW / kBandCols);
-  int2 r = b[0];
-#pragma unroll
-  for (int g = 1; g < TNW / kBandCols; ++g)
-    if (nt * TNW + g * kBandCols < j.N) r = make_int2(min(r.x, b[g].x), max(r.y, b[g].y));
-  return make_int2((r.x + j.koff) / BKN, (r.y + j.koff) / BKN);
-}
+// The units (tile, sub-problem) of one CTA in order: tiles blockIdx.x + i
+// gridDim.x, each with its ng t-points.  One vector of the current tile's
+// record, that of the next tile, and the runs of the current and the next unit
+// are in registers; every load is issued at least a unit before its use.
+struct UnitWalk {
+  int tile, gi;
+  int4 mid, midn;  // second vector of the record: runs, bps, inst, dims
+  uint32_t r, rn;  // runs of this unit and of the next
+  __device__ __forceinline__ int4 vec(const NearArgs &a, int t, int i) const {
+    return __ldg(a.tiles + 3 * (size_t)min(t, a.ntiles - 1) + i);
+  }
+  __device__ __forceinline__ uint32_t runs_of(const NearArgs &a, const int4 &m, int g) const {
+    return __ldg(a.runs + (size_t)(a.p + g) * a.nruns + m.x);
+  }
+  __device__ __forceinline__ explicit UnitWalk(const NearArgs &a) : tile(blockIdx.x), gi(0) {
+    mid = vec(a, tile, 1);
+    midn = vec(a, tile + gridDim.x, 1);
+    r = runs_of(a, mid, 0);
+    rn = a.ng > 1 ? runs_of(a, mid, 1) : runs_of(a, midn, 0);
+  }
+  // returns true when the step enters a new tile
+  __device__ __forceinline__ bool next(const NearArgs &a) {
+    const bool fresh = ++gi == a.ng;
+    if (fresh) {
+      gi = 0;
+      tile += gridDim.x;
+      mid = midn;
+      midn = vec(a, tile + gridDim.x, 1);
+    }
+    r = rn;
+    rn = gi + 1 < a.ng ? runs_of(a, mid, gi + 1) : runs_of(a, midn, 0);
+    return fresh;
+  }
+};
 
 template <bool FINAL, int TNW, int NS>
 __global__ void __maxnreg__(96)
@@ -168,16 +198,16 @@ __global__ void __maxnreg__(96)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *tiles = smem;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NS * C::kStageBytes);
-  // bars: full[NS], empty[NS], pfull[3], pempty[3], cfull, cempty, drain
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + 2 * NS + 9);
+  // bars: full[NS], empty[NS], pfull[kNP], pempty[kNP], drain
+  constexpr int NP = C::kNP;
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + 2 * NS + 2 * NP + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto full = [&](int i) { return smem_u32(bars + i); };
   auto empty = [&](int i) { return smem_u32(bars + NS + i); };
   auto pfull = [&](int i) { return smem_u32(bars + 2 * NS + i); };
-  auto pempty = [&](int i) { return smem_u32(bars + 2 * NS + 3 + i); };
-  const uint32_t cfull = smem_u32(bars + 2 * NS + 6), cempty = smem_u32(bars + 2 * NS + 7);
-  const uint32_t drain = smem_u32(bars + 2 * NS + 8);
+  auto pempty = [&](int i) { return smem_u32(bars + 2 * NS + NP + i); };
+  const uint32_t drain = smem_u32(bars + 2 * NS + 2 * NP);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
@@ -188,8 +218,6 @@ __global__ void __maxnreg__(96)
       mbar_init(pfull(i), 1);
       mbar_init(pempty(i), kNEpiThreads / 32);
     }
-    mbar_init(cfull, 1);
-    mbar_init(cempty, kNEpiThreads / 32);
     mbar_init(drain, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -199,13 +227,10 @@ __global__ void __maxnreg__(96)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tmem_corr = tmem_base + C::kNP * TNW;
   auto on_timeout = [&]() {
     *abort_flag = 1;
     atomicCAS(a.err, 0, 1);
   };
-  const int nunits = a.ntiles * a.ng;
-  auto next_unit = [&](int u) { return u + ((u % a.ng == a.ng - 1) ? (gridDim.x - 1) * a.ng + 1 : 1); };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -215,27 +240,30 @@ __global__ void __maxnreg__(96)
       int issued[NS];
       uint32_t issued_ph[NS];
       for (int i = 0; i < NS; ++i) issued[i] = 0, issued_ph[i] = 0;
-      for (int u = blockIdx.x * a.ng; u < nunits && !*abort_flag; u = next_unit(u)) {
-        const int gi = u % a.ng;
-        const int4 t = a.tiles[u / a.ng];
-        const NearJob &j = a.jobs[t.x];
-        const int2 r = near_kblocks<TNW>(a, j, t.y, gi);
-        const int ay = j.ay + kRowsA * t.z, az = j.az + kRowsB * t.w + gi * a.slot_rows;
-        const int brow = j.brow + (a.p + gi) * j.N + t.y * TNW;
-        for (int kb = r.x; kb <= r.y; ++kb) {
+      UnitWalk u(a);
+      int4 xy = u.vec(a, u.tile, 0), xyn = u.vec(a, u.tile + gridDim.x, 0);
+      while (u.tile < a.ntiles && !*abort_flag) {
+        const int az = xy.z + u.gi * a.slot_rows;
+        const int brow = xy.w + (a.p + u.gi) * u.mid.y;
+        const int k1 = (int)(u.r >> 17);  // last K block of 64
+        for (int kb = (int)(u.r & 0xffff) >> 1; kb <= k1; ++kb) {
           if (!mbar_wait(empty(s), ph ^ 1, a.wait_limit)) {
             on_timeout();
             break;
           }
-          uint8_t *st = tiles + s * C::kStageBytes;
+          const uint32_t st = smem_u32(tiles + s * C::kStageBytes);
           mbar_expect_tx(full(s), C::kStageBytes);
-          tma_load_3d(smem_u32(st), &mapA0, full(s), j.ax + kb * BKN, ay, az);
-          tma_load_3d(smem_u32(st + C::kABytes), &mapA1, full(s), j.ax + kb * BKN, ay, az);
-          tma_load_2d(smem_u32(st + 2 * C::kABytes), &mapB0, full(s), kb * BKN, brow);
-          tma_load_2d(smem_u32(st + 2 * C::kABytes + C::kBBytes), &mapB1, full(s), kb * BKN, brow);
+          tma_load_3d(st, &mapA0, full(s), xy.x + kb * BKN, xy.y, az);
+          tma_load_3d(st + C::kABytes, &mapA1, full(s), xy.x + kb * BKN, xy.y, az);
+          tma_load_2d(st + 2 * C::kABytes, &mapB0, full(s), kb * BKN, brow);
+          tma_load_2d(st + 2 * C::kABytes + C::kBBytes, &mapB1, full(s), kb * BKN, brow);
           issued[s] = 1;
           issued_ph[s] = ph;
           if (++s == NS) s = 0, ph ^= 1;
+        }
+        if (u.next(a)) {
+          xy = xyn;
+          xyn = u.vec(a, u.tile + gridDim.x, 0);
         }
       }
       if (*abort_flag)  // let every copy that was issued land first
@@ -244,58 +272,47 @@ __global__ void __maxnreg__(96)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      int b = 0;         // partial buffer of the current 32-run
-      uint32_t pph = 0;  // phase of the partial buffers' current round
-      int t = 0;
-      bool ok = true;
-      const uint64_t dbase = sdesc128(smem_u32(tiles));
-      for (int u = blockIdx.x * a.ng; u < nunits && ok && !*abort_flag; u = next_unit(u), ++t) {
-        const int gi = u % a.ng;
-        const int4 tl = a.tiles[u / a.ng];
-        const NearJob &j = a.jobs[tl.x];
-        const int2 rc = near_kblocks<TNW>(a, j, tl.y, gi);
-        int nt = j.N - tl.y * TNW;
-        if (nt > TNW) nt = TNW;
-        nt = (nt + 15) & ~15;
-        const uint32_t idesc = idesc_f16kind<true>(BM, nt);
-        for (int kb = rc.x; kb <= rc.y; ++kb) {
-          const bool first = kb == rc.x;
-          if (!mbar_wait(full(s), ph, a.wait_limit) ||
-              (first && !mbar_wait(cempty, (t & 1) ^ 1, a.wait_limit))) {
-            on_timeout();
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t d0 = dbase + (uint64_t)((s * C::kStageBytes) >> 4);
-#pragma unroll
-          for (int rr = 0; rr < BKN / kGroup; ++rr) {
-            if (!mbar_wait(pempty(b), pph ^ 1, a.wait_limit)) {
-              on_timeout();
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint64_t dr = d0 + (uint64_t)((rr * kGroup * 2) >> 4);
-            const uint32_t P = tmem_base + b * TNW;
-            if (first && rr == 0)
-              near_mma_run<TNW, true>(P, tmem_corr, dr, idesc, pfull(b));
-            else
-              near_mma_run<TNW, false>(P, tmem_corr, dr, idesc, pfull(b));
-            if (++b == C::kNP) b = 0, pph ^= 1;
-          }
-          if (!ok) break;
-          umma_commit(empty(s));
-          if (++s == NS) s = 0, ph ^= 1;
+    // warp-uniform loop, one elected lane issues (op3d_mixed.cu)
+    const bool leader = elect_one();
+    int s = 0;
+    uint32_t ph = 0;
+    int b = 0;         // partial buffer of the current run
+    uint32_t pph = 0;  // phase of the partial buffers' current round
+    bool ok = true;
+    const uint64_t dbase = sdesc128(smem_u32(tiles));
+    uint64_t da = dbase;
+    UnitWalk u(a);
+    while (u.tile < a.ntiles && ok && !*abort_flag) {
+      const uint32_t runs = __shfl_sync(0xffffffffu, u.r, 0);
+      const int ncol = __shfl_sync(0xffffffffu, u.mid.w, 0) >> 16;
+      const uint32_t idesc = idesc_f16kind<true>(BM, 0) | ((uint32_t)((ncol + 15) >> 4) << 18);
+      const int r0 = runs & 0xffff, r1 = runs >> 16;
+      for (int run = r0; run <= r1; ++run) {
+        if (!mbar_wait_warp(pempty(b), pph ^ 1, a.wait_limit) ||
+            ((run == r0 || !(run & 1)) && !mbar_wait_warp(full(s), ph, a.wait_limit))) {
+          if (leader) on_timeout();
+          ok = false;
+          break;
         }
-        if (ok) umma_commit(cfull);
+        tc_fence_after();
+        const bool last = (run & 1) || run == r1;  // of this shared-memory stage
+        if (leader) {
+          near_mma_run<TNW>(tmem_base + b * TNW, da + (uint64_t)((run & 1) * ((kGroup * 2) >> 4)),
+                            idesc, pfull(b));
+          if (last) umma_commit(empty(s));
+        }
+        __syncwarp();
+        if (++b == NP) b = 0, pph ^= 1;
+        if (last) {
+          da += (uint64_t)(C::kStageBytes >> 4);
+          if (++s == NS) s = 0, ph ^= 1, da = dbase;
+        }
       }
-      umma_commit(drain);
-      mbar_wait(drain, 0, a.drain_limit);
+      u.next(a);
     }
+    if (leader) umma_commit(drain);
+    __syncwarp();
+    mbar_wait(drain, 0, a.drain_limit);
   } else {
     // ------------------------------------------------------------ epilogue
     // warp w reads TMEM lanes 32 (w % 4) .. +31 (its lane quarter = the
@@ -304,49 +321,24 @@ __global__ void __maxnreg__(96)
     const int q = warp & 3;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
     const uint32_t col0 = ((warp - 2) >> 2) * CW;
-    int g = 0, t = 0;
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
-      const int4 tl = a.tiles[tile];
-      const NearJob &j = a.jobs[tl.x];
+    const uint32_t taddr = tmem_base + lane_off + col0;
+    int b = 0;
+    uint32_t pph = 0;
+    UnitWalk u(a);
+    int4 to = u.vec(a, u.tile, 2), ton = u.vec(a, u.tile + gridDim.x, 2);
+    float2 accg[CW / 2];
+#pragma unroll
+    for (int k = 0; k < CW / 2; ++k) accg[k] = make_float2(0.0f, 0.0f);
+    while (u.tile < a.ntiles) {
+      const int na = u.mid.w & 0xff, nb = (u.mid.w >> 8) & 0xff, ncol = u.mid.w >> 16;
+      const float f = FINAL ? a.wcoef[(size_t)u.mid.z * a.wstride + a.p + u.gi]
+                            : a.gscale[(size_t)u.mid.z * a.gstride + a.p];
       float2 acc[CW / 2];
-      float2 accg[CW / 2];
 #pragma unroll
-      for (int k = 0; k < CW / 2; ++k) accg[k] = make_float2(0.0f, 0.0f);
+      for (int k = 0; k < CW / 2; ++k) acc[k] = make_float2(0.0f, 0.0f);
       bool ok = true;
-      for (int gi = 0; gi < a.ng && ok; ++gi, ++t) {
-        const float fw = FINAL ? a.wcoef[(size_t)j.inst * a.wstride + a.p + gi] : 0.0f;
-#pragma unroll
-        for (int k = 0; k < CW / 2; ++k) acc[k] = make_float2(0.0f, 0.0f);
-        const int2 rc = near_kblocks<TNW>(a, j, tl.y, gi);
-        const int nparts = (rc.y - rc.x + 1) * (BKN / kGroup);
-        for (int pi = 0; pi < nparts; ++pi, ++g) {
-          const int b = g % C::kNP;
-          const bool got =
-              __all_sync(0xffffffffu, mbar_wait(pfull(b), (g / C::kNP) & 1, a.wait_limit));
-          if (!got) {
-            on_timeout();
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-#pragma unroll
-          for (int hh = 0; hh < CW / 16; ++hh) {
-            uint32_t r[16];
-            tmem_ld16(tmem_base + lane_off + b * TNW + col0 + hh * 16, r);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const float2 pv = make_float2(unbias_rz(__uint_as_float(r[2 * k])),
-                                            unbias_rz(__uint_as_float(r[2 * k + 1])));
-              acc[hh * 8 + k] = __fadd2_rn(acc[hh * 8 + k], pv);
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(pempty(b));
-        }
-        if (!ok) break;
-        const bool got = __all_sync(0xffffffffu, mbar_wait(cfull, t & 1, a.wait_limit));
-        if (!got) {
+      for (int left = (int)(u.r >> 16) - (int)(u.r & 0xffff) + 1; left > 0; --left) {
+        if (!mbar_wait_warp(pfull(b), pph, a.wait_limit)) {
           on_timeout();
           ok = false;
           break;
@@ -355,71 +347,78 @@ __global__ void __maxnreg__(96)
 #pragma unroll
         for (int hh = 0; hh < CW / 16; ++hh) {
           uint32_t r[16];
-          tmem_ld16(tmem_corr + lane_off + col0 + hh * 16, r);
+          tmem_ld16(taddr + b * TNW + hh * 16, r);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            acc[hh * 8 + k] = __fadd2_rn(acc[hh * 8 + k], make_float2(__uint_as_float(r[2 * k]),
-                                                                      __uint_as_float(r[2 * k + 1])));
+          for (int k = 0; k < 8; ++k) {
+            const float2 pv = make_float2(unbias_rz(__uint_as_float(r[2 * k])),
+                                          unbias_rz(__uint_as_float(r[2 * k + 1])));
+            acc[hh * 8 + k] = __fadd2_rn(acc[hh * 8 + k], pv);
+          }
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(cempty);
-        if (FINAL) {
-          const float2 f = make_float2(fw, fw);
-#pragma unroll
-          for (int k = 0; k < CW / 2; ++k) accg[k] = __ffma2_rn(f, acc[k], accg[k]);
-        }
+        if (lane == 0) mbar_arrive(pempty(b));
+        if (++b == NP) b = 0, pph ^= 1;
       }
       if (!ok) break;
-      const int n0 = tl.y * TNW + col0;
-      const int av = kRowsA * tl.z + lane, bv = kRowsB * tl.w + q;
-      if (bv >= j.nb) continue;  // warp-uniform: this warp's b row lies outside the job
       if (FINAL) {
-        // V(a, b, n) (+)= the group's sum; one FP64 add per element per group
-        if (av < j.na) {
-          double *dst = j.V + av + j.vs_b * bv;
 #pragma unroll
-          for (int k = 0; k < CW; ++k) {
-            const int n = n0 + k;
-            if (n < j.N) {
-              const double add = (double)((k & 1) ? accg[k >> 1].y : accg[k >> 1].x);
-              if (a.accumulate)
-                atomicAdd(dst + j.vs_n * n, add);
-              else
-                __stcs(dst + j.vs_n * n, add);
+        for (int k = 0; k < CW / 2; ++k) accg[k] = __ffma2_rn(make_float2(f, f), acc[k], accg[k]);
+      }
+      const int nv = min(CW, ncol - (int)col0);  // this warp's columns
+      const long long off = ((long long)(uint32_t)to.x | ((long long)to.y << 32)) + a.sb * q +
+                            a.sn * (long long)col0;
+      if (FINAL) {
+        if (u.gi == a.ng - 1) {
+          // V(a, b, n) (+)= the group's sum; one FP64 add per element per group
+          if (lane < na && q < nb) {
+            double *dst = a.V[u.mid.z] + off + lane;
+#pragma unroll
+            for (int k = 0; k < CW; ++k) {
+              if (k < nv) {
+                const double add = (double)((k & 1) ? accg[k >> 1].y : accg[k >> 1].x);
+                if (a.accumulate)
+                  atomicAdd(dst, add);
+                else
+                  __stcs(dst, add);
+              }
+              dst += a.sn;
             }
           }
+#pragma unroll
+          for (int k = 0; k < CW / 2; ++k) accg[k] = make_float2(0.0f, 0.0f);
         }
-      } else {
-        // next stage: element (a, b, n) at out[((oslice0 + ooff + n) opad + b) ldn + a];
-        // lane pairs swap one value so each lane stores two consecutive a of
-        // one column as one packed FP16 pair per part (the a = na slot of an
-        // odd na is the zero padding of the next stage's rows).
-        const float gs = a.gscale[(size_t)j.inst * a.gstride + a.p];
-        const bool valid = av < j.na;
+      } else if (q < nb) {  // warp-uniform: this warp's b row lies inside the job
+        // next stage: lane pairs swap one value so each lane stores two
+        // consecutive a of one column as one packed FP16 pair per part (the
+        // a = na slot of an odd na is padding of the next stage's rows: zero).
+        const float gs = lane < na ? f : 0.0f;
         const bool odd = lane & 1;
-        const int apair = av & ~1;
-        const long long rowbase = (long long)bv * a.ldn + apair;
+        const uint32_t sel = odd ? 0x3276u : 0x5410u;
+        const bool live = (lane & ~1) < na;
+        const size_t o0 = (size_t)(off + (odd ? a.sn : 0) + (lane & ~1));
+        __half *d0 = a.out0 + o0, *d1 = a.out1 + o0;
 #pragma unroll
         for (int k = 0; k < CW; k += 2) {
-          const int n = n0 + k;
-          if (n < j.N) {  // uniform across the warp
-            const bool has1 = n + 1 < j.N;
-            const float2 v = valid ? __fmul2_rn(acc[k >> 1], make_float2(gs, gs))
-                                   : make_float2(0.0f, 0.0f);
-            const float recv = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
-            const float mine = odd ? v.y : v.x;
-            const float2 vv = odd ? make_float2(recv, mine) : make_float2(mine, recv);
-            const size_t off =
-                (size_t)(a.oslice0 + j.ooff + n + (odd ? 1 : 0)) * a.opad * a.ldn + rowbase;
-            if (apair < j.na && (!odd || has1)) {
-              __half2 hh2[2];
-              split_pair_f16(vv, hh2);
-              *reinterpret_cast<__half2 *>(a.out0 + off) = hh2[0];
-              *reinterpret_cast<__half2 *>(a.out1 + off) = hh2[1];
+          if (k < nv) {  // uniform across the warp
+            __half2 h[2];
+            split_pair_f16(__fmul2_rn(acc[k >> 1], make_float2(gs, gs)), h);
+            const uint32_t m0 = *reinterpret_cast<uint32_t *>(&h[0]);
+            const uint32_t m1 = *reinterpret_cast<uint32_t *>(&h[1]);
+            const uint32_t v0 = __byte_perm(m0, __shfl_xor_sync(0xffffffffu, m0, 1), sel);
+            const uint32_t v1 = __byte_perm(m1, __shfl_xor_sync(0xffffffffu, m1, 1), sel);
+            if (live && (!odd || k + 1 < nv)) {
+              *reinterpret_cast<uint32_t *>(d0) = v0;
+              *reinterpret_cast<uint32_t *>(d1) = v1;
             }
           }
+          d0 += 2 * a.sn;
+          d1 += 2 * a.sn;
         }
+      }
+      if (u.next(a)) {
+        to = ton;
+        ton = u.vec(a, u.tile + gridDim.x, 2);
       }
     }
   }
@@ -502,6 +501,36 @@ __global__ void near_split_matrix_kernel(const double *const *T, const int *own,
     const size_t off = (size_t)row * ldb + koff[v] + k;
     o0[off] = h[0];
     o1[off] = h[1];
+  }
+}
+
+// First and last 32-run of K (lo | hi << 16, in the matrix rows' own K, koff
+// included) holding an entry whose FP16 parts are not both zero, for every
+// (t-point, position, n-tile of `tn` columns); grid (P, entries), rv/rc: the
+// entry's position and n-tile.
+__global__ void near_runs_kernel(const double *const *T, const int *own, const int *nq,
+                                 const int *koff, const int *rv, const int *rc, int tn,
+                                 const double *psc, uint32_t *runs) {
+  const int p = blockIdx.x, e = blockIdx.y, v = rv[e];
+  const int N = own[v], K = nq[v];
+  const double tsc = ldexp(1.0, 14) / psc[p];
+  __shared__ int lo, hi;
+  if (threadIdx.x == 0) lo = K, hi = -1;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int n = rc[e] * tn + (threadIdx.x >> 5); n < min((rc[e] + 1) * tn, N); n += blockDim.x >> 5) {
+    const double *row = T[v] + ((size_t)p * N + n) * K;
+    int l = K, h = -1;
+    for (int k = lane; k < K; k += 32)
+      if (!__heq(__double2half(fabs(row[k]) * tsc), __float2half(0.0f))) l = min(l, k), h = k;
+    atomicMin(&lo, l);
+    atomicMax(&hi, h);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // an all-zero tile keeps one run (its product is zero)
+    const int l = hi < lo ? 0 : (koff[v] + lo) / kGroup, h = hi < lo ? 0 : (koff[v] + hi) / kGroup;
+    runs[(size_t)p * gridDim.y + e] = (uint32_t)l | ((uint32_t)h << 16);
   }
 }
 
@@ -626,6 +655,11 @@ struct NearF16Plan {
   std::vector<int> brow[3], koff[3];
   DevBuf Bp[3];          // two FP16 planes of rows x ldb
   DevBuf l1[3], psc[3];  // per t-point: largest row L1 norm, power-of-two entry scale
+  // per tile width (64, 128): runs of every (t-point, position, n-tile), the
+  // number of entries of a t-point and each position's first entry
+  DevBuf runs[3][2];
+  int nruns[3][2] = {};
+  std::vector<int> run0[3][2];
   int maxnq[3] = {0, 0, 0}, maxown[3] = {0, 0, 0};
 };
 
@@ -639,10 +673,10 @@ struct NearF16Set {
   long long xs_rows = 0;        // rows (y, z) of one density's split input
   DevBuf X, U, W;               // two FP16 planes each (when the set owns them)
   __half *xp = nullptr, *up = nullptr, *wp = nullptr;  // the planes in use
-  DevBuf jobs[3], tiles[3];
+  DevBuf tiles[3];
   int ntiles[3] = {0, 0, 0};
-  std::vector<int4> htiles[3];
-  DevBuf maxbits, gin, g01, wcoef, rhoptr, wptr;
+  DevBuf maxbits, gin, g01, wcoef, rhoptr, wptr, vptr;
+  long long sb[3] = {0, 0, 0}, sn[3] = {0, 0, 0};  // output strides of a b row and a column
   CUtensorMap mapA[3][2], mapB[3][2];
   DevBuf err;
 };
@@ -707,6 +741,25 @@ int near_f16_plan_create(NearF16Plan **out, const NearGeom &geom, cudaStream_t s
                                                            pl->psc[d].as<double>(), pl->ldb[d],
                                                            o0, o1);
     DAGE_CUDA_TRY(cudaGetLastError());
+    TmpBuf ent[2];
+    for (int w = 0; w < 2; ++w) {
+      const int tn = w ? 128 : 64;
+      std::vector<int> rv, rc;
+      for (int v = 0; v < npos; ++v) {
+        pl->run0[d][w].push_back((int)rv.size());
+        for (int c = 0; c < ceil_div(geom.own[d][v], tn); ++c) rv.push_back(v), rc.push_back(c);
+      }
+      const int ne = pl->nruns[d][w] = (int)rv.size();
+      DAGE_TRY(pl->runs[d][w].alloc(sizeof(uint32_t) * (size_t)P * ne));
+      DAGE_TRY(ent[w].alloc(sizeof(int) * 2 * ne));
+      DAGE_CUDA_TRY(cudaMemcpyAsync(ent[w].ptr, rv.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, s));
+      DAGE_CUDA_TRY(cudaMemcpyAsync(ent[w].as<int>() + ne, rc.data(), sizeof(int) * ne,
+                                    cudaMemcpyHostToDevice, s));
+      near_runs_kernel<<<dim3(P, ne), 256, 0, s>>>(dT.as<const double *>(), own, nq, koff,
+                                                   ent[w].as<int>(), ent[w].as<int>() + ne, tn,
+                                                   pl->psc[d].as<double>(), pl->runs[d][w].as<uint32_t>());
+      DAGE_CUDA_TRY(cudaGetLastError());
+    }
     // the tables are freed on return: finish the kernels that read them
     DAGE_CUDA_TRY(cudaStreamSynchronize(s));
   }
@@ -719,6 +772,7 @@ void near_f16_plan_destroy(NearF16Plan *pl) {
     pl->Bp[d].release();
     pl->l1[d].release();
     pl->psc[d].release();
+    for (DevBuf &b : pl->runs[d]) b.release();
   }
   delete pl;
 }
@@ -815,6 +869,7 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   DAGE_TRY(st->wcoef.alloc(sizeof(float) * g.P * n));
   DAGE_TRY(st->rhoptr.alloc(sizeof(double *) * n));
   DAGE_TRY(st->wptr.alloc(sizeof(double *) * n));
+  DAGE_TRY(st->vptr.alloc(sizeof(double *) * n));
   DAGE_TRY(st->err.alloc(sizeof(int)));
   DAGE_CUDA_TRY(cudaMemsetAsync(st->err.ptr, 0, sizeof(int), s0));
   // A maps: x stage over the densities stacked along z; U; W with its slots
@@ -833,30 +888,61 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
     }
   }
   // tiles: per job (density-major, then box), n-tile fastest, then a, then b
-  const int ntn = tile_n;
-  for (int s = 0; s < 3; ++s) {
-    int job = 0;
-    for (int i = 0; i < n; ++i)
-      for (const auto &b : boxes) {
-        int na, nb, N;
-        if (s == 0) {
-          na = g.nq[1][b.pos[1]], nb = g.nq[2][b.pos[2]], N = g.own[0][b.pos[0]];
-        } else if (s == 1) {
-          na = g.nq[2][b.pos[2]], nb = g.own[0][b.pos[0]], N = g.own[1][b.pos[1]];
+  const int tn = tile_n, w = tile_n == 128;
+  std::vector<NearTile> tl[3];
+  long long xoff = 0, yoff = 0;  // first U slice (x own) and W slice (y own) of the job
+  for (int i = 0; i < n; ++i)
+    for (const auto &bx : boxes) {
+      const int vx = bx.pos[0], vy = bx.pos[1], vz = bx.pos[2];
+      const int ox = g.own[0][vx], oy = g.own[1][vy];
+      for (int s = 0; s < 3; ++s) {
+        const int v = bx.pos[s];
+        // x: rows (a = y, b = z) of the near region of density i, K = x;
+        // y: U rows (a = z near, b = x own), K = y near; z: W rows (a = x own,
+        // b = y own), K = z near -> V
+        const int na = s == 0 ? g.nq[1][vy] : s == 1 ? g.nq[2][vz] : ox;
+        const int nb = s == 0 ? g.nq[2][vz] : s == 1 ? ox : oy;
+        const int N = g.own[s][v];
+        NearTile t{};
+        t.ax = s == 0 ? g.q0[0][vx] - pl->koff[0][vx] : 0;
+        t.inst = i;
+        t.bps = N;
+        const int ay = s == 0 ? g.q0[1][vy] : 0;
+        const long long az = s == 0 ? g.q0[2][vz] + (long long)i * g.npts[2] : s == 1 ? xoff : yoff;
+        // element offset of (a, b, n) = (0, 0, 0)
+        long long out, sb, sn;
+        if (s < 2) {
+          sb = d.ld[s + 1];
+          sn = (long long)(s == 0 ? d.zpad : d.xpad) * sb;
+          out = (s == 0 ? xoff : yoff) * sn;
         } else {
-          na = g.own[0][b.pos[0]], nb = g.own[1][b.pos[1]], N = g.own[2][b.pos[2]];
+          sb = g.npts[0];
+          sn = (long long)g.npts[0] * g.npts[1];
+          out = g.p0[0][vx] + sb * g.p0[1][vy] + sn * g.p0[2][vz];
         }
-        const int ta = ceil_div(na, kRowsA), tb = ceil_div(nb, kRowsB), tn = ceil_div(N, ntn);
-        for (int y = 0; y < tb; ++y)
-          for (int x = 0; x < ta; ++x)
-            for (int c = 0; c < tn; ++c) st->htiles[s].push_back(make_int4(job, c, x, y));
-        ++job;
+        st->sb[s] = sb;
+        st->sn[s] = sn;
+        for (int y = 0; y < nb; y += kRowsB)
+          for (int x = 0; x < na; x += kRowsA)
+            for (int c = 0; c * tn < N; ++c) {
+              t.ay = ay + x;
+              t.az = (int)(az + y);
+              t.brow = pl->brow[s][v] + c * tn;
+              t.runs = pl->run0[s][w][v] + c;
+              t.dims = std::min(na - x, kRowsA) | std::min(nb - y, kRowsB) << 8 |
+                       std::min(N - c * tn, tn) << 16;
+              t.out = out + x + sb * y + sn * (long long)(c * tn);
+              tl[s].push_back(t);
+            }
       }
-    st->ntiles[s] = (int)st->htiles[s].size();
-    DAGE_TRY(st->tiles[s].alloc(sizeof(int4) * st->htiles[s].size()));
-    DAGE_CUDA_TRY(cudaMemcpyAsync(st->tiles[s].ptr, st->htiles[s].data(),
-                                  sizeof(int4) * st->htiles[s].size(), cudaMemcpyHostToDevice, s0));
-    DAGE_TRY(st->jobs[s].alloc(sizeof(NearJob) * job));
+      xoff += ox;
+      yoff += oy;
+    }
+  for (int s = 0; s < 3; ++s) {
+    st->ntiles[s] = (int)tl[s].size();
+    DAGE_TRY(st->tiles[s].alloc(sizeof(NearTile) * tl[s].size()));
+    DAGE_CUDA_TRY(cudaMemcpyAsync(st->tiles[s].ptr, tl[s].data(), sizeof(NearTile) * tl[s].size(),
+                                  cudaMemcpyHostToDevice, s0));
   }
   DAGE_CUDA_TRY(cudaStreamSynchronize(s0));
   return 0;
@@ -865,80 +951,18 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
 void near_f16_set_destroy(NearF16Set *st) {
   if (!st) return;
   for (DevBuf *b : {&st->X, &st->U, &st->W, &st->maxbits, &st->gin, &st->g01, &st->wcoef,
-                    &st->rhoptr, &st->wptr, &st->err})
+                    &st->rhoptr, &st->wptr, &st->vptr, &st->err})
     b->release();
-  for (int s = 0; s < 3; ++s) {
-    st->jobs[s].release();
-    st->tiles[s].release();
-  }
+  for (int s = 0; s < 3; ++s) st->tiles[s].release();
   delete st;
 }
 
 int near_f16_set_bind(NearF16Set *st, const double *const *rho, double *const *V,
                       const double *const *w, cudaStream_t s) {
-  const NearF16Plan *pl = st->plan;
-  const NearGeom &g = pl->g;
   const int n = st->n;
-  std::vector<NearJob> js[3];
-  long long xoff = 0, yoff = 0;
-  for (int i = 0; i < n; ++i)
-    for (const auto &b : st->boxes) {
-      const int vx = b.pos[0], vy = b.pos[1], vz = b.pos[2];
-      NearJob x{}, y{}, z{};
-      // stage x: rows (a = y, b = z) of the near region of density i, K = x
-      x.koff = pl->koff[0][vx];
-      x.ax = g.q0[0][vx] - x.koff;
-      x.ay = g.q0[1][vy];
-      x.az = g.q0[2][vz] + i * g.npts[2];
-      x.na = g.nq[1][vy];
-      x.nb = g.nq[2][vz];
-      x.N = g.own[0][vx];
-      x.brow = pl->brow[0][vx];
-      x.kr_ps = ceil_div(x.N, kBandCols);
-      x.band = g.band[0][vx];
-      x.ooff = xoff;  // U slices of this job: x own
-      x.ta = ceil_div(x.na, kRowsA);
-      x.inst = i;
-      // stage y: U rows (a = z near, b = x own), K = y near
-      y.ax = 0;
-      y.ay = 0;
-      y.az = (int)xoff;
-      y.na = g.nq[2][vz];
-      y.nb = g.own[0][vx];
-      y.N = g.own[1][vy];
-      y.brow = pl->brow[1][vy];
-      y.kr_ps = ceil_div(y.N, kBandCols);
-      y.band = g.band[1][vy];
-      y.ooff = yoff;  // W slices: y own
-      y.ta = ceil_div(y.na, kRowsA);
-      y.inst = i;
-      // stage z: W rows (a = x own, b = y own), K = z near -> V
-      z.ax = 0;
-      z.ay = 0;
-      z.az = (int)yoff;
-      z.na = g.own[0][vx];
-      z.nb = g.own[1][vy];
-      z.N = g.own[2][vz];
-      z.brow = pl->brow[2][vz];
-      z.kr_ps = ceil_div(z.N, kBandCols);
-      z.band = g.band[2][vz];
-      z.ta = ceil_div(z.na, kRowsA);
-      z.inst = i;
-      z.V = V[i] + g.p0[0][vx] + (size_t)g.npts[0] * g.p0[1][vy] +
-            (size_t)g.npts[0] * g.npts[1] * g.p0[2][vz];
-      z.vs_b = g.npts[0];
-      z.vs_n = (long long)g.npts[0] * g.npts[1];
-      js[0].push_back(x);
-      js[1].push_back(y);
-      js[2].push_back(z);
-      xoff += x.N;
-      yoff += y.N;
-    }
-  for (int d = 0; d < 3; ++d)
-    DAGE_CUDA_TRY(cudaMemcpyAsync(st->jobs[d].ptr, js[d].data(), sizeof(NearJob) * js[d].size(),
-                                  cudaMemcpyHostToDevice, s));
   DAGE_CUDA_TRY(cudaMemcpyAsync(st->rhoptr.ptr, rho, sizeof(double *) * n, cudaMemcpyHostToDevice, s));
   DAGE_CUDA_TRY(cudaMemcpyAsync(st->wptr.ptr, w, sizeof(double *) * n, cudaMemcpyHostToDevice, s));
+  DAGE_CUDA_TRY(cudaMemcpyAsync(st->vptr.ptr, V, sizeof(double *) * n, cudaMemcpyHostToDevice, s));
   // the host tables are pageable and go out of scope
   DAGE_CUDA_TRY(cudaStreamSynchronize(s));
   return 0;
@@ -977,7 +1001,15 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
   base.ng = 1;
   base.gstride = 2 * P;
   base.wstride = P;
-  auto launch = [&](int stage, bool fin, const NearArgs &a) -> int {
+  const int wi = st->tile_n == 128;
+  auto launch = [&](int stage, NearArgs a) -> int {
+    const bool fin = stage == 2;
+    a.tiles = st->tiles[stage].as<int4>();
+    a.ntiles = st->ntiles[stage];
+    a.runs = pl->runs[stage][wi].as<uint32_t>();
+    a.nruns = pl->nruns[stage][wi];
+    a.sb = st->sb[stage];
+    a.sn = st->sn[stage];
     const CUtensorMap *mA = st->mapA[stage], *mB = st->mapB[stage];
     if (st->tile_n == 64)
       return fin ? launch_near<true, 64, 4>(mA, mB, a, s) : launch_near<false, 64, 4>(mA, mB, a, s);
@@ -987,44 +1019,29 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
     const int slot = p % st->G;
     {  // stage x -> U
       NearArgs a = base;
-      a.jobs = st->jobs[0].as<NearJob>();
-      a.tiles = st->tiles[0].as<int4>();
-      a.ntiles = st->ntiles[0];
       a.p = p;
       a.gscale = st->g01.as<float>();
       a.out0 = st->up;
       a.out1 = st->up + ue;
-      a.oslice0 = 0;
-      a.opad = st->zpad;
-      a.ldn = st->ld[1];
-      DAGE_TRY(launch(0, false, a));
+      DAGE_TRY(launch(0, a));
     }
     {  // stage y -> W slot
       NearArgs a = base;
-      a.jobs = st->jobs[1].as<NearJob>();
-      a.tiles = st->tiles[1].as<int4>();
-      a.ntiles = st->ntiles[1];
       a.p = p;
       a.gscale = st->g01.as<float>() + P;
-      a.out0 = st->wp;
-      a.out1 = st->wp + we;
-      a.oslice0 = (long long)slot * st->ysl;
-      a.opad = st->xpad;
-      a.ldn = st->ld[2];
-      DAGE_TRY(launch(1, false, a));
+      a.out0 = st->wp + slot * st->ysl * st->xpad * st->ld[2];
+      a.out1 = a.out0 + we;
+      DAGE_TRY(launch(1, a));
     }
     if (slot == st->G - 1 || p == P - 1) {  // stage z over the group -> V
       NearArgs a = base;
-      const int p0 = p - slot;
-      a.jobs = st->jobs[2].as<NearJob>();
-      a.tiles = st->tiles[2].as<int4>();
-      a.ntiles = st->ntiles[2];
-      a.p = p0;
+      a.p = p - slot;
       a.ng = slot + 1;
       a.slot_rows = (int)st->ysl;
       a.wcoef = st->wcoef.as<float>();
-      a.accumulate = p0 > 0;
-      DAGE_TRY(launch(2, true, a));
+      a.V = st->vptr.as<double *>();
+      a.accumulate = p - slot > 0;
+      DAGE_TRY(launch(2, a));
     }
   }
   return 0;

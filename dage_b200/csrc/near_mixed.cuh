@@ -18,14 +18,12 @@ namespace dage {
 
 // Geometry of one GBFMM grid (plan): per axis, per box position, the near
 // region (first point, points) and the owned output points, and the FP64
-// near-field matrices T[pos][p][own][nq] with their K bands per (t-point,
-// kBandCols rows).
+// near-field matrices T[pos][p][own][nq].
 struct NearGeom {
   int npts[3] = {0, 0, 0};
   int P = 0;
   std::vector<int> q0[3], nq[3], own[3], p0[3];
   std::vector<const double *> T[3];
-  std::vector<const int2 *> band[3];
 };
 
 // One box of a plan: its position along each axis.
@@ -51,7 +49,7 @@ void near_f16_set_sizes(const NearF16Plan *plan, const std::vector<NearBox> &box
 size_t near_f16_set_bytes(const NearF16Plan *plan, const std::vector<NearBox> &boxes, int n);
 
 // Binds device cubes and per-density t-point weights (device arrays of P
-// doubles): uploads the job tables (synchronises the stream).
+// doubles): uploads their addresses (synchronises the stream).
 int near_f16_set_bind(NearF16Set *s, const double *const *rho, double *const *V,
                       const double *const *w, cudaStream_t st);
 
