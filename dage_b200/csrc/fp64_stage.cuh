@@ -55,6 +55,29 @@ constexpr int kFp64TileM = 128;
 constexpr int kBandCols = 32;     // matrix columns (output points) per K band
 constexpr int kMaxPointGroup = 64;  // t-points of one launch
 
+#ifdef __CUDACC__
+__device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
+  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sa), "l"(gmem),
+               "r"(pred ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// D(8x8) += A(8x4, row) B(4x8, col); lane l holds A[l/4][l%4], B[l%4][l/4]
+// and D[l/4][2(l%4) + {0,1}]
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+#endif
+
 // Contiguous cube stage: X[R * ldx + K], out[R + n * M].
 inline StageDesc cube_stage(const double *X, long long ldx, int M, int N, int K, const double *T,
                             long long ldt, double *out, const int2 *krange) {

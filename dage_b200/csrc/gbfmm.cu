@@ -117,6 +117,9 @@ struct GInst {
   const double *Tm2l;       // plan: M2L matrix per displacement
   const int *ffstart, *ffsrc, *ffdisp;  // plan: far-field lists
   const double *wx, *wy, *wz;           // plan: full-grid integration weights
+  const struct ShTile *shtiles;         // plan: boxes by shape, in tiles of up to 64
+  const int *shboxes;
+  int nshtiles;
   double kappa;  // 0: Coulomb; > 0: Helmholtz kernel e^(-kappa r)/r
   // levels: q and L hold every box of levels 2..maxlevel (level 2 first);
   // the finest level starts at box fine_off.  M2M/L2L: translation matrix
@@ -155,13 +158,6 @@ __device__ __forceinline__ double bessel_ratio_series(double x2h, int n) {
     if (term < 1e-17 * sum) break;
   }
   return sum * c_dfinv[n];
-}
-
-__device__ __forceinline__ void bessel_ratios(double x, int L, double *f) {
-  const double x2 = x * x;
-  f[L] = bessel_ratio_series(0.5 * x2, L);
-  if (L >= 1) f[L - 1] = bessel_ratio_series(0.5 * x2, L - 1);
-  for (int l = L - 2; l >= 0; --l) f[l] = (2 * l + 3) * f[l + 1] + x2 * f[l + 2];
 }
 
 // ---------------------------------------------------------------------------
@@ -215,61 +211,37 @@ int sh_tables_init() {
   return 0;
 }
 
-// solid_harmonics with the coefficient tables (every lane of a warp visits
-// the same (l, m) sequence, so the constant-bank reads are uniform).
-template <class F>
-__device__ __forceinline__ void solid_harmonics_tab(int lmax, double x, double y, double z, F &&f) {
-  const double r2 = x * x + y * y + z * z;
-  f(0, 1.0);
-  if (lmax == 0) return;
-  {
-    double p2 = 0.0, p1 = 1.0;
-    for (int l = 1; l <= lmax; ++l) {
-      const double cur = c_shA[lmi(l, 0)] * (z * p1) - c_shB[lmi(l, 0)] * (r2 * p2);
-      f(lmi(l, 0), cur);
-      p2 = p1;
-      p1 = cur;
-    }
-  }
-  double top = x, bot = y;
-  for (int mm = 1; mm <= lmax; ++mm) {
-    if (mm >= 2) {
-      const double c = c_shC[mm];
-      const double nb = c * (y * top + x * bot);
-      const double nt = c * (x * top - y * bot);
-      top = nt;
-      bot = nb;
-    }
-    f(lmi(mm, mm), top);
-    f(lmi(mm, -mm), bot);
-#pragma unroll 1
-    for (int sgn = 0; sgn < 2; ++sgn) {
-      const int m = sgn ? -mm : mm;
-      double p2 = 0.0, p1 = sgn ? bot : top;
-      for (int l = mm + 1; l <= lmax; ++l) {
-        const double cur = c_shA[lmi(l, m)] * (z * p1) - c_shB[lmi(l, m)] * (r2 * p2);
-        f(lmi(l, m), cur);
-        p2 = p1;
-        p1 = cur;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Multipole moments q_lm(b) = sum rho w S_lm (Helmholtz: i_l(kappa r) Y_lm).
+// Multipole moments q_lm(b) = sum rho w S_lm (Helmholtz: i_l(kappa r) Y_lm) and
+// far-field potential V(r) += sum_lm L_lm S_lm, as matrix products.
+//
+// Boxes of the same shape (the same cells about their centres) have the same
+// harmonics S_lm at their points: 64 boxes on an evenly divided grid, eight
+// shapes of 1 to 27 boxes otherwise.  Both sums are then products with the
+// matrix S(lm, point) of the shape,
+//   q(lm, box) = sum_point S(lm, point) w(point) rho(point, box)
+//   V(point, box) += sum_lm S(lm, point) L(lm, box),
+// on the FP64 tensor pipe, with S made on the fly in shared memory, once for
+// up to 64 boxes.  One evaluation of S per box and point (the former kernels)
+// was bound by its recurrences: 241^3, lmax 12 took 2.9 ms for the moments and
+// 1.4 ms for the potential; 0.50 and 0.45 ms so.
 //
 // The (lmax+1)^2 harmonics of a point are split into lmax+1 lane tasks of
 // lmax+1 values each: task 0 is the m = 0 chain (l = 0..lmax); the others
 // pair the chain of m = +-mm (l = mm..lmax, lmax+1-mm values) with the
 // chain of m = +-(lmax+1-mm) of the same sign (mm values); for odd lmax the
-// chains m = +h and m = -h, h = (lmax+1)/2, form the last task.  A warp
-// evaluates PP = 32/(lmax+1) points at a time, lane p(lmax+1)+t running task
-// t for point p, each lane keeping its lmax+1 sums in registers.  Warps walk
-// columns of the box (PP neighbouring x, one y, every z); at the end the
-// block sums its lanes in a fixed order into one partial per (box, slab).
+// chains m = +h and m = -h, h = (lmax+1)/2, form the last task.
 // ---------------------------------------------------------------------------
-constexpr int kMpWarps = 8;
+constexpr int kShThreads = 512;  // 16 warps
+constexpr int kShCols = 64;      // boxes of one block
+constexpr int kMpPoints = 32;    // points per step of the moments
+constexpr int kMpPitch = kMpPoints + 4;  // shared rows, free of bank conflicts
+
+// Up to 64 boxes of one shape, a column tile of both products.
+struct ShTile {
+  int first, count;  // in the plan's list of boxes by shape
+};
+
 
 // chains of task t: signed m of the first and second chain (task 0: the
 // m = 0 chain alone, m2 unused) and the first chain's length
@@ -307,151 +279,207 @@ __device__ __forceinline__ void mp_step(int L, int t, int k, int &l, int &m) {
   }
 }
 
-template <bool HELM>
-__global__ void __launch_bounds__(kMpWarps * 32, HELM ? 2 : 3)
-    multipoles_kernel(const GInst *__restrict__ insts, int lmax, int nslab) {
-  __shared__ double sA[16 * 16], sB[16 * 16];  // [k][t]
-  __shared__ double red[kMpWarps][32][17];
-  const GInst &I = insts[blockIdx.z];
-  const int L = lmax, L1 = lmax + 1;
-  const int PP = 32 / L1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Shared tables of the harmonics' recurrences, [step k][task t], zero at chain
+// starts, and the lm of each step.
+struct ShTables {
+  double A[16 * 16], B[16 * 16];
+  short lm[16 * 16];
+};
+__device__ __forceinline__ void sh_fill(ShTables &T, int L) {
+  const int L1 = L + 1;
   for (int e = threadIdx.x; e < L1 * L1; e += blockDim.x) {
     const int t = e / L1, k = e % L1;
     int l, m;
     mp_step(L, t, k, l, m);
     const bool start = l == abs(m);
-    sA[k * 16 + t] = start ? 0.0 : c_shA[lmi(l, m)];
-    sB[k * 16 + t] = start ? 0.0 : c_shB[lmi(l, m)];
+    T.A[k * 16 + t] = start ? 0.0 : c_shA[lmi(l, m)];
+    T.B[k * 16 + t] = start ? 0.0 : c_shB[lmi(l, m)];
+    T.lm[k * 16 + t] = (short)lmi(l, m);
   }
-  __syncthreads();
-  const int p = lane / L1, t = lane % L1;
+}
+// The lmax+1 values of task t at (x, y, z), times w [g_l], to out[lm * stride];
+// g: null, or kappa^l f_l(kappa r) per l.
+__device__ __forceinline__ void sh_task(const ShTables &T, int L, int t, double x, double y,
+                                        double z, double w, const double *g, double *out,
+                                        int stride) {
   int m1, m2, len1;
   mp_task(L, t, m1, m2, len1);
   const int a1 = abs(m1), a2 = abs(m2), amax = t == 0 ? 0 : max(a1, a2);
-  const bool helm = HELM && I.kappa > 0.0;  // a batch may mix kernels
-  const BoxInfo b = I.boxes[blockIdx.x];
+  // chain starts S_{a1,+-a1}, S_{a2,+-a2} (task 0: S_00 = 1)
+  double s1 = 1.0, s2 = 0.0, top = x, bot = y;
+  for (int mm = 1; mm <= amax; ++mm) {
+    if (mm >= 2) {
+      const double c = c_shC[mm];
+      const double nb = c * (y * top + x * bot);
+      const double nt = c * (x * top - y * bot);
+      top = nt;
+      bot = nb;
+    }
+    if (mm == a1) s1 = m1 > 0 ? top : bot;
+    if (mm == a2) s2 = m2 > 0 ? top : bot;
+  }
+  const double r2 = x * x + y * y + z * z;
+  double p1 = 0.0, p2 = 0.0;
+  for (int k = 0; k <= L; ++k) {
+    const bool st = k == 0 || k == len1;
+    const double rec = T.A[k * 16 + t] * (z * p1) - T.B[k * 16 + t] * (r2 * p2);
+    const double cur = st ? (k == 0 ? s1 : s2) : rec;
+    p2 = st ? 0.0 : p1;
+    p1 = cur;
+    const double f = g ? w * g[k < len1 ? a1 + k : a2 + k - len1] : w;
+    out[T.lm[k * 16 + t] * stride] = f * cur;
+  }
+}
+// Bessel factors kappa^l f_l(kappa r), l = 0..L, of `n` points into rows of 17:
+// two lanes a point, one series each (l = L and L - 1), then the downward
+// recursion.  pos(i, x, y, z) gives point i; threads from first0 on take part.
+template <class P>
+__device__ __forceinline__ void sh_bessel(int L, double kappa, int n, int first0, P &&pos,
+                                          double (*g)[17]) {
+  const int id = (int)threadIdx.x - first0;
+  if (id < 0 || id >= 2 * n) return;  // whole warps: 2 n is a multiple of 32
+  double x, y, z;
+  pos(id >> 1, x, y, z);
+  const double x2 = (kappa * kappa) * (x * x + y * y + z * z);
+  const int l0 = max(L - (id & 1), 0);
+  const double own = bessel_ratio_series(0.5 * x2, l0);
+  const double other = __shfl_xor_sync(0xffffffffu, own, 1);
+  if (id & 1) return;
+  double *r = g[id >> 1];
+  r[L] = own;
+  if (L >= 1) r[L - 1] = other;
+  for (int l = L - 2; l >= 0; --l) r[l] = (2 * l + 3) * r[l + 1] + x2 * r[l + 2];
+  double kp = 1.0;
+  for (int l = 0; l <= L; ++l) {
+    r[l] *= kp;
+    kp *= kappa;
+  }
+}
+
+// warps of a block along the column tiles of 8 (1, 2, 4 or 8)
+__device__ __forceinline__ int sh_nwarps(int count) {
+  return count > 32 ? 8 : count > 16 ? 4 : count > 8 ? 2 : 1;
+}
+
+// Moments: grid (slab, column tile, density).  A block takes a contiguous range
+// of the shape's points, 32 a step: S w of the next step is made while this
+// step's product runs (two buffers, one barrier a step), the densities arrive
+// by asynchronous copies.  Warp w owns 8 columns and every 16/NW-th row tile.
+__global__ void __launch_bounds__(kShThreads, 1)
+    multipoles_kernel(const GInst *__restrict__ insts, int L, int nslab) {
+  extern __shared__ double sh[];
+  __shared__ ShTables T;
+  __shared__ double F[2][kMpPoints][17];
+  __shared__ long long cbase[kShCols];
+  const GInst &I = insts[blockIdx.z];
+  if ((int)blockIdx.y >= I.nshtiles) return;
+  const ShTile ct = I.shtiles[blockIdx.y];
+  const int L1 = L + 1, N = L1 * L1, MT = (N + 7) / 8;
+  const int rows = MT * 8;
+  double *S = sh;                                // [2][rows][kMpPitch]
+  double *R = sh + 2 * rows * kMpPitch;          // [2][kShCols][kMpPitch]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const BoxInfo b = I.boxes[I.shboxes[ct.first]];  // the shape
   const int ws = I.wstride;
   const double *wx = I.wbox + (0 * 64 + b.pos[0]) * ws;
   const double *wy = I.wbox + (1 * 64 + b.pos[1]) * ws;
   const double *wz = I.wbox + (2 * 64 + b.pos[2]) * ws;
   const double *xs = I.wbox + (3 * 64) * ws;  // point coordinates per axis
   const size_t plane = (size_t)I.Nx * I.Ny;
-
-  double acc[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) acc[k] = 0.0;
-
-  const int nib = (b.np[0] + PP - 1) / PP;
-  const int nbund = nib * b.np[1];
-  for (int u = blockIdx.y * kMpWarps + warp; u < nbund; u += nslab * kMpWarps) {
-    const int j = u / nib, i = (u % nib) * PP + p;
-    const bool valid = p < PP && i < b.np[0];
-    const int ii = valid ? i : 0;
-    const double x = xs[b.p0[0] + ii] - b.c[0];
-    const double y = xs[ws + b.p0[1] + j] - b.c[1];
-    const double wxy = valid ? wx[ii] * wy[j] : 0.0;
-    // chain starts S_{a1,+-a1}, S_{a2,+-a2} (task 0: S_00 = 1)
-    double s1 = 1.0, s2 = 0.0;
-    {
-      double top = x, bot = y;
-      for (int mm = 1; mm <= amax; ++mm) {
-        if (mm >= 2) {
-          const double c = c_shC[mm];
-          const double nb = c * (y * top + x * bot);
-          const double nt = c * (x * top - y * bot);
-          top = nt;
-          bot = nb;
-        }
-        if (mm == a1) s1 = m1 > 0 ? top : bot;
-        if (mm == a2) s2 = m2 > 0 ? top : bot;
-      }
-    }
-    const double *rcol = I.rho + (size_t)(b.p0[0] + ii) + (size_t)I.Nx * (b.p0[1] + j) +
-                         plane * b.p0[2];
-    // Helmholtz: i_l(kappa r) Y_lm(rhat) = kappa^l f_l(kappa r) S_lm(r).  The
-    // factors g_l = kappa^l f_l of the bundle's next CZ z values of each of
-    // its PP columns come first, one lane per point (series for L and L - 1,
-    // downward recursion), into this warp's rows of `red` (free until the
-    // final reduction).
-    if constexpr (!HELM) {
-      for (int kz = 0; kz < b.np[2]; ++kz) {
-        const double v = valid ? rcol[plane * kz] * (wxy * wz[kz]) : 0.0;
-        const double z = xs[2 * ws + b.p0[2] + kz] - b.c[2];
-        const double r2 = x * x + y * y + z * z;
-        double p1 = 0.0, p2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          if (k > L) break;
-          const bool st = k == 0 || k == len1;
-          const double rec = sA[k * 16 + t] * (z * p1) - sB[k * 16 + t] * (r2 * p2);
-          const double cur = st ? (k == 0 ? s1 : s2) : rec;
-          p2 = st ? 0.0 : p1;
-          p1 = cur;
-          acc[k] += v * cur;
-        }
-      }
-      continue;
-    }
-    const int CZ = 32 / PP;
-    const int pi = p < PP ? p : 0;
-    for (int kz0 = 0; kz0 < b.np[2]; kz0 += CZ) {
-      if (helm) {
-        const int ic = min((u % nib) * PP + lane / CZ, b.np[0] - 1);
-        const int kc = min(kz0 + lane % CZ, b.np[2] - 1);
-        const double xc = xs[b.p0[0] + ic] - b.c[0], zc = xs[2 * ws + b.p0[2] + kc] - b.c[2];
-        const double x2 = (I.kappa * I.kappa) * (xc * xc + y * y + zc * zc);
-        double *g = red[warp][lane];
-        g[L] = bessel_ratio_series(0.5 * x2, L);
-        if (L >= 1) g[L - 1] = bessel_ratio_series(0.5 * x2, L - 1);
-        for (int l = L - 2; l >= 0; --l) g[l] = (2 * l + 3) * g[l + 1] + x2 * g[l + 2];
-        double kp = 1.0;
-        for (int l = 0; l <= L; ++l) {
-          g[l] *= kp;
-          kp *= I.kappa;
-        }
-        __syncwarp();
-      }
-      const int kzend = min(kz0 + CZ, b.np[2]);
-      for (int kz = kz0; kz < kzend; ++kz) {
-        const double v = valid ? rcol[plane * kz] * (wxy * wz[kz]) : 0.0;
-        const double z = xs[2 * ws + b.p0[2] + kz] - b.c[2];
-        const double r2 = x * x + y * y + z * z;
-        const double *gp = red[warp][pi * CZ + (kz - kz0)];
-        double p1 = 0.0, p2 = 0.0;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          if (k > L) break;
-          const bool st = k == 0 || k == len1;
-          const double rec = sA[k * 16 + t] * (z * p1) - sB[k * 16 + t] * (r2 * p2);
-          const double cur = st ? (k == 0 ? s1 : s2) : rec;
-          p2 = st ? 0.0 : p1;
-          p1 = cur;
-          const double f = helm ? v * gp[k < len1 ? a1 + k : a2 + k - len1] : v;
-          acc[k] += f * cur;
-        }
-      }
-      // Required before the next chunk's factors overwrite `red` and before
-      // the final store below overwrites it with this lane's sums: every
-      // lane of the warp must be done reading the factor rows.
-      if (helm) __syncwarp();
-    }
+  const double kappa = I.kappa;
+  sh_fill(T, L);
+  for (int c = tid; c < kShCols; c += blockDim.x) {
+    const BoxInfo &o = I.boxes[I.shboxes[ct.first + min(c, ct.count - 1)]];
+    cbase[c] = o.p0[0] + (long long)I.Nx * o.p0[1] + (long long)plane * o.p0[2];
   }
-  // (Helmholtz: ordered after the last reads of the factor rows by the
-  // __syncwarp at the end of the chunk loop above.)
-#pragma unroll
-  for (int k = 0; k < 16; ++k)
-    if (k <= L) red[warp][lane][k] = acc[k];
+  // rows of S beyond N and columns of R beyond the tile's boxes stay zero
+  for (int e = tid; e < 2 * (rows + kShCols) * kMpPitch; e += blockDim.x) sh[e] = 0.0;
   __syncthreads();
-  const int N = L1 * L1;
-  for (int e = threadIdx.x; e < N; e += blockDim.x) {
-    const int tt = e / L1, k = e % L1;
-    int l, m;
-    mp_step(L, tt, k, l, m);
-    double sum = 0.0;
-    for (int w = 0; w < kMpWarps; ++w)
-      for (int pp = 0; pp < PP; ++pp) sum += red[w][pp * L1 + tt][k];
-    I.partial[((size_t)blockIdx.x * nslab + blockIdx.y) * N + lmi(l, m)] = sum;
+  const int npts = b.np[0] * b.np[1] * b.np[2];
+  const int nch = (npts + kMpPoints - 1) / kMpPoints;
+  const int c0 = (int)((long long)nch * blockIdx.x / nslab);
+  const int c1 = (int)((long long)nch * (blockIdx.x + 1) / nslab);
+  auto ijk = [&](int e, int &i, int &j, int &k) {
+    i = e % b.np[0];
+    const int r = e / b.np[0];
+    j = r % b.np[1];
+    k = r / b.np[1];
+  };
+  auto pos = [&](int e, double &x, double &y, double &z) {
+    int i, j, k;
+    ijk(min(e, npts - 1), i, j, k);
+    x = xs[b.p0[0] + i] - b.c[0];
+    y = xs[ws + b.p0[1] + j] - b.c[1];
+    z = xs[2 * ws + b.p0[2] + k] - b.c[2];
+  };
+  auto factors = [&](int c) {  // Bessel factors of step c
+    if (kappa > 0.0 && c < c1)
+      sh_bessel(L, kappa, kMpPoints, kShThreads - 2 * kMpPoints,
+                [&](int i, double &x, double &y, double &z) { pos(c * kMpPoints + i, x, y, z); },
+                F[c & 1]);
+  };
+  auto copy = [&](int c) {  // densities of step c
+    if (c < c1) {
+      const int e = c * kMpPoints + lane;
+      int i, j, k;
+      ijk(min(e, npts - 1), i, j, k);
+      const double *src = I.rho + i + (size_t)I.Nx * j + plane * k;
+      for (int col = warp; col < ct.count; col += kShThreads / 32)
+        cp_async8(R + ((c & 1) * kShCols + col) * kMpPitch + lane, src + cbase[col], e < npts);
+    }
+    cp_async_commit();
+  };
+  auto make = [&](int c) {  // S w of step c
+    if (c >= c1) return;
+    for (int u = tid; u < kMpPoints * L1; u += blockDim.x) {
+      const int pt = u / L1, t = u % L1, e = c * kMpPoints + pt;
+      double x, y, z;
+      pos(e, x, y, z);
+      int i, j, k;
+      ijk(min(e, npts - 1), i, j, k);
+      const double w = e < npts ? wx[i] * wy[j] * wz[k] : 0.0;
+      sh_task(T, L, t, x, y, z, w, kappa > 0.0 ? F[c & 1][pt] : nullptr,
+              S + (c & 1) * rows * kMpPitch + pt, kMpPitch);
+    }
+  };
+  const int NW = sh_nwarps(ct.count), MW = 16 / NW;
+  const int wn = warp % NW, wm = warp / NW;
+  double acc[16][2];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i][0] = acc[i][1] = 0.0;
+  factors(c0);
+  copy(c0);
+  __syncthreads();
+  make(c0);
+  factors(c0 + 1);
+  for (int c = c0; c < c1; ++c) {
+    cp_async_wait<0>();
+    __syncthreads();  // step c's S and R, step c + 1's F are complete; the others free
+    copy(c + 1);
+    factors(c + 2);
+    const double *as = S + (c & 1) * rows * kMpPitch + (lane >> 2) * kMpPitch + (lane & 3);
+    const double *bs = R + ((c & 1) * kShCols + wn * 8 + (lane >> 2)) * kMpPitch + (lane & 3);
+#pragma unroll 2
+    for (int ks = 0; ks < kMpPoints; ks += 4) {
+      const double fb = bs[ks];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int mt = wm + i * MW;
+        if (mt < MT) dmma(acc[i], as[mt * 8 * kMpPitch + ks], fb);  // uniform in the warp
+      }
+    }
+    make(c + 1);
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int lm = (wm + i * MW) * 8 + (lane >> 2);
+    if (lm >= N) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int col = wn * 8 + 2 * (lane & 3) + h;
+      if (col < ct.count)
+        I.partial[((size_t)I.shboxes[ct.first + col] * nslab + blockIdx.x) * N + lm] = acc[i][h];
+    }
   }
 }
 
@@ -462,6 +490,7 @@ __global__ void reduce_slabs_kernel(const GInst *__restrict__ insts, int nslab, 
   const GInst &I = insts[blockIdx.y];
   const int b = idx / N, s = idx % N;
   double acc = 0.0;
+#pragma unroll 8
   for (int k = 0; k < nslab; ++k) acc += I.partial[((size_t)b * nslab + k) * N + s];
   I.q[(size_t)(I.fine_off + b) * N + s] = acc;
 }
@@ -538,20 +567,25 @@ __global__ void helm_m2l_matrices_kernel(const double *__restrict__ R, int rblk,
   }
 }
 
-// L(b) = sum over the far field of b of T(disp) q(src); block (box, density).
-// G = blockDim.x / npad thread groups of npad (N rounded up to warps)
-// threads share a target box: group h takes the sources e = start + h,
-// start + h + G, ... and the groups' sums are added in group order
-// (deterministic).
+// L(b) = sum over the far field of b of T(disp) q(src); block (box, part,
+// density).  G = blockDim.x / npad thread groups of npad (N rounded up to
+// warps) threads share the sources of a block: group h takes the sources
+// e = start + h, start + h + G, ...; the groups' sums are added in group order
+// and, where a box has several parts, the parts' by sum_parts_kernel in part
+// order (deterministic).  The matrices (72 MB at 4x4x4 boxes, lmax 12, read 10
+// times) come from the L2: 64 blocks of one box each took 437 us, the
+// apply at 241^3 0.3 ms more than so.
 __global__ void m2l_apply_kernel(const GInst *__restrict__ insts, int N, int npad) {
   extern __shared__ double qs[];  // [G][N] sources, then [G][N] sums
-  const GInst &I = insts[blockIdx.y];
-  const int b = blockIdx.x;
+  const GInst &I = insts[blockIdx.z];
+  const int b = blockIdx.x, parts = gridDim.y;
   const int kM2LGroups = blockDim.x / npad;
   const int h = threadIdx.x / npad, i = threadIdx.x % npad;
   double *q = qs + (size_t)h * N;
   double acc = 0.0;
-  const int e0 = I.ffstart[b], e1 = I.ffstart[b + 1];
+  const int f0 = I.ffstart[b], nf = I.ffstart[b + 1] - f0;
+  const int e0 = f0 + (int)((long long)nf * blockIdx.y / parts);
+  const int e1 = f0 + (int)((long long)nf * (blockIdx.y + 1) / parts);
   for (int base = e0; base < e1; base += kM2LGroups) {
     const int e = base + h;
     __syncthreads();
@@ -559,8 +593,9 @@ __global__ void m2l_apply_kernel(const GInst *__restrict__ insts, int N, int npa
       for (int k = i; k < N; k += npad) q[k] = I.q[(size_t)I.ffsrc[e] * N + k];
     __syncthreads();
     if (e < e1 && i < N) {
-      const double *T = I.Tm2l + (size_t)I.ffdisp[e] * N * N;
-      for (int k = 0; k < N; ++k) acc += T[(size_t)k * N + i] * q[k];
+      const double *T = I.Tm2l + (size_t)I.ffdisp[e] * N * N + i;
+#pragma unroll 8
+      for (int k = 0; k < N; ++k) acc += T[(size_t)k * N] * q[k];
     }
   }
   double *sums = qs + (size_t)kM2LGroups * N;
@@ -569,8 +604,22 @@ __global__ void m2l_apply_kernel(const GInst *__restrict__ insts, int N, int npa
   if (h == 0 && i < N) {
     double t = sums[i];
     for (int g = 1; g < kM2LGroups; ++g) t += sums[(size_t)g * N + i];
-    I.L[(size_t)b * N + i] = t;
+    if (parts == 1)
+      I.L[(size_t)b * N + i] = t;
+    else
+      I.partial[((size_t)b * parts + blockIdx.y) * N + i] = t;
   }
+}
+
+// L(box, lm) = sum over the parts, fixed order; grid (., density)
+__global__ void sum_parts_kernel(const GInst *__restrict__ insts, int parts, int N, int nbox) {
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= nbox * N) return;
+  const GInst &I = insts[blockIdx.y];
+  const int b = idx / N, s = idx % N;
+  double acc = 0.0;
+  for (int k = 0; k < parts; ++k) acc += I.partial[((size_t)b * parts + k) * N + s];
+  I.L[(size_t)b * N + s] = acc;
 }
 
 // Translation matrices W(d) of the distinct child-to-parent displacements
@@ -667,142 +716,123 @@ __global__ void l2l_kernel(const GInst *__restrict__ insts, int N, int poff, int
   }
 }
 
-// V(r) += sum_lm L_lm S_lm(r - c) over the owned points of every box; block
-// (chunk, box, density).  L = the density's own local expansions unless
-// Lext is given (evaluation of caller-supplied expansions).
-__global__ void l2p_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext,
-                           int lmax) {
-  extern __shared__ double Ls[];
+// Potential: V(r) += sum_lm L_lm S_lm(r - c) over the owned points of every box
+// (Helmholtz: 8 kappa sum (2l+1)/(4 pi) i_l(kappa r) Y_lm L_lm,
+// src/gbfmm/gbfmm_helmholtz3d.F90:1019-1105); grid (chunk, column tile,
+// density).  The tile's expansions stay in shared memory, `pts` points' S at a
+// time beside them (two buffers).  L = the density's own local expansions
+// unless Lext is given (evaluation of caller-supplied expansions).
+__global__ void __launch_bounds__(kShThreads, 1)
+    l2p_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext, int L, int pts) {
+  extern __shared__ double sh[];
+  __shared__ ShTables T;
+  __shared__ double F[2][kMpPoints][17];
+  __shared__ long long cbase[kShCols];
+  __shared__ int cown[kShCols];
   const GInst &I = insts[blockIdx.z];
-  if (I.kappa > 0.0) return;  // Helmholtz instances: l2p_helm_kernel
-  const int N = (lmax + 1) * (lmax + 1);
-  const BoxInfo b = I.boxes[blockIdx.y];
-  const double *L = Lext ? Lext : I.L + (size_t)I.fine_off * N;
-  for (int k = threadIdx.x; k < N; k += blockDim.x) Ls[k] = L[(size_t)blockIdx.y * N + k];
-  __syncthreads();
-  const double *xs = I.wbox + (3 * 64) * I.wstride;
+  if ((int)blockIdx.y >= I.nshtiles) return;
+  const ShTile ct = I.shtiles[blockIdx.y];
+  const int L1 = L + 1, N = L1 * L1;
+  const int pitch = (N + 15) / 16 * 16 + 4, KS = (N + 3) / 4;
+  double *S = sh;                     // [2][pts][pitch]
+  double *E = sh + 2 * pts * pitch;   // [kShCols][pitch]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const BoxInfo b = I.boxes[I.shboxes[ct.first]];  // the shape
   const int ws = I.wstride;
-  const long long n = (long long)b.own[0] * b.own[1] * b.own[2];
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % b.own[0]);
-    const long long r = e / b.own[0];
-    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
-    const int gx = b.p0[0] + i, gy = b.p0[1] + j, gz = b.p0[2] + k;
-    double v = 0.0;
-    const double x = xs[gx] - b.c[0], y = xs[ws + gy] - b.c[1], z = xs[2 * ws + gz] - b.c[2];
-    solid_harmonics_tab(lmax, x, y, z, [&](int lm, double s) { v += Ls[lm] * s; });
-    I.V[(size_t)gx + (size_t)I.Nx * gy + (size_t)I.Nx * I.Ny * gz] += v;
-  }
-}
-
-// Helmholtz L2P, V(r) += 8 kappa sum (2l+1)/(4 pi) i_l(kappa r) Y_lm L_lm
-// (src/gbfmm/gbfmm_helmholtz3d.F90:1019-1105), with the multipole kernel's
-// lane tasks: lane p(lmax+1)+t evaluates task t's harmonics of point p and
-// the point's lanes sum their terms with a segmented shuffle reduction.  The
-// Bessel ratios f_l(kappa r), l = 0..lmax, come first for 32 points per
-// warp, one lane per point (series for lmax and lmax - 1, then the downward
-// recursion f_l = (2l+3) f_{l+1} + (kappa r)^2 f_{l+2}), into shared memory.
-// Block (chunk, box, density); Coulomb instances return.
-constexpr int kL2pHelmWarps = 8;
-constexpr int kL2pHelmThreads = kL2pHelmWarps * 32;  // sF has one row block per warp
-
-__global__ void __launch_bounds__(kL2pHelmThreads)
-    l2p_helm_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext, int lmax) {
-  __shared__ double sA[16 * 16], sB[16 * 16], sLt[16 * 16];  // [k][t]
-  __shared__ double sF[kL2pHelmWarps][32][17];              // [warp][point][l]
-  const GInst &I = insts[blockIdx.z];
-  if (!(I.kappa > 0.0)) return;
-  const int L = lmax, L1 = lmax + 1, N = L1 * L1;
-  const int PP = 32 / L1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const BoxInfo b = I.boxes[blockIdx.y];
-  const double *Lb = (Lext ? Lext : I.L + (size_t)I.fine_off * N) + (size_t)blockIdx.y * N;
+  const double *xs = I.wbox + (3 * 64) * ws;
+  const size_t plane = (size_t)I.Nx * I.Ny;
   const double kappa = I.kappa;
-  for (int e = threadIdx.x; e < N; e += blockDim.x) {
-    const int t = e / L1, k = e % L1;
-    int l, m;
-    mp_step(L, t, k, l, m);
-    const bool start = l == abs(m);
-    sA[k * 16 + t] = start ? 0.0 : c_shA[lmi(l, m)];
-    sB[k * 16 + t] = start ? 0.0 : c_shB[lmi(l, m)];
-    double kp = 8.0 * kappa / (4.0 * 3.141592653589793238);  // 8 kappa^(l+1) (2l+1) / (4 pi)
-    for (int i = 0; i < l; ++i) kp *= kappa;
-    sLt[k * 16 + t] = Lb[lmi(l, m)] * ((2 * l + 1) * kp);
-  }
-  __syncthreads();
-  const int p = lane / L1, t = lane % L1;
-  int m1, m2, len1;
-  mp_task(L, t, m1, m2, len1);
-  const int a1 = abs(m1), a2 = abs(m2), amax = t == 0 ? 0 : max(a1, a2);
-  const double *xs = I.wbox + (3 * 64) * I.wstride;
-  const int ws = I.wstride;
-  const long long n = (long long)b.own[0] * b.own[1] * b.own[2];
-  double(*F)[17] = sF[warp];
-  const long long stride32 = (long long)gridDim.x * (blockDim.x >> 5) * 32;
-  for (long long base32 = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32; base32 < n;
-       base32 += stride32) {
-  {  // Bessel ratios of the 32 points, lane = point
-    const long long e = min(base32 + lane, n - 1);
-    const int i = (int)(e % b.own[0]);
-    const long long r = e / b.own[0];
-    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
-    const double x = xs[b.p0[0] + i] - b.c[0], y = xs[ws + b.p0[1] + j] - b.c[1],
-                 z = xs[2 * ws + b.p0[2] + k] - b.c[2];
-    const double x2 = (kappa * kappa) * (x * x + y * y + z * z);
-    double *f = F[lane];
-    f[L] = bessel_ratio_series(0.5 * x2, L);
-    if (L >= 1) f[L - 1] = bessel_ratio_series(0.5 * x2, L - 1);
-    for (int l = L - 2; l >= 0; --l) f[l] = (2 * l + 3) * f[l + 1] + x2 * f[l + 2];
-  }
-  __syncwarp();
-  for (int sub = 0; sub < 32; sub += PP) {
-    const long long e = base32 + sub + p;
-    const bool valid = p < PP && sub + p < 32 && e < n;
-    const long long ee = valid ? e : 0;
-    const int i = (int)(ee % b.own[0]);
-    const long long r = ee / b.own[0];
-    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
-    const int gx = b.p0[0] + i, gy = b.p0[1] + j, gz = b.p0[2] + k;
-    const double x = xs[gx] - b.c[0], y = xs[ws + gy] - b.c[1], z = xs[2 * ws + gz] - b.c[2];
-    const double r2 = x * x + y * y + z * z;
-    double s1 = 1.0, s2 = 0.0;
-    {
-      double top = x, bot = y;
-      for (int mm = 1; mm <= amax; ++mm) {
-        if (mm >= 2) {
-          const double c = c_shC[mm];
-          const double nb = c * (y * top + x * bot);
-          const double nt = c * (x * top - y * bot);
-          top = nt;
-          bot = nb;
-        }
-        if (mm == a1) s1 = m1 > 0 ? top : bot;
-        if (mm == a2) s2 = m2 > 0 ? top : bot;
+  const double *Lb = Lext ? Lext : I.L + (size_t)I.fine_off * N;
+  sh_fill(T, L);
+  const int NW = sh_nwarps(ct.count);
+  for (int e = tid; e < 2 * pts * pitch; e += blockDim.x) S[e] = 0.0;  // lm from N on: zero
+  for (int e = tid; e < NW * 8 * pitch; e += blockDim.x) {
+    const int c = e / pitch, lm = e % pitch;
+    double v = 0.0;
+    if (c < ct.count && lm < N) {
+      v = Lb[(size_t)I.shboxes[ct.first + c] * N + lm];
+      if (kappa > 0.0) {
+        const int l = (int)sqrtf((float)lm + 0.5f);
+        v *= 8.0 * kappa / (4.0 * 3.141592653589793238) * (2 * l + 1);
       }
     }
-    const double *fp = F[valid ? sub + p : 0];
-    double acc = 0.0, p1 = 0.0, p2 = 0.0;
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      if (kk > L) break;
-      const bool st = kk == 0 || kk == len1;
-      const double rec = sA[kk * 16 + t] * (z * p1) - sB[kk * 16 + t] * (r2 * p2);
-      const double cur = st ? (kk == 0 ? s1 : s2) : rec;
-      p2 = st ? 0.0 : p1;
-      p1 = cur;
-      const double f = fp[kk < len1 ? a1 + kk : a2 + kk - len1];
-      acc += (sLt[kk * 16 + t] * f) * cur;
-    }
-    // segmented sum over the point's lanes t = 0..L (fixed order)
-#pragma unroll
-    for (int off = 1; off < 16; off <<= 1) {
-      const double o = __shfl_down_sync(0xffffffffu, acc, off);
-      if (t + off < L1) acc += o;
-    }
-    if (valid && t == 0) I.V[(size_t)gx + (size_t)I.Nx * gy + (size_t)I.Nx * I.Ny * gz] += acc;
+    E[e] = v;
   }
-  __syncwarp();
+  for (int c = tid; c < kShCols; c += blockDim.x) {
+    const BoxInfo &o = I.boxes[I.shboxes[ct.first + min(c, ct.count - 1)]];
+    cbase[c] = o.p0[0] + (long long)I.Nx * o.p0[1] + (long long)plane * o.p0[2];
+    // which of the shape's last points per axis this box owns
+    cown[c] = (o.own[0] == o.np[0]) | (o.own[1] == o.np[1]) << 1 | (o.own[2] == o.np[2]) << 2;
+  }
+  const int npts = b.np[0] * b.np[1] * b.np[2];
+  const int nch = (npts + pts - 1) / pts;
+  auto ijk = [&](int e, int &i, int &j, int &k) {
+    i = e % b.np[0];
+    const int r = e / b.np[0];
+    j = r % b.np[1];
+    k = r / b.np[1];
+  };
+  auto pos = [&](int e, double &x, double &y, double &z) {
+    int i, j, k;
+    ijk(min(e, npts - 1), i, j, k);
+    x = xs[b.p0[0] + i] - b.c[0];
+    y = xs[ws + b.p0[1] + j] - b.c[1];
+    z = xs[2 * ws + b.p0[2] + k] - b.c[2];
+  };
+  const int c0 = (int)((long long)nch * blockIdx.x / gridDim.x);
+  const int c1 = (int)((long long)nch * (blockIdx.x + 1) / gridDim.x);
+  auto factors = [&](int c) {
+    if (kappa > 0.0 && c < c1)
+      sh_bessel(L, kappa, pts, kShThreads - 2 * pts,
+                [&](int i, double &x, double &y, double &z) { pos(c * pts + i, x, y, z); },
+                F[c & 1]);
+  };
+  auto make = [&](int c) {
+    if (c >= c1) return;
+    for (int u = tid; u < pts * L1; u += blockDim.x) {
+      const int pt = u / L1, t = u % L1;
+      double x, y, z;
+      pos(c * pts + pt, x, y, z);
+      sh_task(T, L, t, x, y, z, 1.0, kappa > 0.0 ? F[c & 1][pt] : nullptr,
+              S + ((c & 1) * pts + pt) * pitch, 1);
+    }
+  };
+  const int MT = pts / 8, MW = 16 / NW;
+  const int wn = warp % NW, wm = warp / NW;
+  factors(c0);
+  __syncthreads();
+  make(c0);
+  factors(c0 + 1);
+  for (int c = c0; c < c1; ++c) {
+    __syncthreads();  // step c's S, step c + 1's F are complete; the others free
+    factors(c + 2);
+    if (wm < MT) {
+      double acc[2][2] = {};
+      const double *as = S + ((c & 1) * pts + wm * 8 + (lane >> 2)) * pitch + (lane & 3);
+      const double *bs = E + (wn * 8 + (lane >> 2)) * pitch + (lane & 3);
+      const bool two = wm + MW < MT;
+#pragma unroll 4
+      for (int ks = 0; ks < KS; ++ks) {
+        const double fb = bs[ks * 4];
+        dmma(acc[0], as[ks * 4], fb);
+        if (two) dmma(acc[1], as[MW * 8 * pitch + ks * 4], fb);
+      }
+#pragma unroll
+      for (int i2 = 0; i2 < 2; ++i2) {
+        const int mt = wm + i2 * MW, e = c * pts + mt * 8 + (lane >> 2);
+        if (mt >= MT || e >= npts) continue;
+        int i, j, k;
+        ijk(e, i, j, k);
+        const int edge = (i == b.np[0] - 1) | (j == b.np[1] - 1) << 1 | (k == b.np[2] - 1) << 2;
+        double *dst = I.V + i + (size_t)I.Nx * j + plane * k;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int col = wn * 8 + 2 * (lane & 3) + h;
+          if (col < ct.count && !(edge & ~cown[col])) dst[cbase[col]] += acc[i2][h];
+        }
+      }
+    }
+    make(c + 1);
   }
 }
 
@@ -844,11 +874,12 @@ __global__ void energy_kernel(const GInst *__restrict__ insts) {
 }
 
 __global__ void energy_sum_kernel(const GInst *__restrict__ insts, double *out) {
-  if (threadIdx.x != 0) return;
   const GInst &I = insts[blockIdx.x];
-  double t = 0.0;
-  for (int k = 0; k < kEnergyBlocks; ++k) t += I.epart[k];
-  out[blockIdx.x] = t;
+  double t = 0.0;  // one warp: lanes stride the partial sums, then a fixed tree
+  for (int k = threadIdx.x; k < kEnergyBlocks; k += 32) t += I.epart[k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // ---------------------------------------------------------------------------
@@ -1094,7 +1125,9 @@ struct dage_gbfmm {
   DevBuf d_Wm2m, d_m2m_disp;
   std::vector<double> m2m_dvec;  // child - parent of each distinct M2M displacement
   DevBuf d_Wm2m_h;               // Helmholtz M2M matrices for the current kappa
-  int wstride = 0, nslab = 16, ndisp = 0;
+  int wstride = 0, nslab = 1, ndisp = 0;
+  DevBuf d_shtiles, d_shboxes;   // boxes by shape (multipoles_kernel, l2p_kernel)
+  int nshtiles = 0;
   DevBuf d_U, d_W, d_desc[3];
   size_t U_per_box = 0, W_per_box = 0;
   std::vector<StageDesc> desc[3];
@@ -1302,6 +1335,34 @@ void rotation_blocks(const double *dhat, int L, std::vector<double> &out) {
   }
 }
 
+// Shared-memory bytes of the moments and of the potential (and the latter's
+// points per step: 16 where two buffers of 32 do not fit), lmax <= 15.
+int sh_mp_smem(int N) {
+  return (int)sizeof(double) * 2 * (ceil_div(N, 8) * 8 + kShCols) * kMpPitch;
+}
+int sh_l2p_smem(int N, int *pts) {
+  const int pitch = (N + 15) / 16 * 16 + 4;
+  for (*pts = 32;; *pts /= 2) {
+    const int bytes = (int)sizeof(double) * (2 * *pts + kShCols) * pitch;
+    if (bytes <= 205 * 1024 || *pts == 16) return bytes;  // 15 KB of static tables beside it
+  }
+}
+int sh_prepare() {
+  static std::mutex mu;
+  static bool done = false;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done) return 0;
+  int pts;
+  constexpr int kMax = (kMaxLmax + 1) * (kMaxLmax + 1);
+  int most = 0;
+  for (int l = 0; l <= kMaxLmax; ++l) most = std::max(most, sh_l2p_smem((l + 1) * (l + 1), &pts));
+  DAGE_CUDA_TRY(cudaFuncSetAttribute(multipoles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     sh_mp_smem(kMax)));
+  DAGE_CUDA_TRY(cudaFuncSetAttribute(l2p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  done = true;
+  return 0;
+}
+
 // M2L matrix of every distinct displacement for the plan's kernel.
 // M2L matrix of every distinct displacement of a plan for the kernel with
 // parameter kappa (0: Coulomb), into T.
@@ -1365,6 +1426,68 @@ int build_m2l_into(const dage_gbfmm *g, double kappa, DevBuf &T) {
 
 int build_m2l(dage_gbfmm *g) { return build_m2l_into(g, g->kappa, g->d_Tm2l); }
 
+// Slabs of points of `work` (column tile, density) pairs: at most one per SM,
+// and eight blocks per SM where the pairs differ in size (uneven splits and
+// batches: the largest shape must not be left on a few SMs).
+int sh_slabs(long long work) {
+  return std::max(1, std::min(sm_count(), ceil_div(8LL * sm_count(), work)));
+}
+
+// The boxes by shape: two positions of an axis are alike if their cells have
+// the same steps and their points the same places about the centre, to the
+// rounding of the coordinates (8 ulp of the largest one).
+int build_shapes(dage_gbfmm *g) {
+  const int nb = 1 << g->level;
+  std::vector<int> kind[3];
+  for (int d = 0; d < 3; ++d) {
+    const Axis &a = g->ax[d];
+    std::vector<int> first(nb, -1);  // a box at each position of the axis
+    for (int i = 0; i < g->nbox; ++i) first[g->boxes[i].pos[d]] = i;
+    const double tol = 8 * std::numeric_limits<double>::epsilon() *
+                       std::max(std::fabs(a.points.front()), std::fabs(a.points.back()));
+    kind[d].assign(nb, -1);
+    int kinds = 0;
+    for (int v = 0; v < nb; ++v) {
+      const BoxInfo &B = g->boxes[first[v]];
+      for (int u = 0; u < v && kind[d][v] < 0; ++u) {
+        const BoxInfo &A = g->boxes[first[u]];
+        if (A.np[d] != B.np[d]) continue;
+        const int cells = (B.np[d] - 1) / (a.nlip - 1);
+        bool same = true;
+        for (int c = 0; c < cells && same; ++c)
+          same = a.h[A.p0[d] / (a.nlip - 1) + c] == a.h[B.p0[d] / (a.nlip - 1) + c];
+        for (int i = 0; i < B.np[d] && same; ++i)
+          same = std::fabs((a.points[A.p0[d] + i] - A.c[d]) - (a.points[B.p0[d] + i] - B.c[d])) <= tol;
+        if (same) kind[d][v] = kind[d][u];
+      }
+      if (kind[d][v] < 0) kind[d][v] = kinds++;
+    }
+  }
+  std::map<std::vector<int>, std::vector<int>> shapes;
+  for (int i = 0; i < g->nbox; ++i) {
+    const int *q = g->boxes[i].pos;
+    shapes[{kind[0][q[0]], kind[1][q[1]], kind[2][q[2]]}].push_back(i);
+  }
+  std::vector<ShTile> tiles;
+  std::vector<int> boxes;
+  for (const auto &sh : shapes)
+    for (size_t i = 0; i < sh.second.size(); ++i) {
+      if (i % kShCols == 0) tiles.push_back({(int)boxes.size(), 0});
+      boxes.push_back(sh.second[i]);
+      ++tiles.back().count;
+    }
+  g->nshtiles = (int)tiles.size();
+  g->nslab = sh_slabs(g->nshtiles);
+  DAGE_TRY(g->d_shtiles.alloc(sizeof(ShTile) * tiles.size()));
+  DAGE_TRY(g->d_shboxes.alloc(sizeof(int) * boxes.size()));
+  DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_shtiles.ptr, tiles.data(), sizeof(ShTile) * tiles.size(),
+                                cudaMemcpyHostToDevice, g->stream));
+  DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_shboxes.ptr, boxes.data(), sizeof(int) * boxes.size(),
+                                cudaMemcpyHostToDevice, g->stream));
+  DAGE_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  return 0;
+}
+
 // Helmholtz M2M matrices of the plan's child-to-parent displacements for
 // kappa: the HelmholtzMultipoleTranslator (helmholtz_multipole_tools.F90:
 // 172-278 with :338-378: rotation to the axis parent - child, coaxial
@@ -1416,6 +1539,7 @@ void set_weights(dage_gbfmm *g) { weights_for(g, g->energy, g->w); }
 int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, int lmax,
                       const dage_quad *quad) {
   DAGE_TRY(sh_tables_init());
+  DAGE_TRY(sh_prepare());
   if (!grid || !quad) return fail(DAGE_E_INVALID, "null argument");
   // levels 2..maxlevel: M2L at every level (the local far field of a level-2
   // box is every box outside its neighbourhood), M2M/L2L between levels
@@ -1673,6 +1797,7 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
                                   cudaMemcpyHostToDevice, s));
   }
   DAGE_TRY(build_m2l(g));
+  DAGE_TRY(build_shapes(g));
   DAGE_TRY(g->d_q.alloc(sizeof(double) * g->nbtot * g->N));
   DAGE_TRY(g->d_L.alloc(sizeof(double) * g->nbtot * g->N));
   DAGE_TRY(g->d_partial.alloc(sizeof(double) * (size_t)g->nbox * g->nslab * g->N));
@@ -1757,6 +1882,9 @@ GInst plan_inst(const dage_gbfmm *g, const double *rho, double *V, double *q, do
   I.wx = g->wts[0].as<double>();
   I.wy = g->wts[1].as<double>();
   I.wz = g->wts[2].as<double>();
+  I.shtiles = g->d_shtiles.as<ShTile>();
+  I.shboxes = g->d_shboxes.as<int>();
+  I.nshtiles = g->nshtiles;
   I.kappa = g->kappa;
   I.fine_off = g->fine_off;
   I.m2m_base = g->level > g->lev0 ? g->lev_off[g->lev0 + 1] : 0;
@@ -1851,31 +1979,33 @@ void near_bounds(const dage_gbfmm *g, int mt[3], int nt[3]) {
   }
 }
 
-int max_owned(const dage_gbfmm *g) {
-  int m = 0;
-  for (const auto &B : g->boxes) m = std::max(m, B.own[0] * B.own[1] * B.own[2]);
-  return m;
-}
-
-int run_multipoles(const GInst *d_inst, int ninst, int nbox, int lmax, int nslab, bool helm,
+// nshtiles: the largest of the instances
+int run_multipoles(const GInst *d_inst, int ninst, int nbox, int nshtiles, int lmax, int nslab,
                    cudaStream_t s) {
   const int N = (lmax + 1) * (lmax + 1);
-  if (helm)
-    multipoles_kernel<true><<<dim3(nbox, nslab, ninst), kMpWarps * 32, 0, s>>>(d_inst, lmax, nslab);
-  else
-    multipoles_kernel<false><<<dim3(nbox, nslab, ninst), kMpWarps * 32, 0, s>>>(d_inst, lmax, nslab);
+  multipoles_kernel<<<dim3(nslab, nshtiles, ninst), kShThreads, sh_mp_smem(N), s>>>(d_inst, lmax,
+                                                                                    nslab);
   DAGE_CUDA_TRY(cudaGetLastError());
   reduce_slabs_kernel<<<dim3((nbox * N + 255) / 256, ninst), 256, 0, s>>>(d_inst, nslab, N, nbox);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
 
-int run_m2l(const GInst *d_inst, int ninst, int nbox, int N, cudaStream_t s) {
+// room: boxes x slabs of the instances' partial buffers, free by then
+int run_m2l(const GInst *d_inst, int ninst, int nbox, int N, long long room, cudaStream_t s) {
   const int npad = ((N + 31) / 32) * 32;           // N <= 256
-  const int groups = std::max(1, std::min(8, 1024 / npad));
-  m2l_apply_kernel<<<dim3(nbox, ninst), npad * groups, sizeof(double) * N * 2 * groups, s>>>(
+  const int groups = std::max(1, std::min(4, 1024 / npad));
+  // parts of a box's sources: two blocks on every SM
+  const int parts = (int)std::max<long long>(
+      1, std::min<long long>({8, room / nbox, ceil_div(2LL * sm_count(), (long long)nbox * ninst)}));
+  m2l_apply_kernel<<<dim3(nbox, parts, ninst), npad * groups, sizeof(double) * N * 2 * groups, s>>>(
       d_inst, N, npad);
   DAGE_CUDA_TRY(cudaGetLastError());
+  if (parts > 1) {
+    sum_parts_kernel<<<dim3(ceil_div((long long)nbox * N, 256), ninst), 256, 0, s>>>(d_inst, parts, N,
+                                                                                   nbox);
+    DAGE_CUDA_TRY(cudaGetLastError());
+  }
   return 0;
 }
 
@@ -1901,20 +2031,12 @@ int run_l2l(const GInst *d_inst, int ninst, const dage_gbfmm *g, cudaStream_t s)
   return 0;
 }
 
-// Coulomb instances run l2p_kernel, Helmholtz instances (when `helm`)
-// l2p_helm_kernel; each kernel returns at once on the other kind.
-int run_l2p(const GInst *d_inst, int ninst, int nbox, int lmax, int maxown, const double *Lext,
-            bool helm, cudaStream_t s) {
-  const int N = (lmax + 1) * (lmax + 1);
-  const int bx = std::min((maxown + 127) / 128, 64);
-  l2p_kernel<<<dim3(bx, nbox, ninst), 128, sizeof(double) * N, s>>>(d_inst, Lext, lmax);
+int run_l2p(const GInst *d_inst, int ninst, int nshtiles, int lmax, const double *Lext,
+            cudaStream_t s) {
+  int pts;
+  const int smem = sh_l2p_smem((lmax + 1) * (lmax + 1), &pts);
+  l2p_kernel<<<dim3(sh_slabs((long long)nshtiles * ninst), nshtiles, ninst), kShThreads, smem, s>>>(d_inst, Lext, lmax, pts);
   DAGE_CUDA_TRY(cudaGetLastError());
-  if (helm) {
-    const int pts = kL2pHelmThreads;  // points per block pass (one per thread)
-    const int hx = std::min((maxown + pts - 1) / pts, 256);
-    l2p_helm_kernel<<<dim3(hx, nbox, ninst), kL2pHelmThreads, 0, s>>>(d_inst, Lext, lmax);
-    DAGE_CUDA_TRY(cudaGetLastError());
-  }
   return 0;
 }
 
@@ -2209,7 +2331,7 @@ struct dage_gbfmm_batch {
   };
   std::vector<MSet> msets;
   DevBuf ws16[3];  // the sets' shared workspace: split input, U, W
-  int mt[3] = {0, 0, 0}, nt[3] = {0, 0, 0}, maxown = 0;
+  int mt[3] = {0, 0, 0}, nt[3] = {0, 0, 0}, nshtiles = 0;
   int tile_n[3] = {64, 64, 64};
   bool tuned = false;
   DevBuf stage_rho, stage_V;  // host-pointer mode
@@ -2308,15 +2430,15 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
   b->N = g0->N;
   b->P = g0->P;
   b->nbox = g0->nbox;
-  b->nslab = n >= 8 ? 4 : g0->nslab;  // many densities fill the GPU with fewer slabs
   b->w = g0->w;
   for (const auto *g : b->plans) {
     near_bounds(g, b->mt, b->nt);
-    b->maxown = std::max(b->maxown, max_owned(g));
+    b->nshtiles = std::max(b->nshtiles, g->nshtiles);
   }
   const size_t per = (size_t)g0->nbtot * b->N;  // every level's boxes
   DAGE_TRY(b->q.alloc(sizeof(double) * per * n));
   DAGE_TRY(b->L.alloc(sizeof(double) * per * n));
+  b->nslab = sh_slabs((long long)b->nshtiles * n);
   DAGE_TRY(b->partial.alloc(sizeof(double) * (size_t)b->nbox * b->N * b->nslab * n));
   DAGE_TRY(b->epart.alloc(sizeof(double) * kEnergyBlocks * n));
   DAGE_TRY(b->energy.alloc(sizeof(double) * n));
@@ -2463,11 +2585,9 @@ int batch_launch(dage_gbfmm_batch *b, const double *const *rho, double *const *V
     }
   for (int i = 0; i < b->n; ++i)
     DAGE_CUDA_TRY(cudaMemsetAsync(V[i], 0, sizeof(double) * b->npts[i], s));
-  bool any_helm = false;
-  for (int i = 0; i < b->n; ++i) any_helm |= b->kern_of[i] >= 0;
-  DAGE_TRY(run_multipoles(d_inst, b->n, b->nbox, b->lmax, b->nslab, any_helm, s));
+  DAGE_TRY(run_multipoles(d_inst, b->n, b->nbox, b->nshtiles, b->lmax, b->nslab, s));
   DAGE_TRY(run_m2m(d_inst, b->n, b->plans[0], s));
-  DAGE_TRY(run_m2l(d_inst, b->n, b->plans[0]->nbtot, b->N, s));
+  DAGE_TRY(run_m2l(d_inst, b->n, b->plans[0]->nbtot, b->N, (long long)b->nbox * b->nslab, s));
   DAGE_TRY(run_l2l(d_inst, b->n, b->plans[0], s));
   for (auto &c : b->chunks) {
     const StageDesc *dd[3] = {c.desc[0].as<StageDesc>(), c.desc[1].as<StageDesc>(),
@@ -2475,7 +2595,7 @@ int batch_launch(dage_gbfmm_batch *b, const double *const *rho, double *const *V
     DAGE_TRY(run_near(dd, c.njobs, b->mt, b->nt, b->P, b->w, b->tile_n, s));
   }
   for (auto &m : b->msets) DAGE_TRY(near_f16_set_run(m.set, s));
-  DAGE_TRY(run_l2p(d_inst, b->n, b->nbox, b->lmax, b->maxown, nullptr, any_helm, s));
+  DAGE_TRY(run_l2p(d_inst, b->n, b->nshtiles, b->lmax, nullptr, s));
   DAGE_TRY(run_energy(d_inst, b->n, b->energy.as<double>(), s));
   return 0;
 }
@@ -2585,9 +2705,9 @@ int dage_gbfmm_apply(dage_gbfmm *g, const double *rho, double *V, unsigned flags
   DAGE_TRY(single_setup(g, d_rho, d_V, g->near16set == nullptr));
   const GInst *d_inst = g->d_inst.as<GInst>();
   DAGE_CUDA_TRY(cudaMemsetAsync(d_V, 0, sizeof(double) * n, s));
-  DAGE_TRY(run_multipoles(d_inst, 1, g->nbox, g->lmax, g->nslab, g->kappa > 0.0, s));
+  DAGE_TRY(run_multipoles(d_inst, 1, g->nbox, g->nshtiles, g->lmax, g->nslab, s));
   DAGE_TRY(run_m2m(d_inst, 1, g, s));
-  DAGE_TRY(run_m2l(d_inst, 1, g->nbtot, g->N, s));
+  DAGE_TRY(run_m2l(d_inst, 1, g->nbtot, g->N, (long long)g->nbox * g->nslab, s));
   DAGE_TRY(run_l2l(d_inst, 1, g, s));
   if (g->near16set) {
     DAGE_TRY(near_f16_set_run(g->near16set, s));
@@ -2598,7 +2718,7 @@ int dage_gbfmm_apply(dage_gbfmm *g, const double *rho, double *V, unsigned flags
                               g->d_desc[2].as<StageDesc>()};
     DAGE_TRY(run_near(dd, g->nbox, mt, nt, g->P, g->w, g->tile_n, s));
   }
-  DAGE_TRY(run_l2p(d_inst, 1, g->nbox, g->lmax, max_owned(g), nullptr, g->kappa > 0.0, s));
+  DAGE_TRY(run_l2p(d_inst, 1, g->nshtiles, g->lmax, nullptr, s));
   if (flags & DAGE_ENERGY) DAGE_TRY(run_energy(d_inst, 1, g->d_energy.as<double>(), s));
   if (!(flags & DAGE_DEVICE_PTRS))
     DAGE_CUDA_TRY(cudaMemcpyAsync(V, d_V, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -2620,8 +2740,7 @@ int dage_gbfmm_multipole_moments(dage_gbfmm *g, const double *rho, unsigned flag
   double *d_V;
   DAGE_TRY(stage_io(g, rho, nullptr, flags & DAGE_DEVICE_PTRS, &d_rho, &d_V));
   DAGE_TRY(single_setup(g, d_rho, nullptr, false));
-  DAGE_TRY(run_multipoles(g->d_inst.as<GInst>(), 1, g->nbox, g->lmax, g->nslab, g->kappa > 0.0,
-                          g->stream));
+  DAGE_TRY(run_multipoles(g->d_inst.as<GInst>(), 1, g->nbox, g->nshtiles, g->lmax, g->nslab, g->stream));
   DAGE_CUDA_TRY(cudaMemcpyAsync(moments, g->d_q.as<double>() + (size_t)g->fine_off * g->N,
                                 sizeof(double) * g->nbox * g->N,
                                 cudaMemcpyDeviceToHost, g->stream));
@@ -2655,8 +2774,7 @@ int dage_gbfmm_evaluate_le(dage_gbfmm *g, const double *local_expansions, double
     d_V = g->d_V.as<double>();
   }
   DAGE_TRY(single_setup(g, nullptr, d_V, false));
-  DAGE_TRY(run_l2p(g->d_inst.as<GInst>(), 1, g->nbox, g->lmax, max_owned(g), dL.as<double>(),
-                   g->kappa > 0.0, s));
+  DAGE_TRY(run_l2p(g->d_inst.as<GInst>(), 1, g->nshtiles, g->lmax, dL.as<double>(), s));
   if (!(flags & DAGE_DEVICE_PTRS))
     DAGE_CUDA_TRY(cudaMemcpyAsync(V, d_V, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   DAGE_CUDA_TRY(cudaStreamSynchronize(s));

@@ -147,27 +147,6 @@ int launch_tmatrix(const TmatArgs &a, int nlip, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 constexpr int BM = kFp64TileM, BK = 16, SROW = BK + 4, NST = 3;
 
-__device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool pred) {
-  const uint32_t sa = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sa), "l"(gmem),
-               "r"(pred ? 8 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-// D(8x8) += A(8x4, row) B(4x8, col); lane l holds A[l/4][l%4], B[l%4][l/4]
-// and D[l/4][2(l%4) + {0,1}]
-__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 template <int TN>
 constexpr int stage_smem() {
   return NST * (BM + TN) * SROW * (int)sizeof(double);
