@@ -198,13 +198,20 @@ __device__ __forceinline__ void stage_tile(const StageDesc &d, const double *X, 
   // this thread copies rows (tid >> 4) + 16 i at K offset tid & 15; row
   // offsets are relative to row m0 (a tile spans 128 rows: 32 bits do)
   const int kk = tid & 15;
+  // (one division for the first row, then steps of 16 rows with carries)
   const uint32_t ad0 = (uint32_t)d.a_d0;
-  const long long abase = ((uint32_t)m0 % ad0) * d.a_s1 + ((uint32_t)m0 / ad0) * d.a_s2;
+  const uint32_t mq = (uint32_t)m0 / ad0, mr = (uint32_t)m0 - mq * ad0;
+  const long long abase = mr * d.a_s1 + mq * d.a_s2;
   int aoff[8];
+  {
+    const int s1 = (int)d.a_s1, s2 = (int)d.a_s2;
+    uint32_t r = mr + (tid >> 4), q = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t m = m0 + (tid >> 4) + 16 * i;
-    aoff[i] = m < (uint32_t)d.M ? (int)((m % ad0) * d.a_s1 + (m / ad0) * d.a_s2 - abase) : -1;
+    for (int i = 0; i < 8; ++i) {
+      while (r >= ad0) r -= ad0, ++q;
+      aoff[i] = m0 + (tid >> 4) + 16 * i < d.M ? ((int)r - (int)mr) * s1 + (int)q * s2 : -1;
+      r += 16;
+    }
   }
   const int nrow = n0 + (tid >> 4);
   const double *xb = X + abase + kk;
@@ -277,11 +284,13 @@ __device__ __forceinline__ void stage_tile(const StageDesc &d, const double *X, 
   cp_async_wait<0>();
 
   const uint32_t od0 = (uint32_t)d.o_d0;
+  uint32_t orow0 = m0 + wm + (lane >> 2), oq = orow0 / od0, orr = orow0 - oq * od0;
 #pragma unroll
   for (int mb = 0; mb < MB; ++mb) {
-    const uint32_t m = m0 + wm + mb * 8 + (lane >> 2);
-    if (m >= (uint32_t)d.M) continue;
-    double *orow = out + (m % od0) * d.o_s1 + (m / od0) * d.o_s2;
+    if (orow0 + mb * 8 >= (uint32_t)d.M) break;
+    while (orr >= od0) orr -= od0, ++oq;
+    double *orow = out + orr * d.o_s1 + oq * d.o_s2;
+    orr += 8;
 #pragma unroll
     for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
