@@ -182,7 +182,7 @@ __device__ __forceinline__ void split_pair_f32(float2 v, float2 m, __nv_bfloat16
 // bytes move 22 B/cycle per SM whatever the source; bulk copies of 16 KB moved
 // 54 (L2-resident source, 148 SMs at once: 15.4 TB/s), 8 KB 43, 32 KB 61.
 // With the column windows below and a warp-uniform MMA issue loop, 481^3
-// fp16x3 takes 45.3 ms per apply (67.0 before), 253^3 bf16x6 10.1 (11.6).
+// fp16x3 takes 45.3 ms per apply (67.0 before), 253^3 bf16x6 10.0 (11.6).
 constexpr int kAtomRows = 8;
 template <int NSX>
 constexpr int atom_bytes() {
@@ -223,6 +223,11 @@ struct StageArgs {
   // wcoef[g].
   // Intermediate stages: ng = 1.
   int ng;
+  // Intermediate stages: tiles of np t-points in one launch, t-point slowest;
+  // slot pt reads outer index + pt * xslot, the pt-th matrix and run lists,
+  // gscale[pt], and writes out + pt * oslot.  Last stage: np = 1.
+  int np, xslot;
+  long long oslot;
   const float *scale;    // s_n, row scales of the t-points (bf16x6)
   const float *wcoef;    // w_p of the t-points (device)
   // FP16 intermediate stages: the stage's power-of-two output factor (device
@@ -276,27 +281,32 @@ __device__ __forceinline__ void corr_product(int nsx, int i, int &a, int &b) {
 }
 
 // The tiles of one CTA, blockIdx.x + i gridDim.x, as (n-tile, row block, outer
-// index): the decoding divides once, then adds with carries.
+// index, t-point slot): the decoding divides once, then adds with carries.
 struct TileWalk {
-  int nt, rb, r1, left;
-  int dnt, drb, dr1;
+  int nt, rb, r1, pt, left;
+  int dnt, drb, dr1, dpt;
   __device__ __forceinline__ explicit TileWalk(const StageArgs &a) {
-    split(a, blockIdx.x, nt, rb, r1);
-    split(a, gridDim.x, dnt, drb, dr1);
+    split(a, blockIdx.x, nt, rb, r1, pt);
+    split(a, gridDim.x, dnt, drb, dr1, dpt);
     left = (a.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1;  // grid <= ntiles
   }
-  __device__ static void split(const StageArgs &a, int t, int &n, int &b, int &o) {
+  __device__ static void split(const StageArgs &a, int t, int &n, int &b, int &o, int &p) {
     n = t % a.n_ntiles;
-    b = t / a.n_ntiles % a.nrb;
-    o = t / a.n_ntiles / a.nrb;
+    t /= a.n_ntiles;
+    b = t % a.nrb;
+    t /= a.nrb;
+    o = t % a.outer;
+    p = t / a.outer;
   }
   __device__ __forceinline__ void next(const StageArgs &a) {
     --left;
     nt += dnt;
     rb += drb;
     r1 += dr1;
+    pt += dpt;
     if (nt >= a.n_ntiles) nt -= a.n_ntiles, ++rb;
     if (rb >= a.nrb) rb -= a.nrb, ++r1;
+    if (r1 >= a.outer) r1 -= a.outer, ++pt;
   }
 };
 
@@ -467,7 +477,11 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
     *abort_flag = 1;
     atomicCAS(a.err, 0, 1);
   };
-  auto run_list = [&](int gi, int nt) { return a.runs + (size_t)(gi * a.n_ntiles + nt) * (a.nkb + 1); };
+  // run list of sub-problem or slot i (past the last tile's slot: the last one's)
+  const int imost = (FINAL ? a.ng : a.np) - 1;
+  auto run_list = [&](int i, int nt) {
+    return a.runs + (size_t)(min(i, imost) * a.n_ntiles + nt) * (a.nkb + 1);
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -481,9 +495,9 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
         const uint32_t abytes = min(16, a.natA - 16 * t.rb) * C::kAtom;
         const int bmost = a.natB - 16 * t.nt;  // row atoms of the matrix from this n-tile on
         for (int gi = 0; gi < a.ng; ++gi) {
-          const uint8_t *xa = a.X + ((size_t)(t.r1 + gi * a.outer) * a.nkb * a.natA + 16 * t.rb) * C::kAtom;
-          const uint8_t *tb = a.T + ((size_t)gi * a.nkb * a.natB + 16 * t.nt) * C::kAtom;
-          const uint32_t *rw = run_list(gi, t.nt);
+          const uint8_t *xa = a.X + ((size_t)(t.r1 + gi * a.outer + t.pt * a.xslot) * a.nkb * a.natA + 16 * t.rb) * C::kAtom;
+          const uint8_t *tb = a.T + ((size_t)(gi + t.pt) * a.nkb * a.natB + 16 * t.nt) * C::kAtom;
+          const uint32_t *rw = run_list(gi + t.pt, t.nt);
           for (uint32_t w = __ldg(rw), wn; w != kRunEnd; w = wn) {
             wn = __ldg(++rw);
             const int kb = run_block(w), g0 = run_first(w);
@@ -529,13 +543,13 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
       uint64_t da = dbase;
       constexpr uint32_t kIdesc = idesc_f16kind<F16>(BM, 0);
       TileWalk t(a);
-      const uint32_t *rw = run_list(0, t.nt);
+      const uint32_t *rw = run_list(t.pt, t.nt);
       uint32_t w = __shfl_sync(0xffffffffu, __ldg(rw), 0);
       while (t.left > 0 && ok && !*abort_flag) {
         for (int gi = 0; gi < a.ng && ok; ++gi) {
           // the first run of the next sub-problem, loaded while this one's MMAs run
           if (gi == a.ng - 1) t.next(a);
-          const uint32_t *rnext = run_list(gi == a.ng - 1 ? 0 : gi + 1, t.nt);
+          const uint32_t *rnext = run_list(gi == a.ng - 1 ? t.pt : gi + 1, t.nt);
           const uint32_t wfirst = __ldg(rnext);
           if (!FOLD && !mbar_wait_warp(cempty, tph, a.wait_limit)) {
             if (leader) on_timeout();
@@ -592,7 +606,6 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
     // fp16x3 scales each t-point's matrix by one power of two, folded into
     // the stage factor gfac.
     constexpr bool kColScale = NSX > 2;
-    const float gfac = (F16 && !FINAL) ? *a.gscale : 1.0f;
     const int q = warp & 3;
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
     const int grp = (warp - 2) >> 2;
@@ -618,9 +631,10 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
       const int ncol = n0 + lane;  // this lane's column
       // intermediate stages: the scale of column ncol, loaded before the
       // partial drains so its latency overlaps them
-      const float scl = (!FINAL && kColScale && ncol < a.N) ? a.scale[ncol] : 0.0f;
+      const float scl = (!FINAL && kColScale && ncol < a.N) ? a.scale[(size_t)t.pt * a.N + ncol] : 0.0f;
+      const float gfac = (F16 && !FINAL) ? a.gscale[t.pt] : 1.0f;
       for (int gi = 0; gi < a.ng && ok; ++gi) {
-        const uint32_t *rw = run_list(gi, t.nt);
+        const uint32_t *rw = run_list(gi + t.pt, t.nt);
         uint32_t w = __ldg(rw);
         // last stage: w_p [s_n of column ncol] for sub-problem gi
         float fcol = FINAL ? a.wcoef[gi] : 0.0f;
@@ -704,7 +718,7 @@ __global__ void __maxnreg__(96) stage_bf16_kernel(const __grid_constant__ StageA
         // padding; lanes beyond it store nothing.)
         const bool odd = lane & 1;
         const size_t nstep = (size_t)a.nkbN * a.natN * (C::kAtom / 2);
-        __nv_bfloat16 *dst = a.out + ((size_t)kbk * a.natN + (r1 >> 3)) * (C::kAtom / 2) +
+        __nv_bfloat16 *dst = a.out + t.pt * a.oslot + ((size_t)kbk * a.natN + (r1 >> 3)) * (C::kAtom / 2) +
                              atom_off(r1, lane & ~1, 0) + nstep * (n0 + (odd ? 1 : 0));
         const bool live = (r0 & ~1) < a.d0;
         const int nv = min(CW, a.N - n0);
@@ -956,6 +970,7 @@ struct MixedState {
   int nparts = 2;   // parts per operand
   int G = 1;        // t-points per pass of the last stage (used slots of X[2])
   int Gmax = 1;     // allocated slots of X[2]
+  int Gi = 1;       // t-points per launch of the first two stages (slots of X[1])
   int ns = 6;       // copy/MMA ring stages of the stage kernel (autotuned)
   DevBuf wdev;      // w_p as FP32 on the device
   // stage inputs: rows d0 (natA atoms), outer indices, K blocks
@@ -974,9 +989,9 @@ struct MixedState {
   DevBuf l1[3], psc[3], w64, maxbits, gin, g01, wcoef;
 };
 
-// One stage launch over ng t-points from p on.
+// One stage launch over n t-points from p on.
 template <int NSX, int NS, bool FINAL, bool F16>
-int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int ng, StageArgs a,
+int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int n, StageArgs a,
                  cudaStream_t s) {
   using C = StageCfg<NSX, NS, F16>;
   auto kern = stage_bf16_kernel<NSX, NS, FINAL, F16>;
@@ -992,7 +1007,9 @@ int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int ng, 
   a.d0 = st.d0[stage];
   a.outer = st.outer[stage];
   a.nrb = ceil_div(a.d0, BM);
-  a.ntiles = a.outer * a.nrb * a.n_ntiles;
+  a.ng = FINAL ? n : 1;
+  a.np = FINAL ? 1 : n;
+  a.ntiles = a.outer * a.nrb * a.n_ntiles * a.np;
   a.nkb = st.nkb[stage];
   a.natA = st.natA[stage];
   a.natB = st.natB[ow];
@@ -1000,7 +1017,6 @@ int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int ng, 
   a.T = st.Tp[ow].as<uint8_t>() + (size_t)p * st.tbytes[ow];
   a.runs = st.runs[ow].as<uint32_t>() + (size_t)p * a.n_ntiles * (a.nkb + 1);
   a.scale = st.sc[ow].as<float>() + (size_t)p * a.N;
-  a.ng = ng;
   const int grid = std::min(a.ntiles, sm_count());
   kern<<<grid, kThreads, C::kSmem, s>>>(a);
   DAGE_CUDA_TRY(cudaGetLastError());
@@ -1037,31 +1053,33 @@ int run_stages(dage_op3d *op, MixedState &st, const double *d_rho, double *d_V, 
   base.err = st.err.as<int>();
   base.wait_limit = g_wait_limit;
   base.drain_limit = 4000000000LL;  // ~2 s: copies and MMAs in flight always finish
-  int p0 = 0;  // first t-point of the open group
-  for (int p = 0; p < op->P; ++p) {
-    for (int stage = 0; stage < 2; ++stage) {
-      StageArgs a = base;
-      // last-stage input: slot p % G of X[2]
-      a.out = reinterpret_cast<__nv_bfloat16 *>(
-          st.X[stage + 1].as<uint8_t>() + (stage == 1 ? (p % st.G) * st.xbytes[2] : 0));
-      a.nkbN = st.nkb[stage + 1];
-      a.natN = st.natA[stage + 1];
-      if (F16) a.gscale = st.g01.as<float>() + (size_t)stage * op->P + p;
-      const int t = op->tmark_begin(0);
-      DAGE_TRY((launch_stage<NSX, NS, false, F16>(op, st, stage, p, 1, a, s)));
-      op->tmark_end(t);
+  for (int p0 = 0; p0 < op->P; p0 += st.G) {  // groups of the last stage
+    const int ng = std::min(st.G, op->P - p0);
+    for (int q = 0; q < ng; q += st.Gi) {  // t-points of one intermediate launch
+      const int p = p0 + q, np = std::min(st.Gi, ng - q);
+      for (int stage = 0; stage < 2; ++stage) {
+        StageArgs a = base;
+        // slots of X[1]: one per t-point of the launch; of X[2]: of the group
+        a.out = reinterpret_cast<__nv_bfloat16 *>(st.X[stage + 1].as<uint8_t>() +
+                                                  (stage == 1 ? q * st.xbytes[2] : 0));
+        a.oslot = (long long)(st.xbytes[stage + 1] / 2);
+        a.xslot = stage == 0 ? 0 : st.outer[1];
+        a.nkbN = st.nkb[stage + 1];
+        a.natN = st.natA[stage + 1];
+        if (F16) a.gscale = st.g01.as<float>() + (size_t)stage * op->P + p;
+        const int t = op->tmark_begin(0);
+        DAGE_TRY((launch_stage<NSX, NS, false, F16>(op, st, stage, p, np, a, s)));
+        op->tmark_end(t);
+      }
     }
-    if (p - p0 + 1 == st.G || p == op->P - 1) {
-      StageArgs a = base;
-      a.wcoef = (F16 ? st.wcoef.as<float>() : st.wdev.as<float>()) + p0;
-      a.V = d_V;
-      a.vn = (long long)op->nout[0] * op->nout[1];
-      a.accumulate = p0 > 0;
-      const int t = op->tmark_begin(0);
-      DAGE_TRY((launch_stage<NSX, NS, true, F16>(op, st, 2, p0, p - p0 + 1, a, s)));
-      op->tmark_end(t);
-      p0 = p + 1;
-    }
+    StageArgs a = base;
+    a.wcoef = (F16 ? st.wcoef.as<float>() : st.wdev.as<float>()) + p0;
+    a.V = d_V;
+    a.vn = (long long)op->nout[0] * op->nout[1];
+    a.accumulate = p0 > 0;
+    const int t = op->tmark_begin(0);
+    DAGE_TRY((launch_stage<NSX, NS, true, F16>(op, st, 2, p0, ng, a, s)));
+    op->tmark_end(t);
   }
   return 0;
 }
@@ -1123,6 +1141,18 @@ int mixed_setup(dage_op3d *op) {
   // rows and outer indices of the three stages: (y, z), (z, x), (x, y)
   const int rows[3] = {op->nin[1], op->nin[2], op->nout[0]};
   const int outer[3] = {op->nin[2], op->nout[0], op->nout[1]};
+  // t-points per launch of the first two stages: a small cube has fewer tiles
+  // than SMs (25^3: 25, 121^3: 121), so as many as it takes for eight tiles on
+  // every SM, or as leave X[1] in a third of the L2 (121^3, 40 t-points: 0.95 ->
+  // 0.51 ms per apply, 25^3 0.33 -> 0.14, 181^3 2.33 -> 2.11; 481^3: one)
+  {
+    const double tiles = std::min((double)outer[0] * ceil_div(rows[0], BM) * ceil_div(op->nout[0], BN),
+                                  (double)outer[1] * ceil_div(rows[1], BM) * ceil_div(op->nout[1], BN));
+    const double bytes = 2.0 * st->nparts * outer[1] * rows[1] * op->nin[1];
+    const double want = std::max(8.0 * sm_count() / tiles, 42e6 / bytes);
+    st->Gi = std::max(1, (int)std::min((double)st->Gmax, std::ceil(want)));
+    if (bytes * st->Gi > (double)(1 << 30)) st->Gi = 1;
+  }
   for (int s = 0; s < 3; ++s) {
     const long long tiles = (long long)outer[s] * ceil_div(rows[s], BM) * ceil_div(op->nout[s], BN);
     if (tiles * st->Gmax >= (1LL << 31) || op->nin[s] >= (1 << 20))
@@ -1133,7 +1163,12 @@ int mixed_setup(dage_op3d *op) {
     st->natA[s] = ceil_div(rows[s], kAtomRows);
     st->xbytes[s] = (size_t)outer[s] * st->nkb[s] * st->natA[s] * (st->nparts * kAtomRows * BK * 2);
     // padding rows and K columns are never written: they stay zero
-    DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : 1)));
+    if (s == 1 && st->Gi > 1 && st->X[1].alloc(st->xbytes[1] * st->Gi)) {
+      cudaGetLastError();  // a group that does not fit the free memory becomes one t-point
+      clear_error();
+      st->Gi = 1;
+    }
+    DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : s == 1 ? st->Gi : 1)));
     DAGE_CUDA_TRY(cudaMemsetAsync(st->X[s].ptr, 0, st->X[s].bytes, op->stream));
   }
   DAGE_TRY(st->err.alloc(sizeof(int)));
