@@ -61,6 +61,7 @@ constexpr int BKN = 64;            // K extent of one shared-memory stage (128-b
 constexpr int kNThreads = 576;     // 18 warps
 constexpr int kNEpiThreads = 512;  // warps 2-17
 constexpr int kNMaxGroup = 4;      // t-points summed per pass of the last stage (W slots)
+constexpr int kUSlots = 2;         // t-points of a stage-x launch (U slots)
 constexpr int kRowsA = 32, kRowsB = 4;  // tile rows: 32 along a x 4 along b
 static_assert(kRowsA * kRowsB == BM, "tile rows");
 
@@ -87,6 +88,9 @@ struct NearArgs {
   int nruns;
   int ntiles;
   int p;               // t-point (the group's first in the last stage)
+  int p2;              // stage x in pairs: the second t-point
+  int az0;             // added to the A outer coordinate (the U slot)
+  long long oslot;     // pairs: output elements between the two U slots
   int ng;              // last stage: t-points of the group (member gi reads slot gi)
   int slot_rows;       // last stage: A outer rows per slot
   const float *gscale; // intermediate: output factor of (inst, p) at gscale[inst * gstride + p]
@@ -150,10 +154,15 @@ __device__ __forceinline__ void near_mma_run(uint32_t P, uint64_t d0, uint32_t i
   umma_commit(pfull_bar);
 }
 
+// Stage x in pairs: its input does not depend on the t-point, so two t-points
+// can share a tile (its halves of TNW / 2 columns): half the A traffic per
+// output and half the per-tile work of every role.
+//
 // The units (tile, sub-problem) of one CTA in order: tiles blockIdx.x + i
 // gridDim.x, each with its ng t-points.  One vector of the current tile's
 // record, that of the next tile, and the runs of the current and the next unit
 // are in registers; every load is issued at least a unit before its use.
+template <bool PAIR>
 struct UnitWalk {
   int tile, gi;
   int4 mid, midn;  // second vector of the record: runs, bps, inst, dims
@@ -162,7 +171,11 @@ struct UnitWalk {
     return __ldg(a.tiles + 3 * (size_t)min(t, a.ntiles - 1) + i);
   }
   __device__ __forceinline__ uint32_t runs_of(const NearArgs &a, const int4 &m, int g) const {
-    return __ldg(a.runs + (size_t)(a.p + g) * a.nruns + m.x);
+    const uint32_t r = __ldg(a.runs + (size_t)(a.p + g) * a.nruns + m.x);
+    if (!PAIR) return r;
+    // union of the two t-points' ranges
+    const uint32_t o = __ldg(a.runs + (size_t)a.p2 * a.nruns + m.x);
+    return min(r & 0xffff, o & 0xffff) | max(r & 0xffff0000u, o & 0xffff0000u);
   }
   __device__ __forceinline__ explicit UnitWalk(const NearArgs &a) : tile(blockIdx.x), gi(0) {
     mid = vec(a, tile, 1);
@@ -185,7 +198,7 @@ struct UnitWalk {
   }
 };
 
-template <bool FINAL, int TNW, int NS>
+template <bool FINAL, int TNW, int NS, bool PAIR>
 __global__ void __maxnreg__(96)
     near_f16_kernel(const __grid_constant__ CUtensorMap mapA0,
                     const __grid_constant__ CUtensorMap mapA1,
@@ -240,10 +253,10 @@ __global__ void __maxnreg__(96)
       int issued[NS];
       uint32_t issued_ph[NS];
       for (int i = 0; i < NS; ++i) issued[i] = 0, issued_ph[i] = 0;
-      UnitWalk u(a);
+      UnitWalk<PAIR> u(a);
       int4 xy = u.vec(a, u.tile, 0), xyn = u.vec(a, u.tile + gridDim.x, 0);
       while (u.tile < a.ntiles && !*abort_flag) {
-        const int az = xy.z + u.gi * a.slot_rows;
+        const int az = xy.z + a.az0 + u.gi * a.slot_rows;
         const int brow = xy.w + (a.p + u.gi) * u.mid.y;
         const int k1 = (int)(u.r >> 17);  // last K block of 64
         for (int kb = (int)(u.r & 0xffff) >> 1; kb <= k1; ++kb) {
@@ -257,6 +270,12 @@ __global__ void __maxnreg__(96)
           tma_load_3d(st + C::kABytes, &mapA1, full(s), xy.x + kb * BKN, xy.y, az);
           tma_load_2d(st + 2 * C::kABytes, &mapB0, full(s), kb * BKN, brow);
           tma_load_2d(st + 2 * C::kABytes + C::kBBytes, &mapB1, full(s), kb * BKN, brow);
+          if (PAIR) {  // the second half of both parts' rows: the second t-point
+            const int brow2 = xy.w + a.p2 * u.mid.y;
+            tma_load_2d(st + 2 * C::kABytes + C::kBBytes / 2, &mapB0, full(s), kb * BKN, brow2);
+            tma_load_2d(st + 2 * C::kABytes + C::kBBytes + C::kBBytes / 2, &mapB1, full(s),
+                        kb * BKN, brow2);
+          }
           issued[s] = 1;
           issued_ph[s] = ph;
           if (++s == NS) s = 0, ph ^= 1;
@@ -281,10 +300,10 @@ __global__ void __maxnreg__(96)
     bool ok = true;
     const uint64_t dbase = sdesc128(smem_u32(tiles));
     uint64_t da = dbase;
-    UnitWalk u(a);
+    UnitWalk<PAIR> u(a);
     while (u.tile < a.ntiles && ok && !*abort_flag) {
       const uint32_t runs = __shfl_sync(0xffffffffu, u.r, 0);
-      const int ncol = __shfl_sync(0xffffffffu, u.mid.w, 0) >> 16;
+      const int ncol = PAIR ? TNW : __shfl_sync(0xffffffffu, u.mid.w, 0) >> 16;
       const uint32_t idesc = idesc_f16kind<true>(BM, 0) | ((uint32_t)((ncol + 15) >> 4) << 18);
       const int r0 = runs & 0xffff, r1 = runs >> 16;
       for (int run = r0; run <= r1; ++run) {
@@ -322,9 +341,12 @@ __global__ void __maxnreg__(96)
     const uint32_t lane_off = (uint32_t)(32 * q) << 16;
     const uint32_t col0 = ((warp - 2) >> 2) * CW;
     const uint32_t taddr = tmem_base + lane_off + col0;
+    // pairs: this warp's t-point and its first column there
+    const int half = PAIR && col0 >= TNW / 2;
+    const int cn0 = PAIR ? (int)(col0 % (TNW / 2)) : (int)col0;
     int b = 0;
     uint32_t pph = 0;
-    UnitWalk u(a);
+    UnitWalk<PAIR> u(a);
     int4 to = u.vec(a, u.tile, 2), ton = u.vec(a, u.tile + gridDim.x, 2);
     float2 accg[CW / 2];
 #pragma unroll
@@ -332,7 +354,7 @@ __global__ void __maxnreg__(96)
     while (u.tile < a.ntiles) {
       const int na = u.mid.w & 0xff, nb = (u.mid.w >> 8) & 0xff, ncol = u.mid.w >> 16;
       const float f = FINAL ? a.wcoef[(size_t)u.mid.z * a.wstride + a.p + u.gi]
-                            : a.gscale[(size_t)u.mid.z * a.gstride + a.p];
+                            : a.gscale[(size_t)u.mid.z * a.gstride + (half ? a.p2 : a.p)];
       float2 acc[CW / 2];
 #pragma unroll
       for (int k = 0; k < CW / 2; ++k) acc[k] = make_float2(0.0f, 0.0f);
@@ -365,9 +387,10 @@ __global__ void __maxnreg__(96)
 #pragma unroll
         for (int k = 0; k < CW / 2; ++k) accg[k] = __ffma2_rn(make_float2(f, f), acc[k], accg[k]);
       }
-      const int nv = min(CW, ncol - (int)col0);  // this warp's columns
+      // this warp's columns (none for the second half of an unpaired t-point)
+      const int nv = half && a.p2 == a.p ? 0 : min(CW, ncol - cn0);
       const long long off = ((long long)(uint32_t)to.x | ((long long)to.y << 32)) + a.sb * q +
-                            a.sn * (long long)col0;
+                            a.sn * (long long)cn0 + (half ? a.oslot : 0);
       if (FINAL) {
         if (u.gi == a.ng - 1) {
           // V(a, b, n) (+)= the group's sum; one FP64 add per element per group
@@ -627,19 +650,20 @@ int make_map_3d(CUtensorMap *m, const void *base, long long inner, long long d1,
   return 0;
 }
 
-template <bool FINAL, int TNW, int NS>
+template <bool FINAL, int TNW, int NS, bool PAIR = false>
 int set_smem_attr() {
   using C = NearCfg<TNW, NS>;
-  DAGE_CUDA_TRY(cudaFuncSetAttribute(near_f16_kernel<FINAL, TNW, NS>,
+  DAGE_CUDA_TRY(cudaFuncSetAttribute(near_f16_kernel<FINAL, TNW, NS, PAIR>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
   return 0;
 }
 
-template <bool FINAL, int TNW, int NS>
+template <bool FINAL, int TNW, int NS, bool PAIR = false>
 int launch_near(const CUtensorMap *mA, const CUtensorMap *mB, const NearArgs &a, cudaStream_t s) {
   using C = NearCfg<TNW, NS>;
   const int grid = std::min(a.ntiles, sm_count());
-  near_f16_kernel<FINAL, TNW, NS><<<grid, kNThreads, C::kSmem, s>>>(mA[0], mA[1], mB[0], mB[1], a);
+  near_f16_kernel<FINAL, TNW, NS, PAIR>
+      <<<grid, kNThreads, C::kSmem, s>>>(mA[0], mA[1], mB[0], mB[1], a);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -678,6 +702,9 @@ struct NearF16Set {
   DevBuf maxbits, gin, g01, wcoef, rhoptr, wptr, vptr;
   long long sb[3] = {0, 0, 0}, sn[3] = {0, 0, 0};  // output strides of a b row and a column
   CUtensorMap mapA[3][2], mapB[3][2];
+  // stage x of two t-points per tile: 0 none, else the columns of each half
+  int xhalf = 0;
+  CUtensorMap mapBx[2];         // its matrix tiles of xhalf rows
   DevBuf err;
 };
 
@@ -686,6 +713,8 @@ int near_f16_prepare() {
   DAGE_TRY((set_smem_attr<true, 64, 4>()));
   DAGE_TRY((set_smem_attr<false, 128, 3>()));
   DAGE_TRY((set_smem_attr<true, 128, 3>()));
+  DAGE_TRY((set_smem_attr<false, 64, 4, true>()));
+  DAGE_TRY((set_smem_attr<false, 128, 3, true>()));
   return 0;
 }
 
@@ -810,7 +839,7 @@ void near_f16_set_sizes(const NearF16Plan *pl, const std::vector<NearBox> &boxes
                         size_t bytes[3]) {
   const SetDims d = set_dims(pl, boxes, n);
   bytes[0] = sizeof(__half) * 2 * ((size_t)n * d.xs_rows * d.ld[0]);
-  bytes[1] = sizeof(__half) * 2 * ((size_t)d.xsl * d.zpad * d.ld[1]);
+  bytes[1] = sizeof(__half) * 2 * ((size_t)kUSlots * d.xsl * d.zpad * d.ld[1]);
   bytes[2] = sizeof(__half) * 2 * ((size_t)d.G * d.ysl * d.xpad * d.ld[2]);
 }
 
@@ -839,11 +868,11 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   st->ysl = d.ysl;
   st->xs_rows = d.xs_rows;
   st->G = d.G;
-  if (d.xsl >= (1LL << 31) / d.zpad || (long long)d.G * d.ysl >= (1LL << 31) / d.xpad ||
+  if (kUSlots * d.xsl >= (1LL << 31) / d.zpad || (long long)d.G * d.ysl >= (1LL << 31) / d.xpad ||
       (long long)n * g.npts[2] >= (1LL << 31))
     return fail(DAGE_E_INVALID, "near-field set too large for 32-bit tensor coordinates");
   const size_t xe = (size_t)n * d.xs_rows * d.ld[0];
-  const size_t ue = (size_t)d.xsl * d.zpad * d.ld[1];
+  const size_t ue = (size_t)kUSlots * d.xsl * d.zpad * d.ld[1];
   const size_t we = (size_t)d.G * d.ysl * d.xpad * d.ld[2];
   if (ws) {  // shared workspace (sets that run one after another)
     st->xp = static_cast<__half *>(ws[0]);
@@ -877,7 +906,7 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   for (int part = 0; part < 2; ++part) {
     DAGE_TRY(make_map_3d(&st->mapA[0][part], x0 + part * xe, g.npts[0], g.npts[1],
                          (long long)n * g.npts[2], d.ld[0], g.npts[1]));
-    DAGE_TRY(make_map_3d(&st->mapA[1][part], u0 + part * ue, d.ld[1], d.zpad, d.xsl, d.ld[1],
+    DAGE_TRY(make_map_3d(&st->mapA[1][part], u0 + part * ue, d.ld[1], d.zpad, kUSlots * d.xsl, d.ld[1],
                          d.zpad));
     DAGE_TRY(make_map_3d(&st->mapA[2][part], w0 + part * we, d.ld[2], d.xpad,
                          (long long)d.G * d.ysl, d.ld[2], d.xpad));
@@ -887,6 +916,17 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
                            pl->rows[s], pl->ldb[s], tile_n));
     }
   }
+  // Two t-points per stage-x tile: with at most 32 own points they share a
+  // 64-column tile (61^3 1.63 -> 1.36 ms an apply, 121^3 3.42 -> 2.94), up to 49
+  // a 128-column one (181^3 9.95 -> 9.19); above that the wider tile's drains
+  // cost more than the shared input saves (241^3 16.1 -> 18.3).
+  st->xhalf = tile_n != 64 ? 0 : pl->maxown[0] <= 32 ? 32 : pl->maxown[0] <= 49 ? 64 : 0;
+  if (st->xhalf)
+    for (int part = 0; part < 2; ++part) {
+      const size_t pe = (size_t)pl->rows[0] * pl->ldb[0];
+      DAGE_TRY(make_map_2d(&st->mapBx[part], pl->Bp[0].as<__half>() + part * pe, pl->ldb[0],
+                           pl->rows[0], pl->ldb[0], st->xhalf));
+    }
   // tiles: per job (density-major, then box), n-tile fastest, then a, then b
   const int tn = tile_n, w = tile_n == 128;
   std::vector<NearTile> tl[3];
@@ -992,7 +1032,7 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
       st->xp, st->xp + xe);
   DAGE_CUDA_TRY(cudaGetLastError());
 
-  const long long ue = st->xsl * st->zpad * st->ld[1];
+  const long long uslot = st->xsl * st->zpad * st->ld[1], ue = kUSlots * uslot;
   const long long we = (long long)st->G * st->ysl * st->xpad * st->ld[2];
   NearArgs base{};
   base.err = st->err.as<int>();
@@ -1011,15 +1051,20 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
     a.sb = st->sb[stage];
     a.sn = st->sn[stage];
     const CUtensorMap *mA = st->mapA[stage], *mB = st->mapB[stage];
+    if (stage == 0 && st->xhalf == 32) return launch_near<false, 64, 4, true>(mA, st->mapBx, a, s);
+    if (stage == 0 && st->xhalf == 64) return launch_near<false, 128, 3, true>(mA, st->mapBx, a, s);
     if (st->tile_n == 64)
       return fin ? launch_near<true, 64, 4>(mA, mB, a, s) : launch_near<false, 64, 4>(mA, mB, a, s);
     return fin ? launch_near<true, 128, 3>(mA, mB, a, s) : launch_near<false, 128, 3>(mA, mB, a, s);
   };
   for (int p = 0; p < P; ++p) {
     const int slot = p % st->G;
-    {  // stage x -> U
+    const bool pairs = st->xhalf > 0;
+    if (!pairs || p % 2 == 0) {  // stage x -> U
       NearArgs a = base;
       a.p = p;
+      a.p2 = std::min(p + 1, P - 1);
+      a.oslot = uslot;
       a.gscale = st->g01.as<float>();
       a.out0 = st->up;
       a.out1 = st->up + ue;
@@ -1028,6 +1073,7 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
     {  // stage y -> W slot
       NearArgs a = base;
       a.p = p;
+      a.az0 = pairs ? (int)(p % 2 * st->xsl) : 0;
       a.gscale = st->g01.as<float>() + P;
       a.out0 = st->wp + slot * st->ysl * st->xpad * st->ld[2];
       a.out1 = a.out0 + we;
