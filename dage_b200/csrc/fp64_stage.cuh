@@ -105,10 +105,11 @@ inline StageDesc cube_stage(const double *X, long long ldx, int M, int N, int K,
 // tile width in n (32, 64 or 128).
 int launch_fp64_stage(const StageDesc &d, int p0, int np, bool sum, double alpha, bool accumulate,
                       cudaStream_t s, int tn);
-// ndesc contractions from a device array, with the matrices of t-point p;
+// ndesc contractions from a device array, with the matrices of the t-points p
+// .. p + np - 1 (summed; their inputs x_ps apart), into output slot `slot`;
 // mtiles bounds the 128-row tile count and ncols the N of every descriptor.
-int launch_fp64_stages(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p,
-                       double alpha, bool accumulate, cudaStream_t s, int tn = 128);
+int launch_fp64_stages(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p, int np,
+                       int slot, double alpha, bool accumulate, cudaStream_t s, int tn);
 
 // Sets the shared-memory limits of every stage kernel variant (done lazily by
 // the launchers; call it before capturing launches into a CUDA graph).

@@ -1130,6 +1130,7 @@ struct dage_gbfmm {
   int nshtiles = 0;
   DevBuf d_U, d_W, d_desc[3];
   size_t U_per_box = 0, W_per_box = 0;
+  int near_g = 1;  // t-points per stage-z launch of the FP64 near field (W slots)
   std::vector<StageDesc> desc[3];
   int tile_n[3] = {64, 64, 64};  // near-field stage tile widths (autotuned)
   // fp16x3 near field on the tensor cores (near_mixed.cu): FP16 matrix
@@ -1425,6 +1426,22 @@ int build_m2l_into(const dage_gbfmm *g, double kappa, DevBuf &T) {
 }
 
 int build_m2l(dage_gbfmm *g) { return build_m2l_into(g, g->kappa, g->d_Tm2l); }
+
+// W slots for `doubles` values of W per t-point: up to 8 t-points in 256 MB.
+int near_group(int P, size_t doubles) {
+  return (int)std::max<size_t>(
+      1, std::min<size_t>({(size_t)P, 8, ((size_t)256 << 20) / std::max<size_t>(8 * doubles, 1)}));
+}
+
+// W for `G` slots; one where the memory does not hold the group.
+int alloc_near_w(DevBuf &W, size_t doubles, int &G) {
+  if (G > 1 && W.alloc(sizeof(double) * doubles * G)) {
+    cudaGetLastError();
+    clear_error();
+    G = 1;
+  }
+  return W.alloc(sizeof(double) * std::max<size_t>(doubles, 1) * G);
+}
 
 // Slabs of points of `work` (column tile, density) pairs: at most one per SM,
 // and eight blocks per SM where the pairs differ in size (uneven splits and
@@ -1841,7 +1858,8 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
   g->W_per_box = maxW;
   if (g->precision == DAGE_FP64) {  // the FP64 near field's intermediates
     DAGE_TRY(g->d_U.alloc(sizeof(double) * maxU * g->nbox));
-    DAGE_TRY(g->d_W.alloc(sizeof(double) * maxW * g->nbox));
+    g->near_g = near_group(g->P, maxW * g->nbox);
+    DAGE_TRY(alloc_near_w(g->d_W, maxW * g->nbox, g->near_g));
   }
   for (int d = 0; d < 3; ++d) {
     DAGE_TRY(g->wts[d].alloc(sizeof(double) * g->npts[d]));
@@ -1896,9 +1914,9 @@ GInst plan_inst(const dage_gbfmm *g, const double *rho, double *V, double *q, do
 
 // Appends the near-field stage descriptors of one density (one per box and
 // stage; t-point p reads its matrices at T + p * t_ps) with intermediates
-// U (U_per_box per box) and W (W_per_box per box).
+// U (U_per_box per box) and W (W_per_box per box; t-point slots wslot apart).
 void near_descs(const dage_gbfmm *g, const double *rho, double *V, double *U0, double *W0,
-                std::vector<StageDesc> ds[3]) {
+                size_t wslot, std::vector<StageDesc> ds[3]) {
   const int Nx = g->npts[0], Ny = g->npts[1];
   for (int b = 0; b < g->nbox; ++b) {
     const BoxInfo &B = g->boxes[b];
@@ -1959,6 +1977,7 @@ void near_descs(const dage_gbfmm *g, const double *rho, double *V, double *U0, d
     z.o_s1 = 1;
     z.o_s2 = Nx;
     z.o_sn = (long long)Nx * Ny;
+    y.o_ps = z.x_ps = (long long)wslot;
     ds[0].push_back(x);
     ds[1].push_back(y);
     ds[2].push_back(z);
@@ -2040,12 +2059,22 @@ int run_l2p(const GInst *d_inst, int ninst, int nshtiles, int lmax, const double
   return 0;
 }
 
+// Per t-point the stages x and y (W carries the weight w_p, or the descriptor's
+// own), per group of G t-points one stage z that sums over their W slots: V is
+// read and written once per group (121^3: a z launch of one t-point is 4 K
+// steps a block behind 32 reductions a thread, 60 us at 18 % of the tensor
+// pipe's rate).
 int run_near(const StageDesc *const d_desc[3], int njobs, const int mt[3], const int nt[3], int P,
-             const std::vector<double> &w, const int tile_n[3], cudaStream_t s) {
-  for (int p = 0; p < P; ++p)
-    for (int st = 0; st < 3; ++st)
-      DAGE_TRY(launch_fp64_stages(d_desc[st], njobs, mt[st], nt[st], p, st < 2 ? 1.0 : w[p],
-                                  st == 2 && p > 0, s, tile_n[st]));
+             const std::vector<double> &w, const int tile_n[3], int G, cudaStream_t s) {
+  for (int p0 = 0; p0 < P; p0 += G) {
+    const int np = std::min(G, P - p0);
+    for (int i = 0; i < np; ++i)
+      for (int st = 0; st < 2; ++st)
+        DAGE_TRY(launch_fp64_stages(d_desc[st], njobs, mt[st], nt[st], p0 + i, 1, st == 1 ? i : 0,
+                                    st == 1 ? w[p0 + i] : 1.0, false, s, tile_n[st]));
+    DAGE_TRY(launch_fp64_stages(d_desc[2], njobs, mt[2], nt[2], p0, np, 0, 1.0, p0 > 0, s,
+                                tile_n[2]));
+  }
   return 0;
 }
 
@@ -2058,11 +2087,11 @@ int run_energy(const GInst *d_inst, int ninst, double *d_out, cudaStream_t s) {
 }
 
 // Autotuner: the tile width (32, 64 or 128 columns) of each near-field
-// stage, chosen by timing every candidate on a batched launch of t-point 0
-// (one warm-up, three timed launches; the launches write the intermediates
+// stage, chosen by timing every candidate on a batched launch of t-point 0 (the
+// last stage: of the first group; one warm-up, three timed launches; the launches write the intermediates
 // and the output cubes of the descriptors, which the caller overwrites).
 int autotune_tiles(const StageDesc *const d_desc[3], int njobs, const int mt[3], const int nt[3],
-                   cudaStream_t s, int tile_n[3]) {
+                   int G, cudaStream_t s, int tile_n[3]) {
   cudaEvent_t e0, e1;
   DAGE_CUDA_TRY(cudaEventCreate(&e0));
   DAGE_CUDA_TRY(cudaEventCreate(&e1));
@@ -2073,7 +2102,8 @@ int autotune_tiles(const StageDesc *const d_desc[3], int njobs, const int mt[3],
     for (int tn : cand) {
       for (int r = 0; r < 4 && !rc; ++r) {
         if (r == 1) cudaEventRecord(e0, s);
-        rc = launch_fp64_stages(d_desc[st], njobs, mt[st], nt[st], 0, 1.0, false, s, tn);
+        rc = launch_fp64_stages(d_desc[st], njobs, mt[st], nt[st], 0, st == 2 ? G : 1, 0, 1.0, false,
+                                s, tn);
       }
       if (rc) break;
       cudaEventRecord(e1, s);
@@ -2114,7 +2144,8 @@ int gbfmm_autotune(dage_gbfmm *g) {
   DAGE_TRY(V.alloc(sizeof(double) * n));
   DAGE_CUDA_TRY(cudaMemsetAsync(rho.ptr, 0, sizeof(double) * n, s));
   std::vector<StageDesc> ds[3];
-  near_descs(g, rho.as<double>(), V.as<double>(), g->d_U.as<double>(), g->d_W.as<double>(), ds);
+  near_descs(g, rho.as<double>(), V.as<double>(), g->d_U.as<double>(), g->d_W.as<double>(),
+             g->W_per_box * g->nbox, ds);
   for (int d = 0; d < 3; ++d)
     DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_desc[d].ptr, ds[d].data(), sizeof(StageDesc) * g->nbox,
                                   cudaMemcpyHostToDevice, s));
@@ -2122,7 +2153,7 @@ int gbfmm_autotune(dage_gbfmm *g) {
   near_bounds(g, mt, nt);
   const StageDesc *dd[3] = {g->d_desc[0].as<StageDesc>(), g->d_desc[1].as<StageDesc>(),
                             g->d_desc[2].as<StageDesc>()};
-  const int rc = autotune_tiles(dd, g->nbox, mt, nt, s, g->tile_n);
+  const int rc = autotune_tiles(dd, g->nbox, mt, nt, g->near_g, s, g->tile_n);
   DAGE_CUDA_TRY(cudaStreamSynchronize(s));
   rho.release();
   V.release();
@@ -2248,7 +2279,7 @@ int single_setup(dage_gbfmm *g, const double *rho, double *V, bool near) {
   DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_inst.ptr, &I, sizeof(GInst), cudaMemcpyHostToDevice, g->stream));
   if (near) {
     std::vector<StageDesc> ds[3];
-    near_descs(g, rho, V, g->d_U.as<double>(), g->d_W.as<double>(), ds);
+    near_descs(g, rho, V, g->d_U.as<double>(), g->d_W.as<double>(), g->W_per_box * g->nbox, ds);
     for (int d = 0; d < 3; ++d)
       DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_desc[d].ptr, ds[d].data(), sizeof(StageDesc) * g->nbox,
                                     cudaMemcpyHostToDevice, g->stream));
@@ -2322,6 +2353,8 @@ struct dage_gbfmm_batch {
   };
   std::vector<Chunk> chunks;
   DevBuf U, W;
+  int near_g = 1;     // t-points per z launch: W slots, wslot doubles apart
+  size_t wslot = 0;
   // fp16x3 near field: sets of densities of one plan each, within the budget
   int precision = DAGE_FP64;
   struct MSet {
@@ -2510,7 +2543,9 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
   }
   b->chunks.push_back(std::move(cur));
   DAGE_TRY(b->U.alloc(sizeof(double) * std::max<size_t>(umax, 1)));
-  DAGE_TRY(b->W.alloc(sizeof(double) * std::max<size_t>(wmax, 1)));
+  b->wslot = wmax;
+  b->near_g = near_group(b->P, wmax);
+  DAGE_TRY(alloc_near_w(b->W, wmax, b->near_g));
   for (auto &c : b->chunks) {
     c.njobs = (c.i1 - c.i0) * b->nbox;
     for (auto &d : c.desc) DAGE_TRY(d.alloc(sizeof(StageDesc) * c.njobs));
@@ -2553,11 +2588,11 @@ int batch_tables(dage_gbfmm_batch *b, const double *const *rho, double *const *V
   for (auto &c : b->chunks) {
     std::vector<StageDesc> ds[3];
     for (int i = c.i0; i < c.i1; ++i) {
-      const size_t z0 = ds[2].size();
+      const size_t z0 = ds[1].size();
       near_descs(b->plans[b->plan_of[i]], rho[i], V[i], b->U.as<double>() + c.uoff[i - c.i0],
-                 b->W.as<double>() + c.woff[i - c.i0], ds);
-      if (b->kern_of[i] >= 0)  // this density's own t-point weights in the z stage
-        for (size_t e = z0; e < ds[2].size(); ++e) ds[2][e].wp = b->kerns[b->kern_of[i]].w.as<double>();
+                 b->W.as<double>() + c.woff[i - c.i0], b->wslot, ds);
+      if (b->kern_of[i] >= 0)  // this density's own t-point weights in the y stage
+        for (size_t e = z0; e < ds[1].size(); ++e) ds[1][e].wp = b->kerns[b->kern_of[i]].w.as<double>();
     }
     for (int d = 0; d < 3; ++d)
       DAGE_CUDA_TRY(cudaMemcpyAsync(c.desc[d].ptr, ds[d].data(), sizeof(StageDesc) * c.njobs,
@@ -2592,7 +2627,7 @@ int batch_launch(dage_gbfmm_batch *b, const double *const *rho, double *const *V
   for (auto &c : b->chunks) {
     const StageDesc *dd[3] = {c.desc[0].as<StageDesc>(), c.desc[1].as<StageDesc>(),
                               c.desc[2].as<StageDesc>()};
-    DAGE_TRY(run_near(dd, c.njobs, b->mt, b->nt, b->P, b->w, b->tile_n, s));
+    DAGE_TRY(run_near(dd, c.njobs, b->mt, b->nt, b->P, b->w, b->tile_n, b->near_g, s));
   }
   for (auto &m : b->msets) DAGE_TRY(near_f16_set_run(m.set, s));
   DAGE_TRY(run_l2p(d_inst, b->n, b->nshtiles, b->lmax, nullptr, s));
@@ -2716,7 +2751,7 @@ int dage_gbfmm_apply(dage_gbfmm *g, const double *rho, double *V, unsigned flags
     near_bounds(g, mt, nt);
     const StageDesc *dd[3] = {g->d_desc[0].as<StageDesc>(), g->d_desc[1].as<StageDesc>(),
                               g->d_desc[2].as<StageDesc>()};
-    DAGE_TRY(run_near(dd, g->nbox, mt, nt, g->P, g->w, g->tile_n, s));
+    DAGE_TRY(run_near(dd, g->nbox, mt, nt, g->P, g->w, g->tile_n, g->near_g, s));
   }
   DAGE_TRY(run_l2p(d_inst, 1, g->nshtiles, g->lmax, nullptr, s));
   if (flags & DAGE_ENERGY) DAGE_TRY(run_energy(d_inst, 1, g->d_energy.as<double>(), s));
@@ -2870,7 +2905,7 @@ int dage_gbfmm_batch_apply(dage_gbfmm_batch *b, const double *const *rho, double
         const auto &c = b->chunks[0];
         const StageDesc *dd[3] = {c.desc[0].as<StageDesc>(), c.desc[1].as<StageDesc>(),
                                   c.desc[2].as<StageDesc>()};
-        DAGE_TRY(autotune_tiles(dd, c.njobs, b->mt, b->nt, s, b->tile_n));
+        DAGE_TRY(autotune_tiles(dd, c.njobs, b->mt, b->nt, b->near_g, s, b->tile_n));
         tune_store(key, {b->tile_n[0], b->tile_n[1], b->tile_n[2]});
       }
       b->tuned = true;

@@ -324,11 +324,12 @@ __global__ void __launch_bounds__(256, stage_blocks<TN>())
 
 template <bool ACCUM, int TN>
 __global__ void __launch_bounds__(256, stage_blocks<TN>())
-    stage_fp64_batched_kernel(const StageDesc *__restrict__ descs, int nt, int p, double alpha) {
+    stage_fp64_batched_kernel(const StageDesc *__restrict__ descs, int nt, int p, int np, int slot,
+                              double alpha) {
   const StageDesc d = descs[blockIdx.z];
   const int m0 = (blockIdx.x / nt) * BM, n0 = (blockIdx.x % nt) * TN;
   if (m0 >= d.M || n0 >= d.N) return;  // uniform across the block
-  stage_tile<ACCUM, TN>(d, d.X, d.out, p, 1, d.wp ? d.wp[p] : alpha, m0, n0);
+  stage_tile<ACCUM, TN>(d, d.X, d.out + slot * d.o_ps, p, np, d.wp ? d.wp[p] : alpha, m0, n0);
 }
 
 // Band of each (t-point, kBandCols rows) of an axis matrix T[p][n][K]: the
@@ -478,14 +479,14 @@ int launch_single(const StageDesc &d, int p0, int np, bool sum, double alpha, cu
 }
 
 template <bool ACCUM, int TN>
-int launch_batched(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p,
-                   double alpha, cudaStream_t s) {
+int launch_batched(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p, int np,
+                   int slot, double alpha, cudaStream_t s) {
   auto kern = stage_fp64_batched_kernel<ACCUM, TN>;
   DAGE_TRY(prepare_fp64_stages());
   const int nt = ceil_div(ncols, TN);
   if ((long long)mtiles * nt >= (1LL << 31) || ndesc > 65535)
     return fail(DAGE_E_UNSUPPORTED, "batch too large");
-  kern<<<dim3(mtiles * nt, 1, ndesc), 256, stage_smem<TN>(), s>>>(d_descs, nt, p, alpha);
+  kern<<<dim3(mtiles * nt, 1, ndesc), 256, stage_smem<TN>(), s>>>(d_descs, nt, p, np, slot, alpha);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -505,12 +506,14 @@ int launch_fp64_stage(const StageDesc &d, int p0, int np, bool sum, double alpha
   return fail(DAGE_E_INVALID, "tile width %d", tn);
 }
 
-int launch_fp64_stages(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p,
-                       double alpha, bool accumulate, cudaStream_t s, int tn) {
+int launch_fp64_stages(const StageDesc *d_descs, int ndesc, int mtiles, int ncols, int p, int np,
+                       int slot, double alpha, bool accumulate, cudaStream_t s, int tn) {
   if (ndesc <= 0) return 0;
-#define DAGE_BATCHED(TNV)                                                                  \
-  return accumulate ? launch_batched<true, TNV>(d_descs, ndesc, mtiles, ncols, p, alpha, s) \
-                    : launch_batched<false, TNV>(d_descs, ndesc, mtiles, ncols, p, alpha, s)
+  if (np < 1 || np > kMaxPointGroup) return fail(DAGE_E_INVALID, "group of %d t-points", np);
+#define DAGE_BATCHED(TNV)                                                                           \
+  return accumulate                                                                                \
+             ? launch_batched<true, TNV>(d_descs, ndesc, mtiles, ncols, p, np, slot, alpha, s)     \
+             : launch_batched<false, TNV>(d_descs, ndesc, mtiles, ncols, p, np, slot, alpha, s)
   switch (tn) {
     case 32: DAGE_BATCHED(32);
     case 64: DAGE_BATCHED(64);
