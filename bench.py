@@ -316,24 +316,36 @@ def run_e2e(op, rho, n, npts, world, args):
                            "api": "dage_op3d_apply per step, host pointers"}}
 
 
-def band_fraction(T, bk=64, bn=128):
-    """Fraction of the dense K range that the stage kernels issue work for:
-    per t-point and 128-row tile of T (i_out, j_in, p), the K blocks of bk
-    between the first and last entry above 2^-64 of its row's power-of-two
-    scale (the kernels' band rule; identical for the three axes of a cube)."""
+def band_fraction(T, prec):
+    """Fraction of the dense product that the stage kernels issue, from the
+    kernels' band rule on the matrix T (i_out, j_in, p) (identical for the
+    three axes of a cube): a band per t-point and 32 output points, from the
+    first to the last entry above 2^-64 of its row's power-of-two scale
+    (fp16x3: the entries whose FP16 parts are not both zero).  FP64: each band
+    in units of 4 K.  Split precision: per tile of 128 and K block of 32 the
+    columns from the first to the last group whose band holds the block."""
     no, ni, P = T.shape
-    nkb = -(-ni // bk)
-    last = ni - (nkb - 1) * bk
     issued = 0.0
     for p in range(P):
         A = np.abs(T[:, :, p])
         s = np.exp2(np.ceil(np.log2(np.maximum(A.max(axis=1), 1e-300))))
         big = A > np.ldexp(s, -64)[:, None]
-        for t0 in range(0, no, bn):
-            cols = np.nonzero(big[t0:t0 + bn].any(axis=0))[0]
-            lo, hi = (cols[0] // bk, cols[-1] // bk) if cols.size else (0, 0)
-            k = (hi - lo) * bk + (last if hi == nkb - 1 else bk)
-            issued += min(bn, no - t0) * k
+        if prec == "fp16x3":
+            big &= (A * (2.0 ** 14 / s.max())).astype(np.float16) != 0
+        bands = []
+        for g0 in range(0, no, 32):
+            cols = np.nonzero(big[g0:g0 + 32].any(axis=0))[0]
+            bands.append((cols[0], cols[-1]) if cols.size else (0, 0))
+        if prec == "fp64":
+            issued += sum((hi // 4 - lo // 4 + 1) * 4 * min(32, no - 32 * g)
+                          for g, (lo, hi) in enumerate(bands))
+            continue
+        for t0 in range(0, len(bands), 4):
+            tile = [(lo // 32, hi // 32) for lo, hi in bands[t0:t0 + 4]]
+            for k in range(-(-ni // 32)):
+                inside = [g for g, (lo, hi) in enumerate(tile) if lo <= k <= hi]
+                if inside:
+                    issued += 32 * (min(32 * (t0 + inside[-1] + 1), no) - 32 * (t0 + inside[0]))
     return issued / (no * ni * P)
 
 
@@ -422,7 +434,7 @@ def run_gpu(args, world, rank, local):
     # one stage of one t-point: M = n^2, N = K = n; the last stage's launches
     # cover up to 8 t-points, so rates use the total stage time of an apply
     dense_flops = 2.0 * n ** 4 * nprod
-    band = band_fraction(op.matrix(0), bk=16 if prec == "fp64" else 32)
+    band = band_fraction(op.matrix(0), prec)
     stage_flops = dense_flops * band    # work the banded contraction issues
     stage_s = k_ms / args.steps / 1e3   # contraction kernels' time per apply
     apply_flops = 3 * (NLIN + NLOG) * stage_flops
@@ -632,6 +644,10 @@ def run_workload(args, world, rank, local):
         clk.start()
         ms = _timed(lambda: op.apply(rho, out=V, energy=True), args.steps, args.warmup, sync)
         clocks = clk.stop()
+        op.set_timing(True)
+        op.apply(rho, out=V, energy=True)
+        stage_launches = op.timing(0)[0]  # of one apply
+        op.set_timing(False)
         # analytic potential sum q erf(sqrt(a) r) / r at the grid points
         x = torch.tensor(axis_points(20, 0.2), dtype=torch.float64, device=dev)
         Z, Y, X = torch.meshgrid(x, x, x, indexing="ij")
@@ -643,7 +659,7 @@ def run_workload(args, world, rank, local):
         n = 121 ** 3
         _line(args, world, "Coulomb-op Mpts/s @121^3 FP64", n / ms / 1e3, "Mpts/s", ms, "f64",
               {"workload": wl, "points_per_axis": 121, "step_bohr": 0.2, "t_points": 40,
-               "gaussians": 2, "seed": SEED}, clocks, 3 * 40 + 2,
+               "gaussians": 2, "seed": SEED}, clocks, stage_launches + 2,
               {"accuracy": {"vs": "analytic sum q erf(sqrt(a) r)/r", "max_rel": err}})
     elif wl in ("gbfmm_241", "gbfmm_241_adaptive", "helmholtz_gbfmm_241", "helmholtz_gbfmm_241"):
         # GBFMM, 241^3 (40 cells, step 0.2), 4^3 boxes, lmax 12, 16 Gaussians
@@ -705,7 +721,10 @@ def run_workload(args, world, rank, local):
               "Mpts/s", ms, "f64" if prec == "fp64" else "f16",
               {"workload": wl, "points_per_axis": 241, "step_bohr": 0.2, "t_points": 40,
                "lmax": 12, "boxes": 64, "gaussians": 16, "seed": SEED, "precision": prec,
-               "near_field_tiles": list(op.tiles)}, clocks, 3 * 40 + 9, extra)
+               "near_field_tiles": list(op.tiles)}, clocks,
+              # near field (fp16x3: 40 + 40 + 10 stages and 3 of the scales and
+              # the split), moments, M2L, L2P, energy
+              (93 if prec != "fp64" else 120) + 7, extra)
     elif wl == "bubbles_inject_301":
         rng = np.random.default_rng(SEED)
         bub, gcube = _molecule_bubbles(dage, rng)
