@@ -25,7 +25,7 @@
 // to the union of the tile's ranges (entries outside are below 2^-64 of their
 // row's scale).  At 241^3, step 0.2, 40 t-points, ranges per 32 columns hold
 // 0.39 of the dense product against 0.71 for ranges per 128 columns in steps
-// of 16.  Measured per apply: 241^3, 40 t-points 27.6 -> 16.8 ms (tensor pipe
+// of 16.  Measured per apply: 241^3, 40 t-points 27.6 -> 16.5 ms (tensor pipe
 // active 71-77 %); 97x121x73, 18 t-points 0.98 -> 0.46 ms and 25^3 492 -> 97 us
 // (with the t-point groups).  With accumulation each output element gets one correctly rounded
 // FP64 add per launch (an L2 reduction; one writer per element).
