@@ -29,11 +29,11 @@
 #include <array>
 #include <limits>
 #include <map>
-#include <mutex>
 #include <vector>
 
 #include "fp64_stage.cuh"
 #include "near_mixed.cuh"
+#include "once_per_device.h"
 #include "tune.h"
 #include "op3d.cuh"
 
@@ -171,15 +171,9 @@ __constant__ double c_shA[kShSize];
 __constant__ double c_shB[kShSize];
 __constant__ double c_shC[kMaxLmax + 1];
 
-// Uploads the tables to the current device once per process and device
-// (called at plan creation, outside any stream capture).
-int sh_tables_init() {
-  static std::mutex mu;
-  static unsigned long long done = 0;  // one bit per device ordinal
-  int dev = 0;
-  DAGE_CUDA_TRY(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev < 64 && (done >> dev) & 1ull) return 0;
+// Uploads the tables to the current device (sh_tables_init: once per device;
+// called at plan creation, outside any stream capture).
+int sh_tables_upload() {
   double A[kShSize] = {}, B[kShSize] = {}, C[kMaxLmax + 1] = {};
   for (int l = 1; l <= kMaxLmax; ++l)
     for (int m = -(l - 1); m <= l - 1; ++m) {
@@ -207,8 +201,13 @@ int sh_tables_init() {
   // Without this wait a kernel could read zeros (a Bessel series cut to its
   // leading term, harmonics of zero).
   DAGE_CUDA_TRY(cudaDeviceSynchronize());
-  if (dev < 64) done |= 1ull << dev;
   return 0;
+}
+int sh_tables_init() {
+  static OncePerDevice once;
+  int dev = 0;
+  DAGE_CUDA_TRY(cudaGetDevice(&dev));
+  return once.run(dev, sh_tables_upload);
 }
 
 // ---------------------------------------------------------------------------
@@ -1349,19 +1348,19 @@ int sh_l2p_smem(int N, int *pts) {
   }
 }
 int sh_prepare() {
-  static std::mutex mu;
-  static bool done = false;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done) return 0;
-  int pts;
-  constexpr int kMax = (kMaxLmax + 1) * (kMaxLmax + 1);
-  int most = 0;
-  for (int l = 0; l <= kMaxLmax; ++l) most = std::max(most, sh_l2p_smem((l + 1) * (l + 1), &pts));
-  DAGE_CUDA_TRY(cudaFuncSetAttribute(multipoles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     sh_mp_smem(kMax)));
-  DAGE_CUDA_TRY(cudaFuncSetAttribute(l2p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  done = true;
-  return 0;
+  static OncePerDevice once;
+  int dev = 0;
+  DAGE_CUDA_TRY(cudaGetDevice(&dev));
+  return once.run(dev, [] {
+    int pts, most = 0;
+    constexpr int kMax = (kMaxLmax + 1) * (kMaxLmax + 1);
+    for (int l = 0; l <= kMaxLmax; ++l) most = std::max(most, sh_l2p_smem((l + 1) * (l + 1), &pts));
+    DAGE_CUDA_TRY(cudaFuncSetAttribute(
+        multipoles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sh_mp_smem(kMax)));
+    DAGE_CUDA_TRY(
+        cudaFuncSetAttribute(l2p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return 0;
+  });
 }
 
 // M2L matrix of every distinct displacement for the plan's kernel.

@@ -18,11 +18,11 @@
 #include <cmath>
 #include <cstdio>
 #include <string>
-#include <mutex>
 #include <cstring>
 
 #include "expo.cuh"
 #include "fp64_stage.cuh"
+#include "once_per_device.h"
 #include "op3d.cuh"
 #include "tune.h"
 
@@ -448,19 +448,18 @@ int attr_variants() {
 }
 
 int prepare_fp64_stages() {
-  // once per process
-  static std::mutex mu;
-  static bool done = false;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done) return 0;
-  DAGE_TRY((attr_variants<false, 32>()));
-  DAGE_TRY((attr_variants<true, 32>()));
-  DAGE_TRY((attr_variants<false, 64>()));
-  DAGE_TRY((attr_variants<true, 64>()));
-  DAGE_TRY((attr_variants<false, 128>()));
-  DAGE_TRY((attr_variants<true, 128>()));
-  done = true;
-  return 0;
+  static OncePerDevice once;
+  int dev = 0;
+  DAGE_CUDA_TRY(cudaGetDevice(&dev));
+  return once.run(dev, [] {
+    DAGE_TRY((attr_variants<false, 32>()));
+    DAGE_TRY((attr_variants<true, 32>()));
+    DAGE_TRY((attr_variants<false, 64>()));
+    DAGE_TRY((attr_variants<true, 64>()));
+    DAGE_TRY((attr_variants<false, 128>()));
+    DAGE_TRY((attr_variants<true, 128>()));
+    return 0;
+  });
 }
 
 template <bool ACCUM, int TN>

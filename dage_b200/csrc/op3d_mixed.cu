@@ -77,6 +77,7 @@
 #include <vector>
 
 #include "fp64_stage.cuh"
+#include "once_per_device.h"
 #include "op3d.cuh"
 #include "tc_common.cuh"
 #include "tune.h"
@@ -995,12 +996,12 @@ int launch_stage(const dage_op3d *op, MixedState &st, int stage, int p, int n, S
                  cudaStream_t s) {
   using C = StageCfg<NSX, NS, F16>;
   auto kern = stage_bf16_kernel<NSX, NS, FINAL, F16>;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice once;
+  DAGE_TRY(once.run(op->device, [&] {
     DAGE_CUDA_TRY(
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem));
-    attr_set = true;
-  }
+    return 0;
+  }));
   const int ow = st.towner[stage];
   a.N = op->nout[stage];
   a.n_ntiles = ceil_div(a.N, BN);
