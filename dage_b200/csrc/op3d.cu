@@ -878,18 +878,26 @@ static int fp64_group(const dage_op3d *op) {
   return std::max(1, std::min({op->P, most, std::max(fill, l2)}));
 }
 
-// The intermediates of G t-points in one allocation (a first apply on a new
-// operator pays ~0.4 ms for each allocation above 1 MB): U, then W at nu.
-// Where a group does not fit the free memory it becomes a single t-point.
-static int fp64_workspace(const dage_op3d *op, DevBuf &buf, int &G, size_t &nu) {
+// The intermediates of a group of t-points in one allocation: U, then W.
+// Where a group does not fit the free memory it becomes a single t-point.  The
+// group is chosen once and kept with its memory: it sets the order of the sums
+// over the t-points, so applies of one operator agree to the last bit, and a
+// later apply frees and allocates nothing.  The tuner takes it at creation;
+// otherwise (its choice known already) the first apply does (~0.4 ms).
+static int fp64_workspace(dage_op3d *op) {
+  if (op->tmp_group) return 0;
   const size_t niy = op->nin[1], niz = op->nin[2], nox = op->nout[0], noy = op->nout[1];
-  for (;;) {
-    nu = G * niy * niz * nox;
-    const int rc = buf.alloc(sizeof(double) * (nu + G * niz * nox * noy));
-    if (!rc || G == 1) return rc;
+  for (int G = fp64_group(op);; G = 1) {
+    const size_t nu = G * niy * niz * nox;
+    const int rc = op->tmp.alloc(sizeof(double) * (nu + G * niz * nox * noy));
+    if (rc && G == 1) return rc;
+    if (!rc) {
+      op->tmp_group = G;
+      op->tmp_w = nu;
+      return 0;
+    }
     cudaGetLastError();
     clear_error();
-    G = 1;
   }
 }
 
@@ -898,8 +906,8 @@ static int fp64_workspace(const dage_op3d *op, DevBuf &buf, int &G, size_t &nu) 
 struct Fp64Stages {
   StageDesc d[3];
 };
-static Fp64Stages fp64_stages(const dage_op3d *op, const double *rho, double *U, double *W,
-                              double *V) {
+static Fp64Stages fp64_stages(const dage_op3d *op, const double *rho, double *V) {
+  double *U = op->tmp.as<double>(), *W = U + op->tmp_w;
   const int nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
   const int nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
   const int M[3] = {niy * niz, niz * nox, nox * noy}, N[3] = {nox, noy, noz},
@@ -938,18 +946,17 @@ static int tune_fp64(dage_op3d *op) {
   cudaStream_t s = op->stream;
   const size_t nix = op->nin[0], niy = op->nin[1], niz = op->nin[2];
   const size_t nox = op->nout[0], noy = op->nout[1], noz = op->nout[2];
-  int G = fp64_group(op);
-  TmpBuf X, U, V;
-  size_t nu;
+  TmpBuf X, V;
   DAGE_TRY(X.alloc(sizeof(double) * nix * niy * niz));
   DAGE_TRY(V.alloc(sizeof(double) * nox * noy * noz));
-  DAGE_TRY(fp64_workspace(op, U, G, nu));
+  DAGE_TRY(fp64_workspace(op));
+  const int G = op->tmp_group;
   DAGE_CUDA_TRY(cudaMemsetAsync(X.ptr, 0, X.bytes, s));
-  DAGE_CUDA_TRY(cudaMemsetAsync(U.ptr, 0, U.bytes, s));
+  DAGE_CUDA_TRY(cudaMemsetAsync(op->tmp.ptr, 0, op->tmp.bytes, s));
   cudaEvent_t e0, e1;
   DAGE_CUDA_TRY(cudaEventCreate(&e0));
   DAGE_CUDA_TRY(cudaEventCreate(&e1));
-  const Fp64Stages st = fp64_stages(op, X.as<double>(), U.as<double>(), U.as<double>() + nu, V.as<double>());
+  const Fp64Stages st = fp64_stages(op, X.as<double>(), V.as<double>());
   const int last = (op->P - 1) / G * G;
   const int ps[3] = {0, last / G / 2 * G, last};
   int rc = 0;
@@ -982,11 +989,9 @@ static int tune_fp64(dage_op3d *op) {
 
 static int apply_fp64(dage_op3d *op, const double *rho, double *V, bool accumulate) {
   cudaStream_t s = op->stream;
-  int G = fp64_group(op);
-  size_t nu;
-  DAGE_TRY(fp64_workspace(op, op->tmp, G, nu));
-  double *U = op->tmp.as<double>();
-  const Fp64Stages st = fp64_stages(op, rho, U, U + nu, V);
+  DAGE_TRY(fp64_workspace(op));
+  const int G = op->tmp_group;
+  const Fp64Stages st = fp64_stages(op, rho, V);
   for (int p = 0; p < op->P; p += G)
     for (int d = 0; d < 3; ++d) {
       const int t = op->tmark_begin(0);

@@ -33,7 +33,11 @@ struct dage_op3d {
   dage::DevBuf wts[3];
   dage::DevBuf d_w;          // weights w_p on the device
   dage::DevBuf d_rho, d_V;   // staging for host pointers
-  dage::DevBuf tmp;          // intermediates of the FP64 path, U then W
+  // intermediates of the FP64 path: U, then W at tmp_w, for tmp_group t-points
+  // (0: not allocated yet; chosen once, see fp64_workspace)
+  dage::DevBuf tmp;
+  int tmp_group = 0;
+  size_t tmp_w = 0;
   dage::DevBuf partials;     // energy reduction partial sums
 
   // FP64 path: contraction tile width (32, 64 or 128 output columns) of each
