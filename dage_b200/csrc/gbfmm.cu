@@ -24,6 +24,7 @@
 // no box).
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <array>
@@ -1426,10 +1427,11 @@ int build_m2l_into(const dage_gbfmm *g, double kappa, DevBuf &T) {
 
 int build_m2l(dage_gbfmm *g) { return build_m2l_into(g, g->kappa, g->d_Tm2l); }
 
-// W slots for `doubles` values of W per t-point: up to 8 t-points in 256 MB.
-int near_group(int P, size_t doubles) {
-  return (int)std::max<size_t>(
-      1, std::min<size_t>({(size_t)P, 8, ((size_t)256 << 20) / std::max<size_t>(8 * doubles, 1)}));
+// W slots for `doubles` values of W per t-point: up to 8 t-points in 256 MB and
+// in `room` bytes.
+int near_group(int P, size_t doubles, size_t room) {
+  return (int)std::max<size_t>(1, std::min<size_t>({(size_t)P, 8, std::min((size_t)256 << 20, room) /
+                                                                      std::max<size_t>(8 * doubles, 1)}));
 }
 
 // W for `G` slots; one where the memory does not hold the group.
@@ -1552,8 +1554,11 @@ void weights_for(const dage_gbfmm *g, double energy, std::vector<double> &w) {
 
 void set_weights(dage_gbfmm *g) { weights_for(g, g->energy, g->w); }
 
+// `single`: an operator of its own, with the expansions and intermediates of
+// one density; without it the geometry, matrices and tables only (a batch's
+// plan: the batch holds the rest).
 int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, int lmax,
-                      const dage_quad *quad) {
+                      const dage_quad *quad, bool single) {
   DAGE_TRY(sh_tables_init());
   DAGE_TRY(sh_prepare());
   if (!grid || !quad) return fail(DAGE_E_INVALID, "null argument");
@@ -1814,9 +1819,11 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
   }
   DAGE_TRY(build_m2l(g));
   DAGE_TRY(build_shapes(g));
-  DAGE_TRY(g->d_q.alloc(sizeof(double) * g->nbtot * g->N));
-  DAGE_TRY(g->d_L.alloc(sizeof(double) * g->nbtot * g->N));
-  DAGE_TRY(g->d_partial.alloc(sizeof(double) * (size_t)g->nbox * g->nslab * g->N));
+  if (single) {
+    DAGE_TRY(g->d_q.alloc(sizeof(double) * g->nbtot * g->N));
+    DAGE_TRY(g->d_L.alloc(sizeof(double) * g->nbtot * g->N));
+    DAGE_TRY(g->d_partial.alloc(sizeof(double) * (size_t)g->nbox * g->nslab * g->N));
+  }
 
   // --- near-field sub-operator matrices per axis position --------------------
   TmpBuf d_tp;
@@ -1855,20 +1862,22 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
   }
   g->U_per_box = maxU;
   g->W_per_box = maxW;
-  if (g->precision == DAGE_FP64) {  // the FP64 near field's intermediates
+  if (single && g->precision == DAGE_FP64) {  // the FP64 near field's intermediates
     DAGE_TRY(g->d_U.alloc(sizeof(double) * maxU * g->nbox));
-    g->near_g = near_group(g->P, maxW * g->nbox);
+    g->near_g = near_group(g->P, maxW * g->nbox, SIZE_MAX);
     DAGE_TRY(alloc_near_w(g->d_W, maxW * g->nbox, g->near_g));
   }
   for (int d = 0; d < 3; ++d) {
     DAGE_TRY(g->wts[d].alloc(sizeof(double) * g->npts[d]));
     DAGE_CUDA_TRY(cudaMemcpyAsync(g->wts[d].ptr, g->ax[d].weights.data(),
                                   sizeof(double) * g->npts[d], cudaMemcpyHostToDevice, s));
-    DAGE_TRY(g->d_desc[d].alloc(sizeof(StageDesc) * g->nbox));
+    if (single) DAGE_TRY(g->d_desc[d].alloc(sizeof(StageDesc) * g->nbox));
   }
-  DAGE_TRY(g->d_epart.alloc(sizeof(double) * kEnergyBlocks));
-  DAGE_TRY(g->d_energy.alloc(sizeof(double)));
-  DAGE_TRY(g->d_inst.alloc(sizeof(GInst)));
+  if (single) {
+    DAGE_TRY(g->d_epart.alloc(sizeof(double) * kEnergyBlocks));
+    DAGE_TRY(g->d_energy.alloc(sizeof(double)));
+    DAGE_TRY(g->d_inst.alloc(sizeof(GInst)));
+  }
   DAGE_CUDA_TRY(cudaStreamSynchronize(s));
   return 0;
 }
@@ -2444,7 +2453,7 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
     if (found < 0) {
       auto *g = new dage_gbfmm();
       g->precision = precision;
-      int rc = gbfmm_create_impl(g, gi, maxlevel, lmax, quad);
+      int rc = gbfmm_create_impl(g, gi, maxlevel, lmax, quad, false);
       if (!rc && precision != DAGE_FP64) rc = near16_init(g, false);
       if (rc) {
         gbfmm_destroy_impl(g);
@@ -2543,7 +2552,9 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
   b->chunks.push_back(std::move(cur));
   DAGE_TRY(b->U.alloc(sizeof(double) * std::max<size_t>(umax, 1)));
   b->wslot = wmax;
-  b->near_g = near_group(b->P, wmax);
+  // the group's further W slots stay within the budget as well
+  const size_t taken = sizeof(double) * umax;
+  b->near_g = near_group(b->P, wmax, budget > taken ? budget - taken : 0);
   DAGE_TRY(alloc_near_w(b->W, wmax, b->near_g));
   for (auto &c : b->chunks) {
     c.njobs = (c.i1 - c.i0) * b->nbox;
@@ -2649,7 +2660,7 @@ int dage_gbfmm_create(const dage_grid1d grid[3], int maxlevel, int lmax, const d
                 "the GBFMM operator runs in DAGE_FP64 or DAGE_MIXED_FP16X3 (near field)");
   auto *g = new dage_gbfmm();
   g->precision = precision;
-  int rc = gbfmm_create_impl(g, grid, maxlevel, lmax, quad);
+  int rc = gbfmm_create_impl(g, grid, maxlevel, lmax, quad, true);
   if (!rc) rc = precision == DAGE_FP64 ? gbfmm_autotune(g) : near16_init(g, true);
   if (rc) {
     gbfmm_destroy_impl(g);
@@ -2670,7 +2681,7 @@ int dage_gbfmm_create_adaptive(const dage_grid1d grid[3], int maxlevel, int lmax
   auto *g = new dage_gbfmm();
   g->precision = precision;
   g->lev0 = 1;
-  int rc = gbfmm_create_impl(g, grid, maxlevel, lmax, quad);
+  int rc = gbfmm_create_impl(g, grid, maxlevel, lmax, quad, true);
   if (!rc) rc = precision == DAGE_FP64 ? gbfmm_autotune(g) : near16_init(g, true);
   if (rc) {
     gbfmm_destroy_impl(g);

@@ -78,3 +78,39 @@ def test_fp64_first_apply_after_tuning_allocates_nothing(dage):
     V1 = _apply(op, rho, V)
     assert _free() == free
     np.testing.assert_array_equal(_apply(op, rho, V), V1)
+
+
+def _near_bytes(cells):
+    """(U, one slot of W) in bytes of the FP64 near field of one density on
+    4 x 4 x 4 boxes: near and own points of the widest box of each axis."""
+    def axis(n):
+        nc = [n // 4 + (v < n % 4) for v in range(4)]
+        near = [sum(nc[max(v - 1, 0):v + 2]) * 6 + 1 for v in range(4)]
+        own = [6 * c + (v == 3) for v, c in enumerate(nc)]
+        return list(zip(near, own))
+    boxes = [(x, y, z) for x in axis(cells[0]) for y in axis(cells[1]) for z in axis(cells[2])]
+    u = max(y[0] * z[0] * x[1] for x, y, z in boxes)
+    w = max(z[0] * x[1] * y[1] for x, y, z in boxes)
+    return 8 * 64 * u, 8 * 64 * w
+
+
+@pytest.mark.parametrize("slots", [1, 3])
+def test_batch_intermediates_stay_in_the_budget(dage, slots):
+    """One density of 121^3 (W of 45 MB, up to five slots without a budget)
+    under a budget of U and `slots` slots of W: the batch takes that and no more
+    (beside the matrices: 3 axes, 4 positions, P t-points, and a few MB of
+    tables), and its plan keeps no intermediates of its own."""
+    cells, P = (20, 20, 20), 8
+    u, w = _near_bytes(cells)
+    g = dage.Grid3D.cube(-12.0, 20, 0.2)
+    quad = dage.GaussQuad(4, 4)
+    rho, V, V1 = _density(g.shape), _density(g.shape), _density(g.shape)
+    single = dage.GBFMMCoulomb3D(g, lmax=2, quad=quad)
+    single.apply(rho, V1)
+    del single
+    matrices = 8 * 3 * 4 * P * 31 * 91
+    free = _free()
+    batch = dage.GBFMMBatch([g], lmax=2, quad=quad, near_budget_bytes=u + slots * w)
+    batch.apply([rho], [V])
+    assert free - _free() <= u + slots * w + matrices + 24 * MIB
+    assert float((V - V1).abs().max()) <= 1e-13 * float(V1.abs().max())
