@@ -2237,7 +2237,7 @@ int near16_tune(dage_gbfmm *g, int *tile) {
   int rc = 0;
   for (int tn : {64, 128}) {
     NearF16Set *set = nullptr;
-    rc = near_f16_set_create(&set, g->near16, boxes, 1, tn, s);
+    rc = near_f16_set_create(&set, g->near16, boxes, 1, tn, true, s);
     const double *rr[1] = {rho.as<double>()};
     double *vv[1] = {V.as<double>()};
     const double *ww[1] = {g->d_wn.as<double>()};
@@ -2275,7 +2275,8 @@ int near16_init(dage_gbfmm *g, bool single) {
   int tile = 64;
   DAGE_TRY(near16_tune(g, &tile));
   for (int d = 0; d < 3; ++d) g->tile_n[d] = tile;
-  if (single) DAGE_TRY(near_f16_set_create(&g->near16set, g->near16, near_boxes(g), 1, tile, g->stream));
+  if (single)
+    DAGE_TRY(near_f16_set_create(&g->near16set, g->near16, near_boxes(g), 1, tile, true, g->stream));
   return 0;
 }
 
@@ -2494,7 +2495,8 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
       for (int i = 0; i < n; ++i) {
         if (b->plan_of[i] != (int)k) continue;
         if (!cur.dens.empty() &&
-            near_f16_set_bytes(b->plans[k]->near16, boxes, (int)cur.dens.size() + 1) > budget) {
+            near_f16_set_bytes(b->plans[k]->near16, boxes, (int)cur.dens.size() + 1,
+                               b->plans[k]->tile_n[0]) > budget) {
           b->msets.push_back(cur);
           cur.dens.clear();
         }
@@ -2502,24 +2504,35 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
       }
       if (!cur.dens.empty()) b->msets.push_back(cur);
     }
-    // one workspace for all sets (they run one after another on the stream)
-    size_t wsb[3] = {0, 0, 0};
-    for (auto &m : b->msets) {
-      const dage_gbfmm *g = b->plans[m.plan];
-      size_t sb[3];
-      near_f16_set_sizes(g->near16, near_boxes(g), (int)m.dens.size(), sb);
-      for (int k = 0; k < 3; ++k) wsb[k] = std::max(wsb[k], sb[k]);
+    // one workspace for all sets (they run one after another on the stream);
+    // where it does not fit the free memory with two slots of U, one
+    bool pair = true;
+    for (;;) {
+      size_t wsb[3] = {0, 0, 0};
+      for (auto &m : b->msets) {
+        const dage_gbfmm *g = b->plans[m.plan];
+        size_t sb[3];
+        near_f16_set_sizes(g->near16, near_boxes(g), (int)m.dens.size(), g->tile_n[0], pair, sb);
+        for (int k = 0; k < 3; ++k) wsb[k] = std::max(wsb[k], sb[k]);
+      }
+      int rc = 0;
+      for (int k = 0; k < 3 && !rc; ++k) rc = b->ws16[k].alloc(wsb[k]);
+      if (!rc) break;
+      if (!pair) return rc;
+      cudaGetLastError();
+      clear_error();
+      for (DevBuf &w : b->ws16) w.release();
+      pair = false;
     }
     void *ws[3];
     for (int k = 0; k < 3; ++k) {
-      DAGE_TRY(b->ws16[k].alloc(wsb[k]));
-      DAGE_CUDA_TRY(cudaMemsetAsync(b->ws16[k].ptr, 0, wsb[k], b->stream));
+      DAGE_CUDA_TRY(cudaMemsetAsync(b->ws16[k].ptr, 0, b->ws16[k].bytes, b->stream));
       ws[k] = b->ws16[k].ptr;
     }
     for (auto &m : b->msets) {
       const dage_gbfmm *g = b->plans[m.plan];
       DAGE_TRY(near_f16_set_create(&m.set, g->near16, near_boxes(g), (int)m.dens.size(),
-                                   g->tile_n[0], b->stream, ws));
+                                   g->tile_n[0], pair, b->stream, ws));
     }
     for (int d = 0; d < 3; ++d) b->tile_n[d] = b->plans[0]->tile_n[d];
     b->tuned = true;

@@ -61,7 +61,6 @@ constexpr int BKN = 64;            // K extent of one shared-memory stage (128-b
 constexpr int kNThreads = 576;     // 18 warps
 constexpr int kNEpiThreads = 512;  // warps 2-17
 constexpr int kNMaxGroup = 4;      // t-points summed per pass of the last stage (W slots)
-constexpr int kUSlots = 2;         // t-points of a stage-x launch (U slots)
 constexpr int kRowsA = 32, kRowsB = 4;  // tile rows: 32 along a x 4 along b
 static_assert(kRowsA * kRowsB == BM, "tile rows");
 
@@ -704,6 +703,7 @@ struct NearF16Set {
   CUtensorMap mapA[3][2], mapB[3][2];
   // stage x of two t-points per tile: 0 none, else the columns of each half
   int xhalf = 0;
+  int us = 1;                   // slots of U: two where stage x takes two t-points
   CUtensorMap mapBx[2];         // its matrix tiles of xhalf rows
   DevBuf err;
 };
@@ -811,9 +811,20 @@ namespace {
 struct SetDims {
   long long ld[3], xs_rows, xsl, ysl;
   int zpad, xpad, G;
+  int xhalf, us;  // see NearF16Set
 };
 
-SetDims set_dims(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n) {
+// Two t-points per stage-x tile, the columns of each half (0: one t-point):
+// with at most 32 own points they share a 64-column tile (61^3 1.63 -> 1.36 ms
+// an apply, 121^3 3.42 -> 2.94), up to 49 a 128-column one (181^3, 46 points,
+// 9.95 -> 9.19); with 60 the wider tile's drains cost more than the shared
+// input saves (241^3 16.1 -> 18.3; between 49 and 60 not measured).
+int pair_half(const NearF16Plan *pl, int tile_n) {
+  return tile_n != 64 ? 0 : pl->maxown[0] <= 32 ? 32 : pl->maxown[0] <= 49 ? 64 : 0;
+}
+
+SetDims set_dims(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n, int tile_n,
+                 bool pair) {
   SetDims d{};
   const NearGeom &g = pl->g;
   d.ld[0] = round_up(g.npts[0], 8);
@@ -830,27 +841,31 @@ SetDims set_dims(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n
   d.xsl *= n;
   d.ysl *= n;
   d.G = std::min(g.P, kNMaxGroup);
+  d.xhalf = pair ? pair_half(pl, tile_n) : 0;
+  if (2 * d.xsl >= (1LL << 31) / d.zpad) d.xhalf = 0;  // 32-bit tensor coordinates
+  d.us = d.xhalf ? 2 : 1;
   return d;
 }
 
 }  // namespace
 
 void near_f16_set_sizes(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n,
-                        size_t bytes[3]) {
-  const SetDims d = set_dims(pl, boxes, n);
+                        int tile_n, bool pair, size_t bytes[3]) {
+  const SetDims d = set_dims(pl, boxes, n, tile_n, pair);
   bytes[0] = sizeof(__half) * 2 * ((size_t)n * d.xs_rows * d.ld[0]);
-  bytes[1] = sizeof(__half) * 2 * ((size_t)kUSlots * d.xsl * d.zpad * d.ld[1]);
+  bytes[1] = sizeof(__half) * 2 * ((size_t)d.us * d.xsl * d.zpad * d.ld[1]);
   bytes[2] = sizeof(__half) * 2 * ((size_t)d.G * d.ysl * d.xpad * d.ld[2]);
 }
 
-size_t near_f16_set_bytes(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n) {
+size_t near_f16_set_bytes(const NearF16Plan *pl, const std::vector<NearBox> &boxes, int n,
+                          int tile_n) {
   size_t b[3];
-  near_f16_set_sizes(pl, boxes, n, b);
+  near_f16_set_sizes(pl, boxes, n, tile_n, true, b);
   return b[0] + b[1] + b[2];
 }
 
 int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vector<NearBox> &boxes,
-                        int n, int tile_n, cudaStream_t s0, void *const ws[3]) {
+                        int n, int tile_n, bool pair, cudaStream_t s0, void *const ws[3]) {
   if (tile_n != 64 && tile_n != 128) return fail(DAGE_E_INVALID, "near-field tile width %d", tile_n);
   auto *st = new NearF16Set();
   *out = st;
@@ -860,7 +875,22 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   st->boxes = boxes;
   const NearGeom &g = pl->g;
   st->P = g.P;
-  const SetDims d = set_dims(pl, boxes, n);
+  SetDims d = set_dims(pl, boxes, n, tile_n, pair);
+  if (!ws) {
+    size_t bytes[3];
+    near_f16_set_sizes(pl, boxes, n, tile_n, pair, bytes);
+    DAGE_TRY(st->X.alloc(bytes[0]));
+    DAGE_TRY(st->W.alloc(bytes[2]));
+    if (d.us == 2 && st->U.alloc(bytes[1])) {  // no room for two slots
+      cudaGetLastError();
+      clear_error();
+      d = set_dims(pl, boxes, n, tile_n, false);
+      near_f16_set_sizes(pl, boxes, n, tile_n, false, bytes);
+    }
+    DAGE_TRY(st->U.alloc(bytes[1]));
+  }
+  st->xhalf = d.xhalf;
+  st->us = d.us;
   for (int s = 0; s < 3; ++s) st->ld[s] = d.ld[s];
   st->zpad = d.zpad;
   st->xpad = d.xpad;
@@ -868,20 +898,17 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   st->ysl = d.ysl;
   st->xs_rows = d.xs_rows;
   st->G = d.G;
-  if (kUSlots * d.xsl >= (1LL << 31) / d.zpad || (long long)d.G * d.ysl >= (1LL << 31) / d.xpad ||
+  if (d.us * d.xsl >= (1LL << 31) / d.zpad || (long long)d.G * d.ysl >= (1LL << 31) / d.xpad ||
       (long long)n * g.npts[2] >= (1LL << 31))
     return fail(DAGE_E_INVALID, "near-field set too large for 32-bit tensor coordinates");
   const size_t xe = (size_t)n * d.xs_rows * d.ld[0];
-  const size_t ue = (size_t)kUSlots * d.xsl * d.zpad * d.ld[1];
+  const size_t ue = (size_t)d.us * d.xsl * d.zpad * d.ld[1];
   const size_t we = (size_t)d.G * d.ysl * d.xpad * d.ld[2];
   if (ws) {  // shared workspace (sets that run one after another)
     st->xp = static_cast<__half *>(ws[0]);
     st->up = static_cast<__half *>(ws[1]);
     st->wp = static_cast<__half *>(ws[2]);
   } else {
-    DAGE_TRY(st->X.alloc(sizeof(__half) * 2 * xe));
-    DAGE_TRY(st->U.alloc(sizeof(__half) * 2 * ue));
-    DAGE_TRY(st->W.alloc(sizeof(__half) * 2 * we));
     // Elements the stages never write (tile edges, padding) are read only
     // against zero matrix columns or into rows that are not stored: they
     // must be finite, so the buffers start as zeros (every later write is
@@ -906,7 +933,7 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
   for (int part = 0; part < 2; ++part) {
     DAGE_TRY(make_map_3d(&st->mapA[0][part], x0 + part * xe, g.npts[0], g.npts[1],
                          (long long)n * g.npts[2], d.ld[0], g.npts[1]));
-    DAGE_TRY(make_map_3d(&st->mapA[1][part], u0 + part * ue, d.ld[1], d.zpad, kUSlots * d.xsl, d.ld[1],
+    DAGE_TRY(make_map_3d(&st->mapA[1][part], u0 + part * ue, d.ld[1], d.zpad, d.us * d.xsl, d.ld[1],
                          d.zpad));
     DAGE_TRY(make_map_3d(&st->mapA[2][part], w0 + part * we, d.ld[2], d.xpad,
                          (long long)d.G * d.ysl, d.ld[2], d.xpad));
@@ -916,11 +943,6 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
                            pl->rows[s], pl->ldb[s], tile_n));
     }
   }
-  // Two t-points per stage-x tile: with at most 32 own points they share a
-  // 64-column tile (61^3 1.63 -> 1.36 ms an apply, 121^3 3.42 -> 2.94), up to 49
-  // a 128-column one (181^3 9.95 -> 9.19); above that the wider tile's drains
-  // cost more than the shared input saves (241^3 16.1 -> 18.3).
-  st->xhalf = tile_n != 64 ? 0 : pl->maxown[0] <= 32 ? 32 : pl->maxown[0] <= 49 ? 64 : 0;
   if (st->xhalf)
     for (int part = 0; part < 2; ++part) {
       const size_t pe = (size_t)pl->rows[0] * pl->ldb[0];
@@ -1032,7 +1054,7 @@ int near_f16_set_run(NearF16Set *st, cudaStream_t s) {
       st->xp, st->xp + xe);
   DAGE_CUDA_TRY(cudaGetLastError());
 
-  const long long uslot = st->xsl * st->zpad * st->ld[1], ue = kUSlots * uslot;
+  const long long uslot = st->xsl * st->zpad * st->ld[1], ue = st->us * uslot;
   const long long we = (long long)st->G * st->ysl * st->xpad * st->ld[2];
   NearArgs base{};
   base.err = st->err.as<int>();

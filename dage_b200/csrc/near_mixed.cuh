@@ -38,15 +38,19 @@ int near_f16_plan_create(NearF16Plan **out, const NearGeom &geom, cudaStream_t s
 void near_f16_plan_destroy(NearF16Plan *p);
 
 // n densities of one plan; tile width 64 or 128 output columns.  ws: null
-// (the set allocates its intermediates) or three zero-initialised device
-// buffers of at least near_f16_set_sizes bytes (split input, U, W) that
-// sets running one after another on one stream may share.
+// (the set allocates its intermediates; where two slots of U do not fit the
+// free memory, one, and stage x takes one t-point per tile) or three
+// zero-initialised device buffers of at least near_f16_set_sizes bytes (split
+// input, U, W) that sets running one after another on one stream may share.
+// pair: stage x may take two t-points per tile (two slots of U) where that is
+// the faster form; without it one, with the same results.
 int near_f16_set_create(NearF16Set **out, const NearF16Plan *plan, const std::vector<NearBox> &boxes,
-                        int n, int tile_n, cudaStream_t s, void *const ws[3] = nullptr);
+                        int n, int tile_n, bool pair, cudaStream_t s, void *const ws[3] = nullptr);
 void near_f16_set_destroy(NearF16Set *s);
 void near_f16_set_sizes(const NearF16Plan *plan, const std::vector<NearBox> &boxes, int n,
-                        size_t bytes[3]);
-size_t near_f16_set_bytes(const NearF16Plan *plan, const std::vector<NearBox> &boxes, int n);
+                        int tile_n, bool pair, size_t bytes[3]);
+size_t near_f16_set_bytes(const NearF16Plan *plan, const std::vector<NearBox> &boxes, int n,
+                          int tile_n);
 
 // Binds device cubes and per-density t-point weights (device arrays of P
 // doubles): uploads their addresses (synchronises the stream).

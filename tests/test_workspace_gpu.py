@@ -114,3 +114,72 @@ def test_batch_intermediates_stay_in_the_budget(dage, slots):
     batch.apply([rho], [V])
     assert free - _free() <= u + slots * w + matrices + 24 * MIB
     assert float((V - V1).abs().max()) <= 1e-13 * float(V1.abs().max())
+
+
+def _u16_slot(ncell, nbox_axis=4):
+    """Bytes of one U slot of the fp16x3 near field (two FP16 planes of
+    [x own of every box][z near, padded to 32][y near, padded to 8])."""
+    nc = [ncell // nbox_axis + (v < ncell % nbox_axis) for v in range(nbox_axis)]
+    near = max(sum(nc[max(v - 1, 0):v + 2]) for v in range(nbox_axis)) * 6 + 1
+    return 4 * (ncell * 6 + 1) * nbox_axis**2 * (-(-near // 32) * 32) * (-(-near // 8) * 8)
+
+
+def _near16_bytes(ncell, P):
+    """The set's other intermediates (split input, W) and the plan's matrices."""
+    n = ncell * 6 + 1
+    nc = [ncell // 4 + (v < ncell % 4) for v in range(4)]
+    own = max(6 * c + (v == 3) for v, c in enumerate(nc))
+    near = max(sum(nc[max(v - 1, 0):v + 2]) for v in range(4)) * 6 + 1
+    x = 4 * n * n * (-(-n // 8) * 8)
+    w = 4 * min(P, 4) * n * 16 * (-(-own // 32) * 32) * (-(-near // 8) * 8)
+    return x + w + 3 * (8 + 4 + 2) * P * n * (near + 8)
+
+
+def test_near_field_takes_one_u_slot_where_t_points_do_not_share_tiles(dage):
+    """217^3 owns 54 or 55 points a box: one t-point per stage-x tile, one slot
+    of U (a second one would be 448 MB)."""
+    ncell, quad = 36, dage.GaussQuad(2, 2)
+    g = dage.Grid3D.cube(-21.6, ncell, 0.2)
+    rho, V = _density(g.shape), _density(g.shape)
+    dage.GBFMMCoulomb3D(g, lmax=2, quad=quad, precision="fp16x3").apply(rho, V)  # tunes
+    free = _free()
+    op = dage.GBFMMCoulomb3D(g, lmax=2, quad=quad, precision="fp16x3")
+    op.apply(rho, V)
+    used = free - _free()
+    slot = _u16_slot(ncell)
+    assert slot > 400 * MIB
+    assert used <= slot + _near16_bytes(ncell, 4) + 64 * MIB
+
+
+def test_near_field_with_room_for_one_u_slot(dage, monkeypatch):
+    """181^3 owns 45 or 46 points a box: two t-points share a stage-x tile
+    where there is room for two slots of U; where there is not, one is taken,
+    with the same bits.  Single operator and batch."""
+    monkeypatch.setenv("DAGE_NEAR16_TILE", "64")
+    ncell, quad = 30, dage.GaussQuad(3, 2)
+    g = dage.Grid3D.cube(-18.0, ncell, 0.2)
+    rho, V = _density(g.shape), _density(g.shape)
+    slot = _u16_slot(ncell)
+
+    def single():
+        op = dage.GBFMMCoulomb3D(g, lmax=2, quad=quad, precision="fp16x3")
+        op.apply(rho, V)
+        return op
+
+    def batch():
+        b = dage.GBFMMBatch([g], lmax=2, quad=quad, precision="fp16x3")
+        b.apply([rho], [V])
+        return b
+
+    for make in (single, batch):
+        make()  # kernels loaded
+        free = _free()
+        keep = make()
+        need = free - _free()
+        want = V.cpu().numpy()
+        del keep
+        V.zero_()
+        with _Leave(need - slot // 2):
+            keep = make()
+            del keep
+        np.testing.assert_array_equal(V.cpu().numpy(), want)
