@@ -34,6 +34,15 @@ int sm_count() {
   return count;
 }
 
+bool room_to_spare(size_t bytes) {
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= free / 4;
+}
+
 int DevBuf::alloc(size_t n) {
   if (n <= bytes && ptr) return 0;
   release();

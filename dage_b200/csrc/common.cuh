@@ -39,6 +39,11 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // Number of SMs of the current device (cached per process).
 int sm_count();
 
+// True where `bytes` that only make a call faster (further slots of an
+// intermediate) are at most a quarter of the device's free memory: what the
+// same operator or its caller needs afterwards must not fail for them.
+bool room_to_spare(size_t bytes);
+
 // RAII-free device buffer owned by an operator handle.
 struct DevBuf {
   void *ptr = nullptr;

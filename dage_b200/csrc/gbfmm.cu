@@ -1434,9 +1434,10 @@ int near_group(int P, size_t doubles, size_t room) {
                                                                       std::max<size_t>(8 * doubles, 1)}));
 }
 
-// W for `G` slots; one where the memory does not hold the group.
+// W for `G` slots; one where the group takes too much of the free memory.
 int alloc_near_w(DevBuf &W, size_t doubles, int &G) {
-  if (G > 1 && W.alloc(sizeof(double) * doubles * G)) {
+  if (G > 1 && (!room_to_spare(sizeof(double) * doubles * (G - 1)) ||
+                W.alloc(sizeof(double) * doubles * G))) {
     cudaGetLastError();
     clear_error();
     G = 1;
@@ -2505,7 +2506,7 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
       if (!cur.dens.empty()) b->msets.push_back(cur);
     }
     // one workspace for all sets (they run one after another on the stream);
-    // where it does not fit the free memory with two slots of U, one
+    // where two slots of U take too much of the free memory, with one
     bool pair = true;
     for (;;) {
       size_t wsb[3] = {0, 0, 0};
@@ -2515,7 +2516,7 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
         near_f16_set_sizes(g->near16, near_boxes(g), (int)m.dens.size(), g->tile_n[0], pair, sb);
         for (int k = 0; k < 3; ++k) wsb[k] = std::max(wsb[k], sb[k]);
       }
-      int rc = 0;
+      int rc = pair && !room_to_spare(wsb[1] / 2) ? DAGE_E_NOMEM : 0;
       for (int k = 0; k < 3 && !rc; ++k) rc = b->ws16[k].alloc(wsb[k]);
       if (!rc) break;
       if (!pair) return rc;

@@ -38,8 +38,8 @@ int near_f16_plan_create(NearF16Plan **out, const NearGeom &geom, cudaStream_t s
 void near_f16_plan_destroy(NearF16Plan *p);
 
 // n densities of one plan; tile width 64 or 128 output columns.  ws: null
-// (the set allocates its intermediates; where two slots of U do not fit the
-// free memory, one, and stage x takes one t-point per tile) or three
+// (the set allocates its intermediates; where two slots of U take too much of
+// the free memory, one, and stage x takes one t-point per tile) or three
 // zero-initialised device buffers of at least near_f16_set_sizes bytes (split
 // input, U, W) that sets running one after another on one stream may share.
 // pair: stage x may take two t-points per tile (two slots of U) where that is

@@ -879,15 +879,17 @@ static int fp64_group(const dage_op3d *op) {
 }
 
 // The intermediates of a group of t-points in one allocation: U, then W.
-// Where a group does not fit the free memory it becomes a single t-point.  The
-// group is chosen once and kept with its memory: it sets the order of the sums
+// Where a group takes too much of the free memory it becomes a single t-point.
+// The group is chosen once and kept with its memory: it sets the order of the sums
 // over the t-points, so applies of one operator agree to the last bit, and a
 // later apply frees and allocates nothing.  The tuner takes it at creation;
 // otherwise (its choice known already) the first apply does (~0.4 ms).
 static int fp64_workspace(dage_op3d *op) {
   if (op->tmp_group) return 0;
   const size_t niy = op->nin[1], niz = op->nin[2], nox = op->nout[0], noy = op->nout[1];
-  for (int G = fp64_group(op);; G = 1) {
+  int G = fp64_group(op);
+  if (G > 1 && !room_to_spare(sizeof(double) * (G - 1) * niz * nox * (niy + noy))) G = 1;
+  for (;; G = 1) {
     const size_t nu = G * niy * niz * nox;
     const int rc = op->tmp.alloc(sizeof(double) * (nu + G * niz * nox * noy));
     if (rc && G == 1) return rc;

@@ -1163,12 +1163,14 @@ int mixed_setup(dage_op3d *op) {
     st->nkb[s] = ceil_div(op->nin[s], BK);
     st->natA[s] = ceil_div(rows[s], kAtomRows);
     st->xbytes[s] = (size_t)outer[s] * st->nkb[s] * st->natA[s] * (st->nparts * kAtomRows * BK * 2);
-    // padding rows and K columns are never written: they stay zero
-    if (s == 1 && st->Gi > 1 && st->X[1].alloc(st->xbytes[1] * st->Gi)) {
-      cudaGetLastError();  // a group that does not fit the free memory becomes one t-point
+    // a group that takes too much of the free memory becomes one t-point
+    if (s == 1 && st->Gi > 1 &&
+        (!room_to_spare(st->xbytes[1] * (st->Gi - 1)) || st->X[1].alloc(st->xbytes[1] * st->Gi))) {
+      cudaGetLastError();
       clear_error();
       st->Gi = 1;
     }
+    // padding rows and K columns are never written: they stay zero
     DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : s == 1 ? st->Gi : 1)));
     DAGE_CUDA_TRY(cudaMemsetAsync(st->X[s].ptr, 0, st->X[s].bytes, op->stream));
   }

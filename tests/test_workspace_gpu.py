@@ -183,3 +183,48 @@ def test_near_field_with_room_for_one_u_slot(dage, monkeypatch):
             keep = make()
             del keep
         np.testing.assert_array_equal(V.cpu().numpy(), want)
+
+
+def test_split_precision_group_leaves_the_rest_its_room(dage):
+    """121^3, fp16x3: six slots of the first intermediate take 35 MB more than
+    one; an operator with 20 MB less than that form needs takes one slot, with
+    the same bits."""
+    g = dage.Grid3D.cube(-12.0, 20, 0.2)
+    quad = dage.GaussQuad(7, 6)
+    rho, V = _density(g.shape), _density(g.shape)
+
+    def make():
+        op = dage.Coulomb3D(g, quad=quad, precision="fp16x3")
+        op.apply(rho, V)
+        return op
+
+    make()  # tunes
+    free = _free()
+    keep = make()
+    need = free - _free()
+    want = V.cpu().numpy()
+    del keep
+    V.zero_()
+    with _Leave(need - 20 * MIB):
+        keep = make()
+        del keep
+    np.testing.assert_array_equal(V.cpu().numpy(), want)
+
+
+def test_fp64_near_field_group_leaves_host_cubes_their_room(dage):
+    """GBFMM 121^3: five W slots (180 MB more than one) must not take the
+    memory of the two 14 MB cubes that a host-array apply stages."""
+    g = dage.Grid3D.cube(-12.0, 20, 0.2)
+    quad = dage.GaussQuad(4, 4)
+    rho, V = _density(g.shape), _density(g.shape)
+    host = np.asfortranarray(rho.cpu().numpy().transpose(2, 1, 0))
+    make = lambda: dage.GBFMMCoulomb3D(g, lmax=2, quad=quad)  # noqa: E731
+    make().apply(rho, V)  # tunes
+    free = _free()
+    keep = make()
+    need = free - _free()
+    want = keep.apply(host)
+    del keep
+    with _Leave(need + 10 * MIB):
+        got = make().apply(host)
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
