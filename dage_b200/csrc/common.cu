@@ -49,6 +49,7 @@ int DevBuf::alloc(size_t n) {
   if (n == 0) return 0;
   cudaError_t e = cudaMalloc(&ptr, n);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // or the next launch's check would report it
     ptr = nullptr;
     return fail(DAGE_E_NOMEM, "cudaMalloc(%zu bytes) failed: %s", n, cudaGetErrorString(e));
   }

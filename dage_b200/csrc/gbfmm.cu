@@ -1438,7 +1438,6 @@ int near_group(int P, size_t doubles, size_t room) {
 int alloc_near_w(DevBuf &W, size_t doubles, int &G) {
   if (G > 1 && (!room_to_spare(sizeof(double) * doubles * (G - 1)) ||
                 W.alloc(sizeof(double) * doubles * G))) {
-    cudaGetLastError();
     clear_error();
     G = 1;
   }
@@ -2520,7 +2519,6 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
       for (int k = 0; k < 3 && !rc; ++k) rc = b->ws16[k].alloc(wsb[k]);
       if (!rc) break;
       if (!pair) return rc;
-      cudaGetLastError();
       clear_error();
       for (DevBuf &w : b->ws16) w.release();
       pair = false;

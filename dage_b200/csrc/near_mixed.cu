@@ -882,7 +882,6 @@ int near_f16_set_create(NearF16Set **out, const NearF16Plan *pl, const std::vect
     DAGE_TRY(st->X.alloc(bytes[0]));
     DAGE_TRY(st->W.alloc(bytes[2]));
     if (d.us == 2 && (!room_to_spare(bytes[1] / 2) || st->U.alloc(bytes[1]))) {  // no room for two
-      cudaGetLastError();
       clear_error();
       d = set_dims(pl, boxes, n, tile_n, false);
       near_f16_set_sizes(pl, boxes, n, tile_n, false, bytes);

@@ -898,7 +898,6 @@ static int fp64_workspace(dage_op3d *op) {
       op->tmp_w = nu;
       return 0;
     }
-    cudaGetLastError();
     clear_error();
   }
 }

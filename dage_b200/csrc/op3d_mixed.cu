@@ -1166,7 +1166,6 @@ int mixed_setup(dage_op3d *op) {
     // a group that takes too much of the free memory becomes one t-point
     if (s == 1 && st->Gi > 1 &&
         (!room_to_spare(st->xbytes[1] * (st->Gi - 1)) || st->X[1].alloc(st->xbytes[1] * st->Gi))) {
-      cudaGetLastError();
       clear_error();
       st->Gi = 1;
     }

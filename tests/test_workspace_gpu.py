@@ -228,3 +228,20 @@ def test_fp64_near_field_group_leaves_host_cubes_their_room(dage):
     with _Leave(need + 10 * MIB):
         got = make().apply(host)
     assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
+
+
+def test_refused_allocation_leaves_no_error_behind(dage):
+    """A creation refused for memory fails with DAGE_E_NOMEM; the next one, of
+    an operator that fits, is not affected."""
+    g = dage.Grid3D.cube(-7.8, 13, 0.2)
+    quad = dage.GaussQuad(3, 3)
+    rho, V = _density(g.shape), _density(g.shape)
+    dage.Coulomb3D(g, quad=quad).apply(rho, V)
+    want = V.cpu().numpy()
+    with _Leave(64 * MIB):
+        with pytest.raises(dage.DageError) as e:
+            dage.Coulomb3D(dage.Grid3D.cube(-24.0, 40, 0.2), quad=quad, precision="bf16x6")
+        assert e.value.code == -3
+        del e
+        got = _apply(dage.Coulomb3D(g, quad=quad), rho, V)
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()  # another group of t-points
