@@ -102,6 +102,7 @@ struct BoxInfo {
   int q0[3], nq[3];     // near-field region points
   int pos[3];           // box position along each axis
   double c[3];          // expansion centre
+  int route;            // forms of its moments and potential (set_routes)
 };
 
 // One density of a batch (a batch of one for dage_gbfmm_apply): its cubes,
@@ -211,6 +212,47 @@ int sh_tables_init() {
   return once.run(dev, sh_tables_upload);
 }
 
+// solid_harmonics with the coefficient tables (every lane of a warp visits
+// the same (l, m) sequence, so the constant-bank reads are uniform).
+template <class F>
+__device__ __forceinline__ void solid_harmonics_tab(int lmax, double x, double y, double z, F &&f) {
+  const double r2 = x * x + y * y + z * z;
+  f(0, 1.0);
+  if (lmax == 0) return;
+  {
+    double p2 = 0.0, p1 = 1.0;
+    for (int l = 1; l <= lmax; ++l) {
+      const double cur = c_shA[lmi(l, 0)] * (z * p1) - c_shB[lmi(l, 0)] * (r2 * p2);
+      f(lmi(l, 0), cur);
+      p2 = p1;
+      p1 = cur;
+    }
+  }
+  double top = x, bot = y;
+  for (int mm = 1; mm <= lmax; ++mm) {
+    if (mm >= 2) {
+      const double c = c_shC[mm];
+      const double nb = c * (y * top + x * bot);
+      const double nt = c * (x * top - y * bot);
+      top = nt;
+      bot = nb;
+    }
+    f(lmi(mm, mm), top);
+    f(lmi(mm, -mm), bot);
+#pragma unroll 1
+    for (int sgn = 0; sgn < 2; ++sgn) {
+      const int m = sgn ? -mm : mm;
+      double p2 = 0.0, p1 = sgn ? bot : top;
+      for (int l = mm + 1; l <= lmax; ++l) {
+        const double cur = c_shA[lmi(l, m)] * (z * p1) - c_shB[lmi(l, m)] * (r2 * p2);
+        f(lmi(l, m), cur);
+        p2 = p1;
+        p1 = cur;
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Multipole moments q_lm(b) = sum rho w S_lm (Helmholtz: i_l(kappa r) Y_lm) and
 // far-field potential V(r) += sum_lm L_lm S_lm, as matrix products.
@@ -222,9 +264,12 @@ int sh_tables_init() {
 //   q(lm, box) = sum_point S(lm, point) w(point) rho(point, box)
 //   V(point, box) += sum_lm S(lm, point) L(lm, box),
 // on the FP64 tensor pipe, with S made on the fly in shared memory, once for
-// up to 64 boxes.  One evaluation of S per box and point (the former kernels)
-// was bound by its recurrences: 241^3, lmax 12 took 2.9 ms for the moments and
-// 1.4 ms for the potential; 0.50 and 0.45 ms so.
+// up to 64 boxes.  One evaluation of S per box and point (the *_box_kernel
+// forms) is bound by its recurrences: 241^3, lmax 12 takes 2.9 ms for the
+// moments and 1.4 ms for the potential; 0.50 and 0.45 ms so.
+//
+// That pays where enough boxes share S, since making it in shared memory costs
+// several times a box's own evaluation in registers; set_routes draws the line.
 //
 // The (lmax+1)^2 harmonics of a point are split into lmax+1 lane tasks of
 // lmax+1 values each: task 0 is the m = 0 chain (l = 0..lmax); the others
@@ -237,11 +282,20 @@ constexpr int kShCols = 64;      // boxes of one block
 constexpr int kMpPoints = 32;    // points per step of the moments
 constexpr int kMpPitch = kMpPoints + 4;  // shared rows, free of bank conflicts
 
+// Bits of a box's route: 0 the moments as a product for the Coulomb kernel, 1
+// for the Helmholtz kernel, 2 and 3 the potential (set_routes).
+__host__ __device__ inline bool sh_moments_product(int route, bool helm) {
+  return (route >> (helm ? 1 : 0)) & 1;
+}
+__host__ __device__ inline bool sh_potential_product(int route, bool helm) {
+  return (route >> (helm ? 3 : 2)) & 1;
+}
+
 // Up to 64 boxes of one shape, a column tile of both products.
 struct ShTile {
   int first, count;  // in the plan's list of boxes by shape
+  int route;         // of its boxes
 };
-
 
 // chains of task t: signed m of the first and second chain (task 0: the
 // m = 0 chain alone, m2 unused) and the first chain's length
@@ -361,12 +415,169 @@ __device__ __forceinline__ int sh_nwarps(int count) {
   return count > 32 ? 8 : count > 16 ? 4 : count > 8 ? 2 : 1;
 }
 
-// Moments: grid (slab, column tile, density).  A block takes a contiguous range
+// Moments, one box at a time: grid (box, slab, density).  A warp evaluates
+// PP = 32/(lmax+1) points at a time, lane p(lmax+1)+t running task t for point
+// p, each lane keeping its lmax+1 sums in registers.  Warps walk columns of the
+// box (PP neighbouring x, one y, every z); at the end the block sums its lanes
+// in a fixed order into one partial per (box, slab); a box has `stride` of them.
+constexpr int kMpWarps = 8;
+constexpr int kMpSlabs = 16;  // slabs of a box (4 with 8 densities or more)
+
+template <bool HELM>
+__global__ void __launch_bounds__(kMpWarps * 32, HELM ? 2 : 3)
+    multipoles_box_kernel(const GInst *__restrict__ insts, int lmax, int nslab, int stride) {
+  __shared__ double sA[16 * 16], sB[16 * 16];  // [k][t]
+  __shared__ double red[kMpWarps][32][17];
+  const GInst &I = insts[blockIdx.z];
+  const int L = lmax, L1 = lmax + 1;
+  if (sh_moments_product(I.boxes[blockIdx.x].route, I.kappa > 0.0)) return;  // multipoles_kernel
+  const int PP = 32 / L1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int e = threadIdx.x; e < L1 * L1; e += blockDim.x) {
+    const int t = e / L1, k = e % L1;
+    int l, m;
+    mp_step(L, t, k, l, m);
+    const bool start = l == abs(m);
+    sA[k * 16 + t] = start ? 0.0 : c_shA[lmi(l, m)];
+    sB[k * 16 + t] = start ? 0.0 : c_shB[lmi(l, m)];
+  }
+  __syncthreads();
+  const int p = lane / L1, t = lane % L1;
+  int m1, m2, len1;
+  mp_task(L, t, m1, m2, len1);
+  const int a1 = abs(m1), a2 = abs(m2), amax = t == 0 ? 0 : max(a1, a2);
+  const bool helm = HELM && I.kappa > 0.0;  // a batch may mix kernels
+  const BoxInfo b = I.boxes[blockIdx.x];
+  const int ws = I.wstride;
+  const double *wx = I.wbox + (0 * 64 + b.pos[0]) * ws;
+  const double *wy = I.wbox + (1 * 64 + b.pos[1]) * ws;
+  const double *wz = I.wbox + (2 * 64 + b.pos[2]) * ws;
+  const double *xs = I.wbox + (3 * 64) * ws;  // point coordinates per axis
+  const size_t plane = (size_t)I.Nx * I.Ny;
+
+  double acc[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] = 0.0;
+
+  const int nib = (b.np[0] + PP - 1) / PP;
+  const int nbund = nib * b.np[1];
+  for (int u = blockIdx.y * kMpWarps + warp; u < nbund; u += nslab * kMpWarps) {
+    const int j = u / nib, i = (u % nib) * PP + p;
+    const bool valid = p < PP && i < b.np[0];
+    const int ii = valid ? i : 0;
+    const double x = xs[b.p0[0] + ii] - b.c[0];
+    const double y = xs[ws + b.p0[1] + j] - b.c[1];
+    const double wxy = valid ? wx[ii] * wy[j] : 0.0;
+    // chain starts S_{a1,+-a1}, S_{a2,+-a2} (task 0: S_00 = 1)
+    double s1 = 1.0, s2 = 0.0;
+    {
+      double top = x, bot = y;
+      for (int mm = 1; mm <= amax; ++mm) {
+        if (mm >= 2) {
+          const double c = c_shC[mm];
+          const double nb = c * (y * top + x * bot);
+          const double nt = c * (x * top - y * bot);
+          top = nt;
+          bot = nb;
+        }
+        if (mm == a1) s1 = m1 > 0 ? top : bot;
+        if (mm == a2) s2 = m2 > 0 ? top : bot;
+      }
+    }
+    const double *rcol = I.rho + (size_t)(b.p0[0] + ii) + (size_t)I.Nx * (b.p0[1] + j) +
+                         plane * b.p0[2];
+    // Helmholtz: i_l(kappa r) Y_lm(rhat) = kappa^l f_l(kappa r) S_lm(r).  The
+    // factors g_l = kappa^l f_l of the bundle's next CZ z values of each of
+    // its PP columns come first, one lane per point (series for L and L - 1,
+    // downward recursion), into this warp's rows of `red` (free until the
+    // final reduction).
+    if constexpr (!HELM) {
+      for (int kz = 0; kz < b.np[2]; ++kz) {
+        const double v = valid ? rcol[plane * kz] * (wxy * wz[kz]) : 0.0;
+        const double z = xs[2 * ws + b.p0[2] + kz] - b.c[2];
+        const double r2 = x * x + y * y + z * z;
+        double p1 = 0.0, p2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          if (k > L) break;
+          const bool st = k == 0 || k == len1;
+          const double rec = sA[k * 16 + t] * (z * p1) - sB[k * 16 + t] * (r2 * p2);
+          const double cur = st ? (k == 0 ? s1 : s2) : rec;
+          p2 = st ? 0.0 : p1;
+          p1 = cur;
+          acc[k] += v * cur;
+        }
+      }
+      continue;
+    }
+    const int CZ = 32 / PP;
+    const int pi = p < PP ? p : 0;
+    for (int kz0 = 0; kz0 < b.np[2]; kz0 += CZ) {
+      if (helm) {
+        const int ic = min((u % nib) * PP + lane / CZ, b.np[0] - 1);
+        const int kc = min(kz0 + lane % CZ, b.np[2] - 1);
+        const double xc = xs[b.p0[0] + ic] - b.c[0], zc = xs[2 * ws + b.p0[2] + kc] - b.c[2];
+        const double x2 = (I.kappa * I.kappa) * (xc * xc + y * y + zc * zc);
+        double *g = red[warp][lane];
+        g[L] = bessel_ratio_series(0.5 * x2, L);
+        if (L >= 1) g[L - 1] = bessel_ratio_series(0.5 * x2, L - 1);
+        for (int l = L - 2; l >= 0; --l) g[l] = (2 * l + 3) * g[l + 1] + x2 * g[l + 2];
+        double kp = 1.0;
+        for (int l = 0; l <= L; ++l) {
+          g[l] *= kp;
+          kp *= I.kappa;
+        }
+        __syncwarp();
+      }
+      const int kzend = min(kz0 + CZ, b.np[2]);
+      for (int kz = kz0; kz < kzend; ++kz) {
+        const double v = valid ? rcol[plane * kz] * (wxy * wz[kz]) : 0.0;
+        const double z = xs[2 * ws + b.p0[2] + kz] - b.c[2];
+        const double r2 = x * x + y * y + z * z;
+        const double *gp = red[warp][pi * CZ + (kz - kz0)];
+        double p1 = 0.0, p2 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          if (k > L) break;
+          const bool st = k == 0 || k == len1;
+          const double rec = sA[k * 16 + t] * (z * p1) - sB[k * 16 + t] * (r2 * p2);
+          const double cur = st ? (k == 0 ? s1 : s2) : rec;
+          p2 = st ? 0.0 : p1;
+          p1 = cur;
+          const double f = helm ? v * gp[k < len1 ? a1 + k : a2 + k - len1] : v;
+          acc[k] += f * cur;
+        }
+      }
+      // Required before the next chunk's factors overwrite `red` and before
+      // the final store below overwrites it with this lane's sums: every
+      // lane of the warp must be done reading the factor rows.
+      if (helm) __syncwarp();
+    }
+  }
+  // (Helmholtz: ordered after the last reads of the factor rows by the
+  // __syncwarp at the end of the chunk loop above.)
+#pragma unroll
+  for (int k = 0; k < 16; ++k)
+    if (k <= L) red[warp][lane][k] = acc[k];
+  __syncthreads();
+  const int N = L1 * L1;
+  for (int e = threadIdx.x; e < N; e += blockDim.x) {
+    const int tt = e / L1, k = e % L1;
+    int l, m;
+    mp_step(L, tt, k, l, m);
+    double sum = 0.0;
+    for (int w = 0; w < kMpWarps; ++w)
+      for (int pp = 0; pp < PP; ++pp) sum += red[w][pp * L1 + tt][k];
+    I.partial[((size_t)blockIdx.x * stride + blockIdx.y) * N + lmi(l, m)] = sum;
+  }
+}
+
+// Moments as products: grid (slab, column tile, density).  A block takes a contiguous range
 // of the shape's points, 32 a step: S w of the next step is made while this
 // step's product runs (two buffers, one barrier a step), the densities arrive
 // by asynchronous copies.  Warp w owns 8 columns and every 16/NW-th row tile.
 __global__ void __launch_bounds__(kShThreads, 1)
-    multipoles_kernel(const GInst *__restrict__ insts, int L, int nslab) {
+    multipoles_kernel(const GInst *__restrict__ insts, int L, int nslab, int stride) {
   extern __shared__ double sh[];
   __shared__ ShTables T;
   __shared__ double F[2][kMpPoints][17];
@@ -374,6 +585,7 @@ __global__ void __launch_bounds__(kShThreads, 1)
   const GInst &I = insts[blockIdx.z];
   if ((int)blockIdx.y >= I.nshtiles) return;
   const ShTile ct = I.shtiles[blockIdx.y];
+  if (!sh_moments_product(ct.route, I.kappa > 0.0)) return;  // multipoles_box_kernel
   const int L1 = L + 1, N = L1 * L1, MT = (N + 7) / 8;
   const int rows = MT * 8;
   double *S = sh;                                // [2][rows][kMpPitch]
@@ -478,20 +690,30 @@ __global__ void __launch_bounds__(kShThreads, 1)
     for (int h = 0; h < 2; ++h) {
       const int col = wn * 8 + 2 * (lane & 3) + h;
       if (col < ct.count)
-        I.partial[((size_t)I.shboxes[ct.first + col] * nslab + blockIdx.x) * N + lm] = acc[i][h];
+        I.partial[((size_t)I.shboxes[ct.first + col] * stride + blockIdx.x) * N + lm] = acc[i][h];
     }
   }
 }
 
-// q(box, lm) = sum over slabs, fixed order; grid (., density)
-__global__ void reduce_slabs_kernel(const GInst *__restrict__ insts, int nslab, int N, int nbox) {
+// q(box, lm) = sum over the slabs of the box's form, fixed order; grid (., density)
+__global__ void reduce_slabs_kernel(const GInst *__restrict__ insts, int nslab, int mslab, int stride,
+                                    int N, int nbox) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nbox * N) return;
   const GInst &I = insts[blockIdx.y];
   const int b = idx / N, s = idx % N;
+  const int n = sh_moments_product(I.boxes[b].route, I.kappa > 0.0) ? nslab : mslab;
+  const double *p = I.partial + (size_t)b * stride * N + s;
   double acc = 0.0;
-#pragma unroll 8
-  for (int k = 0; k < nslab; ++k) acc += I.partial[((size_t)b * nslab + k) * N + s];
+  int k = 0;
+  for (; k + 8 <= n; k += 8) {  // eight loads in flight, added in order
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = p[(size_t)(k + i) * N];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc += v[i];
+  }
+  for (; k < n; ++k) acc += p[(size_t)k * N];
   I.q[(size_t)(I.fine_off + b) * N + s] = acc;
 }
 
@@ -718,10 +940,149 @@ __global__ void l2l_kernel(const GInst *__restrict__ insts, int N, int poff, int
 
 // Potential: V(r) += sum_lm L_lm S_lm(r - c) over the owned points of every box
 // (Helmholtz: 8 kappa sum (2l+1)/(4 pi) i_l(kappa r) Y_lm L_lm,
-// src/gbfmm/gbfmm_helmholtz3d.F90:1019-1105); grid (chunk, column tile,
-// density).  The tile's expansions stay in shared memory, `pts` points' S at a
-// time beside them (two buffers).  L = the density's own local expansions
-// unless Lext is given (evaluation of caller-supplied expansions).
+// src/gbfmm/gbfmm_helmholtz3d.F90:1019-1105).  L = the density's own local
+// expansions unless Lext is given (evaluation of caller-supplied expansions).
+// The potential, one box at a time: every thread evaluates the harmonics of its
+// points; block (chunk, box, density).
+__global__ void l2p_box_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext,
+                               int lmax) {
+  extern __shared__ double Ls[];
+  const GInst &I = insts[blockIdx.z];
+  if (I.kappa > 0.0) return;  // Helmholtz instances: l2p_helm_box_kernel
+  if (sh_potential_product(I.boxes[blockIdx.y].route, false)) return;  // l2p_kernel
+  const int N = (lmax + 1) * (lmax + 1);
+  const BoxInfo b = I.boxes[blockIdx.y];
+  const double *L = Lext ? Lext : I.L + (size_t)I.fine_off * N;
+  for (int k = threadIdx.x; k < N; k += blockDim.x) Ls[k] = L[(size_t)blockIdx.y * N + k];
+  __syncthreads();
+  const double *xs = I.wbox + (3 * 64) * I.wstride;
+  const int ws = I.wstride;
+  const long long n = (long long)b.own[0] * b.own[1] * b.own[2];
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(e % b.own[0]);
+    const long long r = e / b.own[0];
+    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
+    const int gx = b.p0[0] + i, gy = b.p0[1] + j, gz = b.p0[2] + k;
+    double v = 0.0;
+    const double x = xs[gx] - b.c[0], y = xs[ws + gy] - b.c[1], z = xs[2 * ws + gz] - b.c[2];
+    solid_harmonics_tab(lmax, x, y, z, [&](int lm, double s) { v += Ls[lm] * s; });
+    I.V[(size_t)gx + (size_t)I.Nx * gy + (size_t)I.Nx * I.Ny * gz] += v;
+  }
+}
+
+// The Helmholtz potential, one box at a time, with the lane tasks of
+// multipoles_box_kernel: lane p(lmax+1)+t evaluates task t's harmonics of point p and
+// the point's lanes sum their terms with a segmented shuffle reduction.  The
+// Bessel ratios f_l(kappa r), l = 0..lmax, come first for 32 points per
+// warp, one lane per point (series for lmax and lmax - 1, then the downward
+// recursion f_l = (2l+3) f_{l+1} + (kappa r)^2 f_{l+2}), into shared memory.
+// Block (chunk, box, density); Coulomb instances return.
+constexpr int kL2pHelmWarps = 8;
+constexpr int kL2pHelmThreads = kL2pHelmWarps * 32;  // sF has one row block per warp
+
+__global__ void __launch_bounds__(kL2pHelmThreads)
+    l2p_helm_box_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext, int lmax) {
+  __shared__ double sA[16 * 16], sB[16 * 16], sLt[16 * 16];  // [k][t]
+  __shared__ double sF[kL2pHelmWarps][32][17];              // [warp][point][l]
+  const GInst &I = insts[blockIdx.z];
+  if (!(I.kappa > 0.0)) return;
+  if (sh_potential_product(I.boxes[blockIdx.y].route, true)) return;  // l2p_kernel
+  const int L = lmax, L1 = lmax + 1, N = L1 * L1;
+  const int PP = 32 / L1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const BoxInfo b = I.boxes[blockIdx.y];
+  const double *Lb = (Lext ? Lext : I.L + (size_t)I.fine_off * N) + (size_t)blockIdx.y * N;
+  const double kappa = I.kappa;
+  for (int e = threadIdx.x; e < N; e += blockDim.x) {
+    const int t = e / L1, k = e % L1;
+    int l, m;
+    mp_step(L, t, k, l, m);
+    const bool start = l == abs(m);
+    sA[k * 16 + t] = start ? 0.0 : c_shA[lmi(l, m)];
+    sB[k * 16 + t] = start ? 0.0 : c_shB[lmi(l, m)];
+    double kp = 8.0 * kappa / (4.0 * 3.141592653589793238);  // 8 kappa^(l+1) (2l+1) / (4 pi)
+    for (int i = 0; i < l; ++i) kp *= kappa;
+    sLt[k * 16 + t] = Lb[lmi(l, m)] * ((2 * l + 1) * kp);
+  }
+  __syncthreads();
+  const int p = lane / L1, t = lane % L1;
+  int m1, m2, len1;
+  mp_task(L, t, m1, m2, len1);
+  const int a1 = abs(m1), a2 = abs(m2), amax = t == 0 ? 0 : max(a1, a2);
+  const double *xs = I.wbox + (3 * 64) * I.wstride;
+  const int ws = I.wstride;
+  const long long n = (long long)b.own[0] * b.own[1] * b.own[2];
+  double(*F)[17] = sF[warp];
+  const long long stride32 = (long long)gridDim.x * (blockDim.x >> 5) * 32;
+  for (long long base32 = ((long long)blockIdx.x * (blockDim.x >> 5) + warp) * 32; base32 < n;
+       base32 += stride32) {
+  {  // Bessel ratios of the 32 points, lane = point
+    const long long e = min(base32 + lane, n - 1);
+    const int i = (int)(e % b.own[0]);
+    const long long r = e / b.own[0];
+    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
+    const double x = xs[b.p0[0] + i] - b.c[0], y = xs[ws + b.p0[1] + j] - b.c[1],
+                 z = xs[2 * ws + b.p0[2] + k] - b.c[2];
+    const double x2 = (kappa * kappa) * (x * x + y * y + z * z);
+    double *f = F[lane];
+    f[L] = bessel_ratio_series(0.5 * x2, L);
+    if (L >= 1) f[L - 1] = bessel_ratio_series(0.5 * x2, L - 1);
+    for (int l = L - 2; l >= 0; --l) f[l] = (2 * l + 3) * f[l + 1] + x2 * f[l + 2];
+  }
+  __syncwarp();
+  for (int sub = 0; sub < 32; sub += PP) {
+    const long long e = base32 + sub + p;
+    const bool valid = p < PP && sub + p < 32 && e < n;
+    const long long ee = valid ? e : 0;
+    const int i = (int)(ee % b.own[0]);
+    const long long r = ee / b.own[0];
+    const int j = (int)(r % b.own[1]), k = (int)(r / b.own[1]);
+    const int gx = b.p0[0] + i, gy = b.p0[1] + j, gz = b.p0[2] + k;
+    const double x = xs[gx] - b.c[0], y = xs[ws + gy] - b.c[1], z = xs[2 * ws + gz] - b.c[2];
+    const double r2 = x * x + y * y + z * z;
+    double s1 = 1.0, s2 = 0.0;
+    {
+      double top = x, bot = y;
+      for (int mm = 1; mm <= amax; ++mm) {
+        if (mm >= 2) {
+          const double c = c_shC[mm];
+          const double nb = c * (y * top + x * bot);
+          const double nt = c * (x * top - y * bot);
+          top = nt;
+          bot = nb;
+        }
+        if (mm == a1) s1 = m1 > 0 ? top : bot;
+        if (mm == a2) s2 = m2 > 0 ? top : bot;
+      }
+    }
+    const double *fp = F[valid ? sub + p : 0];
+    double acc = 0.0, p1 = 0.0, p2 = 0.0;
+#pragma unroll
+    for (int kk = 0; kk < 16; ++kk) {
+      if (kk > L) break;
+      const bool st = kk == 0 || kk == len1;
+      const double rec = sA[kk * 16 + t] * (z * p1) - sB[kk * 16 + t] * (r2 * p2);
+      const double cur = st ? (kk == 0 ? s1 : s2) : rec;
+      p2 = st ? 0.0 : p1;
+      p1 = cur;
+      const double f = fp[kk < len1 ? a1 + kk : a2 + kk - len1];
+      acc += (sLt[kk * 16 + t] * f) * cur;
+    }
+    // segmented sum over the point's lanes t = 0..L (fixed order)
+#pragma unroll
+    for (int off = 1; off < 16; off <<= 1) {
+      const double o = __shfl_down_sync(0xffffffffu, acc, off);
+      if (t + off < L1) acc += o;
+    }
+    if (valid && t == 0) I.V[(size_t)gx + (size_t)I.Nx * gy + (size_t)I.Nx * I.Ny * gz] += acc;
+  }
+  __syncwarp();
+  }
+}
+
+// The potential as products: grid (chunk, column tile, density).  The tile's expansions stay in shared memory, `pts` points' S at a
+// time beside them (two buffers).
 __global__ void __launch_bounds__(kShThreads, 1)
     l2p_kernel(const GInst *__restrict__ insts, const double *__restrict__ Lext, int L, int pts) {
   extern __shared__ double sh[];
@@ -732,6 +1093,7 @@ __global__ void __launch_bounds__(kShThreads, 1)
   const GInst &I = insts[blockIdx.z];
   if ((int)blockIdx.y >= I.nshtiles) return;
   const ShTile ct = I.shtiles[blockIdx.y];
+  if (!sh_potential_product(ct.route, I.kappa > 0.0)) return;  // l2p_box_kernel, l2p_helm_box_kernel
   const int L1 = L + 1, N = L1 * L1;
   const int pitch = (N + 15) / 16 * 16 + 4, KS = (N + 3) / 4;
   double *S = sh;                     // [2][pts][pitch]
@@ -1128,6 +1490,8 @@ struct dage_gbfmm {
   int wstride = 0, nslab = 1, ndisp = 0;
   DevBuf d_shtiles, d_shboxes;   // boxes by shape (multipoles_kernel, l2p_kernel)
   int nshtiles = 0;
+  std::vector<ShTile> shtiles;
+  std::vector<int> shboxes;
   DevBuf d_U, d_W, d_desc[3];
   size_t U_per_box = 0, W_per_box = 0;
   int near_g = 1;  // t-points per stage-z launch of the FP64 near field (W slots)
@@ -1451,6 +1815,43 @@ int sh_slabs(long long work) {
   return std::max(1, std::min(sm_count(), ceil_div(8LL * sm_count(), work)));
 }
 
+// What the two forms of the moments or of the potential have to do over the
+// densities of a call: column tiles of the products, and boxes that go one at a
+// time (Coulomb, Helmholtz).
+struct ShLoad {
+  long long tiles = 0, boxes[2] = {0, 0};
+  void add(bool product, bool helm, int count) {
+    if (product)
+      ++tiles;
+    else
+      boxes[helm] += count;
+  }
+};
+struct ShLoads {
+  ShLoad moments, potential;
+  void add(const dage_gbfmm *g, bool helm) {
+    for (const ShTile &t : g->shtiles) {
+      moments.add(sh_moments_product(t.route, helm), helm, t.count);
+      potential.add(sh_potential_product(t.route, helm), helm, t.count);
+    }
+  }
+};
+
+// Partial sums per box of the moments: the slabs of either form, the products'
+// at most 256 MB of them over all boxes and densities (they are as many as fill
+// the GPU, whichever kernel a density has).
+int mp_box_slabs(int ninst) { return ninst >= 8 ? 4 : kMpSlabs; }
+int mp_slab_room(const ShLoads &coulomb, const ShLoads &helm, int ninst, long long nbox, int N) {
+  long long most = 1;
+  int boxes = 0;
+  for (const ShLoads *l : {&coulomb, &helm}) {
+    if (l->moments.tiles) most = std::max<long long>(most, sh_slabs(l->moments.tiles));
+    if (l->moments.boxes[0] + l->moments.boxes[1]) boxes = mp_box_slabs(ninst);
+  }
+  most = std::min(most, (1LL << 28) / (8 * nbox * N * ninst));
+  return (int)std::max<long long>({most, boxes, 1});
+}
+
 // The boxes by shape: two positions of an axis are alike if their cells have
 // the same steps and their points the same places about the centre, to the
 // rounding of the coordinates (8 ulp of the largest one).
@@ -1486,23 +1887,86 @@ int build_shapes(dage_gbfmm *g) {
     const int *q = g->boxes[i].pos;
     shapes[{kind[0][q[0]], kind[1][q[1]], kind[2][q[2]]}].push_back(i);
   }
-  std::vector<ShTile> tiles;
+  std::vector<ShTile> &tiles = g->shtiles;
   std::vector<int> boxes;
   for (const auto &sh : shapes)
     for (size_t i = 0; i < sh.second.size(); ++i) {
-      if (i % kShCols == 0) tiles.push_back({(int)boxes.size(), 0});
+      if (i % kShCols == 0) tiles.push_back({(int)boxes.size(), 0, 0});
       boxes.push_back(sh.second[i]);
       ++tiles.back().count;
     }
   g->nshtiles = (int)tiles.size();
-  g->nslab = sh_slabs(g->nshtiles);
+  g->shboxes = boxes;
   DAGE_TRY(g->d_shtiles.alloc(sizeof(ShTile) * tiles.size()));
   DAGE_TRY(g->d_shboxes.alloc(sizeof(int) * boxes.size()));
-  DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_shtiles.ptr, tiles.data(), sizeof(ShTile) * tiles.size(),
-                                cudaMemcpyHostToDevice, g->stream));
   DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_shboxes.ptr, boxes.data(), sizeof(int) * boxes.size(),
                                 cudaMemcpyHostToDevice, g->stream));
   DAGE_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  return 0;
+}
+
+// Chooses the form of the moments and of the potential for the boxes of plans
+// that a call runs together (`uses` densities each), and uploads it.
+//
+// Measured, both forms on the same grids (4^3 boxes in tiles of 1 to 64 alike,
+// 7^3 to 61^3 points a box, lmax 0 to 15): over all boxes the product costs
+// f + sum of points (A / alike - B) more than one box at a time, with A for
+// making S, B for what S saves, f for its launch and idle blocks.  A tile is
+// taken where it saves anything (alike >= A / B), and only if all that are
+// taken save f; twice that where others go one at a time beside them, whose
+// launch then remains.  Fewer than 8 others go with the products: so few boxes
+// do not fill the GPU (139^3, Helmholtz potential, lmax 12: the one box that
+// is like no other took 40 us beside products of 434).  Microseconds of an API call, one at a time -> product,
+// 64 boxes, lmax 12:
+//   Coulomb moments      61^3 points  1 alike: 3237 -> 28275   64: 3237 -> 1012
+//                        31^3         1 alike:  544 ->  3878   64:  544 ->  296
+//   Helmholtz moments    31^3         4 alike: 1033 ->  1283    8: 1033 ->  741
+//   Coulomb potential    31^3         8 alike:  299 ->   412   16:  299 ->  256
+//   Helmholtz potential  31^3         2 alike: 1246 ->  1350    4: 1246 ->  781
+// For lmax 0 to 2 the Coulomb products lose at any number of boxes; from lmax
+// 14 on the potential takes 16 points a step and needs more boxes alike.
+// DAGE_GBFMM_FORM=box|product fixes the form (tests of both).
+int set_routes(const std::vector<dage_gbfmm *> &plans, const std::vector<int> &uses) {
+  const int lmax = plans[0]->lmax;
+  const double l1 = lmax + 1, wide = lmax >= 14 ? 1.0 : 0.0;
+  const double coulomb = 9.0 + 700.0 / (l1 * l1);
+  const double ratio[4] = {coulomb, 1.0 + 70.0 / l1, coulomb + 6.0 * wide,
+                           1.7 + 11.0 / l1 + 2.0 * wide};  // A / B
+  // f / B, in points
+  const double fixed[4] = {64 * 30000.0 / l1, 64 * 10000.0 / l1, 64 * 30000.0 / l1, 64 * 4000.0 / l1};
+  const char *form = std::getenv("DAGE_GBFMM_FORM");
+  const bool all = form && !std::strcmp(form, "product"), none = form && !std::strcmp(form, "box");
+  for (auto *g : plans)
+    for (ShTile &t : g->shtiles) t.route = 0;
+  for (int k = 0; k < 4; ++k) {
+    double saved = 0.0, lost = 0.0;  // by the tiles that share enough, by the rest
+    long long rest = 0;              // boxes
+    for (size_t i = 0; i < plans.size(); ++i)
+      for (const ShTile &t : plans[i]->shtiles) {
+        const int *np = plans[i]->boxes[plans[i]->shboxes[t.first]].np;
+        const double d = (double)uses[i] * np[0] * np[1] * np[2] * (t.count - ratio[k]);
+        if (d >= 0.0) {
+          saved += d;
+        } else {
+          lost -= d;
+          rest += (long long)uses[i] * t.count;
+        }
+      }
+    const bool with = rest < 8;  // the rest goes with the products
+    const bool take = with ? saved - lost >= fixed[k] : saved >= 2 * fixed[k];
+    for (auto *g : plans)
+      for (ShTile &t : g->shtiles)
+        if (all || (!none && take && (with || t.count >= ratio[k]))) t.route |= 1 << k;
+  }
+  for (auto *g : plans) {
+    for (const ShTile &t : g->shtiles)
+      for (int i = 0; i < t.count; ++i) g->boxes[g->shboxes[t.first + i]].route = t.route;
+    DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_boxes.ptr, g->boxes.data(), sizeof(BoxInfo) * g->nbox,
+                                  cudaMemcpyHostToDevice, g->stream));
+    DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_shtiles.ptr, g->shtiles.data(),
+                                  sizeof(ShTile) * g->shtiles.size(), cudaMemcpyHostToDevice, g->stream));
+    DAGE_CUDA_TRY(cudaStreamSynchronize(g->stream));
+  }
   return 0;
 }
 
@@ -1628,9 +2092,7 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
       }
     }
   }
-  DAGE_TRY(g->d_boxes.alloc(sizeof(BoxInfo) * g->nbox));
-  DAGE_CUDA_TRY(cudaMemcpyAsync(g->d_boxes.ptr, g->boxes.data(), sizeof(BoxInfo) * g->nbox,
-                                cudaMemcpyHostToDevice, s));
+  DAGE_TRY(g->d_boxes.alloc(sizeof(BoxInfo) * g->nbox));  // uploaded by set_routes
 
   // --- per-position box weights + point coordinates -------------------------
   int maxn = 0;
@@ -1820,6 +2282,11 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
   DAGE_TRY(build_m2l(g));
   DAGE_TRY(build_shapes(g));
   if (single) {
+    DAGE_TRY(set_routes({g}, {1}));
+    ShLoads coulomb, helm;
+    coulomb.add(g, false);
+    helm.add(g, true);
+    g->nslab = mp_slab_room(coulomb, helm, 1, g->nbox, g->N);
     DAGE_TRY(g->d_q.alloc(sizeof(double) * g->nbtot * g->N));
     DAGE_TRY(g->d_L.alloc(sizeof(double) * g->nbtot * g->N));
     DAGE_TRY(g->d_partial.alloc(sizeof(double) * (size_t)g->nbox * g->nslab * g->N));
@@ -2006,14 +2473,31 @@ void near_bounds(const dage_gbfmm *g, int mt[3], int nt[3]) {
   }
 }
 
-// nshtiles: the largest of the instances
-int run_multipoles(const GInst *d_inst, int ninst, int nbox, int nshtiles, int lmax, int nslab,
-                   cudaStream_t s) {
-  const int N = (lmax + 1) * (lmax + 1);
-  multipoles_kernel<<<dim3(nslab, nshtiles, ninst), kShThreads, sh_mp_smem(N), s>>>(d_inst, lmax,
-                                                                                    nslab);
+int max_owned(const dage_gbfmm *g) {
+  int m = 0;
+  for (const auto &B : g->boxes) m = std::max(m, B.own[0] * B.own[1] * B.own[2]);
+  return m;
+}
+
+// nshtiles: the largest of the instances; stride: partial sums of a box
+int run_multipoles(const GInst *d_inst, int ninst, int nbox, int nshtiles, int lmax,
+                   const ShLoad &load, int stride, cudaStream_t s) {
+  const int N = (lmax + 1) * (lmax + 1), mslab = std::min(mp_box_slabs(ninst), stride);
+  const int nslab = load.tiles ? std::min(sh_slabs(load.tiles), stride) : 1;
+  if (load.boxes[1])
+    multipoles_box_kernel<true><<<dim3(nbox, mslab, ninst), kMpWarps * 32, 0, s>>>(d_inst, lmax,
+                                                                                  mslab, stride);
+  else if (load.boxes[0])
+    multipoles_box_kernel<false><<<dim3(nbox, mslab, ninst), kMpWarps * 32, 0, s>>>(d_inst, lmax,
+                                                                                   mslab, stride);
   DAGE_CUDA_TRY(cudaGetLastError());
-  reduce_slabs_kernel<<<dim3((nbox * N + 255) / 256, ninst), 256, 0, s>>>(d_inst, nslab, N, nbox);
+  if (load.tiles) {
+    multipoles_kernel<<<dim3(nslab, nshtiles, ninst), kShThreads, sh_mp_smem(N), s>>>(
+        d_inst, lmax, nslab, stride);
+    DAGE_CUDA_TRY(cudaGetLastError());
+  }
+  reduce_slabs_kernel<<<dim3((nbox * N + 255) / 256, ninst), 256, 0, s>>>(d_inst, nslab, mslab,
+                                                                         stride, N, nbox);
   DAGE_CUDA_TRY(cudaGetLastError());
   return 0;
 }
@@ -2058,12 +2542,28 @@ int run_l2l(const GInst *d_inst, int ninst, const dage_gbfmm *g, cudaStream_t s)
   return 0;
 }
 
-int run_l2p(const GInst *d_inst, int ninst, int nshtiles, int lmax, const double *Lext,
-            cudaStream_t s) {
-  int pts;
-  const int smem = sh_l2p_smem((lmax + 1) * (lmax + 1), &pts);
-  l2p_kernel<<<dim3(sh_slabs((long long)nshtiles * ninst), nshtiles, ninst), kShThreads, smem, s>>>(d_inst, Lext, lmax, pts);
-  DAGE_CUDA_TRY(cudaGetLastError());
+// maxown: the most owned points of a box
+int run_l2p(const GInst *d_inst, int ninst, int nbox, int nshtiles, int lmax, const ShLoad &load,
+            int maxown, const double *Lext, cudaStream_t s) {
+  const int N = (lmax + 1) * (lmax + 1);
+  if (load.boxes[0]) {
+    const int bx = std::min((maxown + 127) / 128, 64);
+    l2p_box_kernel<<<dim3(bx, nbox, ninst), 128, sizeof(double) * N, s>>>(d_inst, Lext, lmax);
+    DAGE_CUDA_TRY(cudaGetLastError());
+  }
+  if (load.boxes[1]) {
+    const int pts = kL2pHelmThreads;  // points per block pass (one per thread)
+    const int hx = std::min((maxown + pts - 1) / pts, 256);
+    l2p_helm_box_kernel<<<dim3(hx, nbox, ninst), kL2pHelmThreads, 0, s>>>(d_inst, Lext, lmax);
+    DAGE_CUDA_TRY(cudaGetLastError());
+  }
+  if (load.tiles) {
+    int pts;
+    const int smem = sh_l2p_smem(N, &pts);
+    l2p_kernel<<<dim3(sh_slabs(load.tiles), nshtiles, ninst), kShThreads, smem, s>>>(d_inst, Lext,
+                                                                                    lmax, pts);
+    DAGE_CUDA_TRY(cudaGetLastError());
+  }
   return 0;
 }
 
@@ -2373,7 +2873,7 @@ struct dage_gbfmm_batch {
   };
   std::vector<MSet> msets;
   DevBuf ws16[3];  // the sets' shared workspace: split input, U, W
-  int mt[3] = {0, 0, 0}, nt[3] = {0, 0, 0}, nshtiles = 0;
+  int mt[3] = {0, 0, 0}, nt[3] = {0, 0, 0}, nshtiles = 0, maxown = 0;
   int tile_n[3] = {64, 64, 64};
   bool tuned = false;
   DevBuf stage_rho, stage_V;  // host-pointer mode
@@ -2476,11 +2976,20 @@ int batch_create_impl(dage_gbfmm_batch *b, int n, const dage_grid1d *grids, int 
   for (const auto *g : b->plans) {
     near_bounds(g, b->mt, b->nt);
     b->nshtiles = std::max(b->nshtiles, g->nshtiles);
+    b->maxown = std::max(b->maxown, max_owned(g));
   }
   const size_t per = (size_t)g0->nbtot * b->N;  // every level's boxes
   DAGE_TRY(b->q.alloc(sizeof(double) * per * n));
   DAGE_TRY(b->L.alloc(sizeof(double) * per * n));
-  b->nslab = sh_slabs((long long)b->nshtiles * n);
+  std::vector<int> uses(b->plans.size(), 0);
+  for (int p : b->plan_of) ++uses[p];
+  DAGE_TRY(set_routes(b->plans, uses));
+  ShLoads coulomb, helm;
+  for (int i = 0; i < n; ++i) {
+    coulomb.add(b->plans[b->plan_of[i]], false);
+    helm.add(b->plans[b->plan_of[i]], true);
+  }
+  b->nslab = mp_slab_room(coulomb, helm, n, b->nbox, b->N);
   DAGE_TRY(b->partial.alloc(sizeof(double) * (size_t)b->nbox * b->N * b->nslab * n));
   DAGE_TRY(b->epart.alloc(sizeof(double) * kEnergyBlocks * n));
   DAGE_TRY(b->energy.alloc(sizeof(double) * n));
@@ -2642,7 +3151,9 @@ int batch_launch(dage_gbfmm_batch *b, const double *const *rho, double *const *V
     }
   for (int i = 0; i < b->n; ++i)
     DAGE_CUDA_TRY(cudaMemsetAsync(V[i], 0, sizeof(double) * b->npts[i], s));
-  DAGE_TRY(run_multipoles(d_inst, b->n, b->nbox, b->nshtiles, b->lmax, b->nslab, s));
+  ShLoads load;
+  for (int i = 0; i < b->n; ++i) load.add(b->plans[b->plan_of[i]], b->kern_of[i] >= 0);
+  DAGE_TRY(run_multipoles(d_inst, b->n, b->nbox, b->nshtiles, b->lmax, load.moments, b->nslab, s));
   DAGE_TRY(run_m2m(d_inst, b->n, b->plans[0], s));
   DAGE_TRY(run_m2l(d_inst, b->n, b->plans[0]->nbtot, b->N, (long long)b->nbox * b->nslab, s));
   DAGE_TRY(run_l2l(d_inst, b->n, b->plans[0], s));
@@ -2652,7 +3163,7 @@ int batch_launch(dage_gbfmm_batch *b, const double *const *rho, double *const *V
     DAGE_TRY(run_near(dd, c.njobs, b->mt, b->nt, b->P, b->w, b->tile_n, b->near_g, s));
   }
   for (auto &m : b->msets) DAGE_TRY(near_f16_set_run(m.set, s));
-  DAGE_TRY(run_l2p(d_inst, b->n, b->nshtiles, b->lmax, nullptr, s));
+  DAGE_TRY(run_l2p(d_inst, b->n, b->nbox, b->nshtiles, b->lmax, load.potential, b->maxown, nullptr, s));
   DAGE_TRY(run_energy(d_inst, b->n, b->energy.as<double>(), s));
   return 0;
 }
@@ -2762,7 +3273,9 @@ int dage_gbfmm_apply(dage_gbfmm *g, const double *rho, double *V, unsigned flags
   DAGE_TRY(single_setup(g, d_rho, d_V, g->near16set == nullptr));
   const GInst *d_inst = g->d_inst.as<GInst>();
   DAGE_CUDA_TRY(cudaMemsetAsync(d_V, 0, sizeof(double) * n, s));
-  DAGE_TRY(run_multipoles(d_inst, 1, g->nbox, g->nshtiles, g->lmax, g->nslab, s));
+  ShLoads load;
+  load.add(g, g->kappa > 0.0);
+  DAGE_TRY(run_multipoles(d_inst, 1, g->nbox, g->nshtiles, g->lmax, load.moments, g->nslab, s));
   DAGE_TRY(run_m2m(d_inst, 1, g, s));
   DAGE_TRY(run_m2l(d_inst, 1, g->nbtot, g->N, (long long)g->nbox * g->nslab, s));
   DAGE_TRY(run_l2l(d_inst, 1, g, s));
@@ -2775,7 +3288,7 @@ int dage_gbfmm_apply(dage_gbfmm *g, const double *rho, double *V, unsigned flags
                               g->d_desc[2].as<StageDesc>()};
     DAGE_TRY(run_near(dd, g->nbox, mt, nt, g->P, g->w, g->tile_n, g->near_g, s));
   }
-  DAGE_TRY(run_l2p(d_inst, 1, g->nshtiles, g->lmax, nullptr, s));
+  DAGE_TRY(run_l2p(d_inst, 1, g->nbox, g->nshtiles, g->lmax, load.potential, max_owned(g), nullptr, s));
   if (flags & DAGE_ENERGY) DAGE_TRY(run_energy(d_inst, 1, g->d_energy.as<double>(), s));
   if (!(flags & DAGE_DEVICE_PTRS))
     DAGE_CUDA_TRY(cudaMemcpyAsync(V, d_V, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
@@ -2797,7 +3310,10 @@ int dage_gbfmm_multipole_moments(dage_gbfmm *g, const double *rho, unsigned flag
   double *d_V;
   DAGE_TRY(stage_io(g, rho, nullptr, flags & DAGE_DEVICE_PTRS, &d_rho, &d_V));
   DAGE_TRY(single_setup(g, d_rho, nullptr, false));
-  DAGE_TRY(run_multipoles(g->d_inst.as<GInst>(), 1, g->nbox, g->nshtiles, g->lmax, g->nslab, g->stream));
+  ShLoads load;
+  load.add(g, g->kappa > 0.0);
+  DAGE_TRY(run_multipoles(g->d_inst.as<GInst>(), 1, g->nbox, g->nshtiles, g->lmax, load.moments,
+                          g->nslab, g->stream));
   DAGE_CUDA_TRY(cudaMemcpyAsync(moments, g->d_q.as<double>() + (size_t)g->fine_off * g->N,
                                 sizeof(double) * g->nbox * g->N,
                                 cudaMemcpyDeviceToHost, g->stream));
@@ -2831,7 +3347,10 @@ int dage_gbfmm_evaluate_le(dage_gbfmm *g, const double *local_expansions, double
     d_V = g->d_V.as<double>();
   }
   DAGE_TRY(single_setup(g, nullptr, d_V, false));
-  DAGE_TRY(run_l2p(g->d_inst.as<GInst>(), 1, g->nshtiles, g->lmax, dL.as<double>(), s));
+  ShLoads load;
+  load.add(g, g->kappa > 0.0);
+  DAGE_TRY(run_l2p(g->d_inst.as<GInst>(), 1, g->nbox, g->nshtiles, g->lmax, load.potential,
+                   max_owned(g), dL.as<double>(), s));
   if (!(flags & DAGE_DEVICE_PTRS))
     DAGE_CUDA_TRY(cudaMemcpyAsync(V, d_V, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   DAGE_CUDA_TRY(cudaStreamSynchronize(s));
