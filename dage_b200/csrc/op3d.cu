@@ -879,17 +879,16 @@ static int fp64_group(const dage_op3d *op) {
 }
 
 // The intermediates of a group of t-points in one allocation: U, then W.
-// Where a group takes too much of the free memory it becomes a single t-point.
-// The group is chosen once and kept with its memory: it sets the order of the sums
+// Where a group does not fit the free memory it becomes a single t-point.  The
+// group is chosen once and kept with its memory: it sets the order of the sums
 // over the t-points, so applies of one operator agree to the last bit, and a
-// later apply frees and allocates nothing.  The tuner takes it at creation;
-// otherwise (its choice known already) the first apply does (~0.4 ms).
+// later apply frees and allocates nothing (op3d_alloc may take the group back
+// where the operator could not go on otherwise).  The tuner takes it at
+// creation; if its choice is known already the first apply does (~0.4 ms).
 static int fp64_workspace(dage_op3d *op) {
   if (op->tmp_group) return 0;
   const size_t niy = op->nin[1], niz = op->nin[2], nox = op->nout[0], noy = op->nout[1];
-  int G = fp64_group(op);
-  if (G > 1 && !room_to_spare(sizeof(double) * (G - 1) * niz * nox * (niy + noy))) G = 1;
-  for (;; G = 1) {
+  for (int G = std::min(fp64_group(op), op->tmp_most);; G = 1) {
     const size_t nu = G * niy * niz * nox;
     const int rc = op->tmp.alloc(sizeof(double) * (nu + G * niz * nox * noy));
     if (rc && G == 1) return rc;
@@ -900,6 +899,21 @@ static int fp64_workspace(dage_op3d *op) {
     }
     clear_error();
   }
+}
+
+int op3d_alloc(dage_op3d *op, DevBuf &buf, size_t bytes) {
+  const int rc = buf.alloc(bytes);
+  if (!rc) return 0;
+  if (op->precision != DAGE_FP64) {
+    if (!mixed_shrink(op)) return rc;
+  } else {
+    if (op->tmp_group <= 1) return rc;
+    op->tmp.release();
+    op->tmp_group = 0;
+    op->tmp_most = 1;
+  }
+  clear_error();
+  return buf.alloc(bytes);
 }
 
 // The three stages of one group of t-points: every t-point's U and W in its
@@ -1166,8 +1180,8 @@ int op3d_enqueue(dage_op3d *op, const double *rho, double *V, unsigned flags, do
   double *d_V = V;
   DAGE_CUDA_TRY(cudaEventRecord(op->ev0, s));
   if (!dev) {
-    DAGE_TRY(op->d_rho.alloc(sizeof(double) * nin));
-    DAGE_TRY(op->d_V.alloc(sizeof(double) * nout));
+    DAGE_TRY(op3d_alloc(op, op->d_rho, sizeof(double) * nin));
+    DAGE_TRY(op3d_alloc(op, op->d_V, sizeof(double) * nout));
     DAGE_CUDA_TRY(cudaMemcpyAsync(op->d_rho.ptr, rho, sizeof(double) * nin,
                                   cudaMemcpyHostToDevice, s));
     if (acc)
@@ -1216,8 +1230,8 @@ int pipe_open(dage_op3d *op) {
   const size_t nin = (size_t)op->nin[0] * op->nin[1] * op->nin[2];
   const size_t nout = (size_t)op->nout[0] * op->nout[1] * op->nout[2];
   for (int k = 0; k < 2; ++k) {
-    DAGE_TRY(op->pipe_rho[k].alloc(sizeof(double) * nin));
-    DAGE_TRY(op->pipe_V[k].alloc(sizeof(double) * nout));
+    DAGE_TRY(op3d_alloc(op, op->pipe_rho[k], sizeof(double) * nin));
+    DAGE_TRY(op3d_alloc(op, op->pipe_V[k], sizeof(double) * nout));
   }
   DAGE_CUDA_TRY(cudaEventRecord(op->ev0, op->pipe_in));
   op->pipe_open = true;

@@ -34,9 +34,9 @@ struct dage_op3d {
   dage::DevBuf d_w;          // weights w_p on the device
   dage::DevBuf d_rho, d_V;   // staging for host pointers
   // intermediates of the FP64 path: U, then W at tmp_w, for tmp_group t-points
-  // (0: not allocated yet; chosen once, see fp64_workspace)
+  // (0: not allocated yet; chosen once, at most tmp_most, see fp64_workspace)
   dage::DevBuf tmp;
-  int tmp_group = 0;
+  int tmp_group = 0, tmp_most = 1 << 30;
   size_t tmp_w = 0;
   dage::DevBuf partials;     // energy reduction partial sums
 
@@ -97,6 +97,11 @@ int launch_finalize(const double *f1, double *f2_or_V, const double *rho_for_cod
 
 int finalize_partials_count();
 
+// buf.alloc(bytes) for what an operator needs beside its intermediates: where
+// it fails, a group of t-points gives back its slots but one, and it is tried
+// again.
+int op3d_alloc(dage_op3d *op, DevBuf &buf, size_t bytes);
+
 // Gauss-Legendre t-points/weights on the GPU (host copies + device tp).
 int build_quadrature(const dage_quad &q, std::vector<double> &tp, std::vector<double> &tw,
                      DevBuf &d_tp, cudaStream_t s);
@@ -118,6 +123,8 @@ int mixed_apply(dage_op3d *op, const double *d_rho, double *d_V, cudaStream_t s)
 int mixed_enqueue(dage_op3d *op, const double *d_rho, double *d_V, cudaStream_t s);
 int mixed_check(dage_op3d *op, cudaStream_t s);
 int mixed_set_weights(dage_op3d *op);
+// gives back the slots of a group of t-points: true if there were any
+bool mixed_shrink(dage_op3d *op);
 int mixed_tune(dage_op3d *op);
 int mixed_schedule(const dage_op3d *op, int *ring_stages, int *group);
 void mixed_destroy(dage_op3d *op);

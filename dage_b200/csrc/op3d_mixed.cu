@@ -1132,6 +1132,20 @@ static int split_matrices(dage_op3d *op, MixedState *st, int ax) {
   return 0;
 }
 
+// X[1] for Gi t-points, or for one where they do not fit; nothing where it is
+// there (an apply looks again: one that was shrunk may have lost it).
+static int first_slots(dage_op3d *op, MixedState *st) {
+  if (st->X[1].ptr) return 0;
+  if (st->Gi > 1 && st->X[1].alloc(st->xbytes[1] * st->Gi)) {
+    clear_error();
+    st->Gi = 1;
+  }
+  DAGE_TRY(st->X[1].alloc(st->xbytes[1] * st->Gi));
+  DAGE_CUDA_TRY(cudaMemsetAsync(st->X[1].ptr, 0, st->X[1].bytes, op->stream));
+  DAGE_CUDA_TRY(cudaStreamSynchronize(op->stream));
+  return 0;
+}
+
 int mixed_setup(dage_op3d *op) {
   auto *st = new MixedState();
   op->mixed = st;
@@ -1163,14 +1177,9 @@ int mixed_setup(dage_op3d *op) {
     st->nkb[s] = ceil_div(op->nin[s], BK);
     st->natA[s] = ceil_div(rows[s], kAtomRows);
     st->xbytes[s] = (size_t)outer[s] * st->nkb[s] * st->natA[s] * (st->nparts * kAtomRows * BK * 2);
-    // a group that takes too much of the free memory becomes one t-point
-    if (s == 1 && st->Gi > 1 &&
-        (!room_to_spare(st->xbytes[1] * (st->Gi - 1)) || st->X[1].alloc(st->xbytes[1] * st->Gi))) {
-      clear_error();
-      st->Gi = 1;
-    }
+    if (s == 1) continue;  // below
     // padding rows and K columns are never written: they stay zero
-    DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : s == 1 ? st->Gi : 1)));
+    DAGE_TRY(st->X[s].alloc(st->xbytes[s] * (s == 2 ? st->Gmax : 1)));
     DAGE_CUDA_TRY(cudaMemsetAsync(st->X[s].ptr, 0, st->X[s].bytes, op->stream));
   }
   DAGE_TRY(st->err.alloc(sizeof(int)));
@@ -1191,7 +1200,18 @@ int mixed_setup(dage_op3d *op) {
     DAGE_TRY(st->g01.alloc(sizeof(float) * 2 * op->P));
     DAGE_TRY(st->wcoef.alloc(sizeof(float) * op->P));
   }
-  return mixed_set_weights(op);
+  DAGE_TRY(mixed_set_weights(op));
+  // last, since its group is what can be done without
+  return first_slots(op, st);
+}
+
+bool mixed_shrink(dage_op3d *op) {
+  auto *st = static_cast<MixedState *>(op->mixed);
+  if (!st || st->Gi <= 1 || !st->X[1].ptr) return false;
+  cudaStreamSynchronize(op->stream);
+  st->X[1].release();
+  st->Gi = 1;
+  return !first_slots(op, st);
 }
 
 int mixed_set_weights(dage_op3d *op) {
@@ -1217,6 +1237,7 @@ int mixed_apply(dage_op3d *op, const double *d_rho, double *d_V, cudaStream_t s)
 int mixed_enqueue(dage_op3d *op, const double *d_rho, double *d_V, cudaStream_t s) {
   auto *st = static_cast<MixedState *>(op->mixed);
   if (!st) return fail(DAGE_E_INVALID, "mixed state missing");
+  DAGE_TRY(first_slots(op, st));
   int rc;
   if (st->f16)
     rc = st->ns == 4 ? run_stages<2, 4, true>(op, *st, d_rho, d_V, s)
@@ -1274,8 +1295,8 @@ int mixed_tune(dage_op3d *op) {
   const size_t nin = (size_t)op->nin[0] * op->nin[1] * op->nin[2];
   const size_t nout = (size_t)op->nout[0] * op->nout[1] * op->nout[2];
   TmpBuf rho, V;
-  DAGE_TRY(rho.alloc(sizeof(double) * nin));
-  DAGE_TRY(V.alloc(sizeof(double) * nout));
+  DAGE_TRY(op3d_alloc(op, rho, sizeof(double) * nin));
+  DAGE_TRY(op3d_alloc(op, V, sizeof(double) * nout));
   cudaStream_t s = op->stream;
   fill_kernel<<<(int)std::min<size_t>((nin + 255) / 256, (size_t)sm_count() * 16), 256, 0, s>>>(
       rho.as<double>(), nin, 1.0);

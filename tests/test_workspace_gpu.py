@@ -245,3 +245,26 @@ def test_refused_allocation_leaves_no_error_behind(dage):
         del e
         got = _apply(dage.Coulomb3D(g, quad=quad), rho, V)
     assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()  # another group of t-points
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp16x3"])
+def test_group_gives_way_to_host_cubes(dage, precision):
+    """121^3: an operator whose group of t-points took the memory that a
+    host-array apply stages its two 14 MB cubes in gives the group back."""
+    g = dage.Grid3D.cube(-12.0, 20, 0.2)
+    op = dage.Coulomb3D(g, quad=dage.GaussQuad(9, 8), precision=precision)
+    rho, V = _density(g.shape), _density(g.shape)
+    want = _apply(op, rho, V).transpose(2, 1, 0)
+    host = np.asfortranarray(rho.cpu().numpy().transpose(2, 1, 0))
+    with _Leave(10 * MIB):
+        got = op.apply(host)
+    assert np.abs(got - want).max() <= (1e-13 if precision == "fp64" else 0) * np.abs(want).max()
+    with _Leave(10 * MIB):  # and stays as it is then
+        np.testing.assert_array_equal(op.apply(host), got)
+        out = [np.empty(g.shape, order="F")]
+        with pytest.raises(dage.DageError) as e:  # the pipeline's second pair of cubes: no room left
+            dage.apply_batched([op], [host], out)
+        assert e.value.code == -3
+        del e
+    dage.apply_batched([op], [host], out)
+    np.testing.assert_array_equal(out[0], got)
