@@ -57,7 +57,8 @@ std::string tune_device_key() {
   std::string name = prop.name;
   for (char &c : name)
     if (c == ' ') c = '_';
-  return name + "/sm" + std::to_string(prop.multiProcessorCount);
+  return name + "/sm" + std::to_string(prop.multiProcessorCount) + "/r" +
+         std::to_string(kTuneRevision);
 }
 
 bool tune_lookup(const std::string &key, std::vector<int> &val) {
