@@ -1728,7 +1728,6 @@ int sh_prepare() {
   });
 }
 
-// M2L matrix of every distinct displacement for the plan's kernel.
 // M2L matrix of every distinct displacement of a plan for the kernel with
 // parameter kappa (0: Coulomb), into T.
 int build_m2l_into(const dage_gbfmm *g, double kappa, DevBuf &T) {
@@ -2316,6 +2315,7 @@ int gbfmm_create_impl(dage_gbfmm *g, const dage_grid1d grid[3], int maxlevel, in
       DAGE_TRY(g->Tnear[d][v].alloc(sizeof(double) * (size_t)g->P * own * nq));
       DAGE_TRY(build_axis_matrix(ain, g->ax[d].points.data() + pos_p0[d][v], own,
                                  d_tp.as<double>(), g->P, g->Tnear[d][v].as<double>(), s));
+      if (g->precision != DAGE_FP64) continue;  // near_mixed.cu keeps run tables of its own
       DAGE_TRY(g->band_near[d][v].alloc(sizeof(int2) * (size_t)g->P * ceil_div(own, kBandCols)));
       DAGE_TRY(launch_band(g->Tnear[d][v].as<double>(), nq, own, g->P,
                            g->band_near[d][v].as<int2>(), s));
@@ -2596,8 +2596,9 @@ int run_energy(const GInst *d_inst, int ninst, double *d_out, cudaStream_t s) {
 
 // Autotuner: the tile width (32, 64 or 128 columns) of each near-field
 // stage, chosen by timing every candidate on a batched launch of t-point 0 (the
-// last stage: of the first group; one warm-up, three timed launches; the launches write the intermediates
-// and the output cubes of the descriptors, which the caller overwrites).
+// last stage: of the first group; one warm-up, three timed launches; the
+// launches write the intermediates and the output cubes of the descriptors,
+// which the caller overwrites).
 int autotune_tiles(const StageDesc *const d_desc[3], int njobs, const int mt[3], const int nt[3],
                    int G, cudaStream_t s, int tile_n[3]) {
   cudaEvent_t e0, e1;

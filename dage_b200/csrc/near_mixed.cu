@@ -743,7 +743,6 @@ int near_f16_plan_create(NearF16Plan **out, const NearGeom &geom, cudaStream_t s
     DAGE_TRY(pl->l1[d].alloc(sizeof(double) * P));
     DAGE_TRY(pl->psc[d].alloc(sizeof(double) * P));
     // per-position tables on the device
-    std::vector<long long> tab;  // T pointers, then own, nq, brow, koff as int
     TmpBuf dT, dI, stats;
     DAGE_TRY(dT.alloc(sizeof(double *) * npos));
     DAGE_TRY(dI.alloc(sizeof(int) * 4 * npos));
@@ -815,10 +814,12 @@ struct SetDims {
 };
 
 // Two t-points per stage-x tile, the columns of each half (0: one t-point):
-// with at most 32 own points they share a 64-column tile (61^3 1.63 -> 1.36 ms
-// an apply, 121^3 3.42 -> 2.94), up to 49 a 128-column one (181^3, 46 points,
-// 9.95 -> 9.19); with 60 the wider tile's drains cost more than the shared
-// input saves (241^3 16.1 -> 18.3; between 49 and 60 not measured).
+// with at most 32 own points they share a 64-column tile, up to 49 a
+// 128-column one; above that the wider tile's drains cost more than the shared
+// input saves.  Apply with one t-point per tile -> two, ms, lmax 2, 40 t-points:
+// 31 points (121^3) 3.27 -> 2.81; 36 (133^3) 5.04 -> 4.62; 48 (181^3) 8.07 ->
+// 7.35; 49 (193^3) 11.5 -> 10.9; 54 (205^3) 9.92 -> 9.10, but (211^3) 14.0 ->
+// 14.3; 55 (217^3) 13.1 -> 14.6; 61 (241^3) 15.9 -> 18.3.
 int pair_half(const NearF16Plan *pl, int tile_n) {
   return tile_n != 64 ? 0 : pl->maxown[0] <= 32 ? 32 : pl->maxown[0] <= 49 ? 64 : 0;
 }

@@ -53,16 +53,17 @@
 // stored value is below 2^15 and values below 2^-39 of the bound flush.  The
 // tensor core's toward-zero rounding of the FP32 partials (~0.5 ulp per
 // rounding, all of one sign for positive sums) is then the largest error
-// left; the epilogue adds half an ulp to each partial on average (+1 ulp to
-// the odd ones) before summing, which removes that bias.
+// left; the epilogue moves every partial one ulp away from zero before summing
+// (unbias_rz), which removes that bias on average.
 //
 // Kernel structure (one persistent CTA per SM, 18 warps):
 //   warp 0      producer: bulk copies of X and T tiles -> shared-memory ring
 //   warp 1      TMEM allocator + MMA issuer (one elected lane)
 //   warps 2-17  epilogue, four warps per scheduler (32 columns each):
 //               partial sums -> scale -> split -> global stores
-// TMEM holds three 128-column partial buffers (the MMAs of the next slices
-// overlap the epilogue's reads) and the 128-column correction accumulator.
+// TMEM holds 128-column partial buffers (the MMAs of the next slices overlap
+// the epilogue's reads): three and a 128-column correction accumulator in the
+// BF16 modes, four and none in fp16x3, whose partials take the corrections.
 // Every mbarrier wait is bounded (clock64 budget); on timeout the CTA
 // records the failure in a device flag, drains its in-flight copies and
 // MMAs, frees TMEM and returns.
