@@ -35,3 +35,31 @@ def test_against_fp64_operator(dage, precision, cells, out_cells):
     V = dage.Operator3D(g, go, quad, precision=precision).apply(rho, coda=False)
     V64 = dage.Operator3D(g, go, quad).apply(rho, coda=False)
     assert np.abs(V - V64).max() <= BARS[precision] * np.abs(V64).max()
+
+
+@pytest.mark.parametrize("precision,ncell,nlin,nlog", [
+    ("fp16x3", 30, 7, 6),   # 181^3: two t-points per intermediate launch, 13 in all: 2 2 2 2 | 2 2 1
+    ("bf16x3", 27, 7, 6),   # 163^3: three: 3 3 2 | 3 2
+    ("bf16x6", 24, 8, 3),   # 145^3, three parts: three: 3 3 2 | 3
+])
+def test_groups_of_several_intermediate_launches(dage, precision, ncell, nlin, nlog):
+    """More than one launch of the first two stages per group of the last one:
+    slots of the second intermediate written at their offset in the group, slots
+    of the first one reused, a last launch of fewer t-points.  (One t-point per
+    launch, 481^3, and the whole group in one, the cubes above, have none of
+    these.)  A t-point in the wrong slot is an error of the t-point's share."""
+    import torch
+
+    g = dage.Grid3D.cube(-0.6 * ncell, ncell, 0.2)
+    quad = dage.GaussQuad(nlin, nlog)
+    n = g.shape[0]
+    gen = torch.Generator(device="cuda").manual_seed(ncell)
+    rho = torch.rand(n, n, n, dtype=torch.float64, device="cuda", generator=gen)
+    V, V64 = torch.empty_like(rho), torch.empty_like(rho)
+    op = dage.Coulomb3D(g, quad=quad, precision=precision)
+    op.apply(rho, V)
+    dage.Coulomb3D(g, quad=quad).apply(rho, V64)
+    assert float((V - V64).abs().max()) <= BARS[precision] * float(V64.abs().max())
+    again = torch.empty_like(V)
+    op.apply(rho, again)
+    assert torch.equal(V, again)
