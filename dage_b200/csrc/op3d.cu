@@ -911,6 +911,7 @@ int op3d_alloc(dage_op3d *op, DevBuf &buf, size_t bytes) {
     op->tmp.release();
     op->tmp_group = 0;
     op->tmp_most = 1;
+    DAGE_TRY(fp64_workspace(op));  // its own slot first: the operator stays usable
   }
   clear_error();
   return buf.alloc(bytes);
